@@ -238,6 +238,26 @@ int ed_grad_energy(const ed_basis* b, const int32_t* pairs_host, int64_t nbonds,
                    double* dD_host, double* dh_host) {
   if (!b || !psi_dev || (nbonds > 0 && !pairs_host)) return ed_fail(ED_EINVAL, "null argument");
   const int N = b->nspins;
+  for (int64_t q = 0; q < 2 * nbonds; ++q)
+    if (pairs_host[q] < 0 || pairs_host[q] >= N) return ed_fail(ED_EINVAL, "site index out of range");
+  {
+    // a real psi (the solver's eigenvectors): the S^z moments and flip sums of
+    // all bonds at once (ed_corr.cu)
+    ed_corr c;
+    const int rc = ed_corr_real(b, (const double2*)psi_dev, true, pairs_host, nbonds, c);
+    if (rc == ED_OK) {
+      const double inv = 1.0 / c.W;
+      for (int64_t q = 0; q < nbonds; ++q) {
+        const int i = pairs_host[2 * q], j = pairs_host[2 * q + 1];
+        if (dJ_host) dJ_host[q] = (i == j ? 0.5 * c.zz(i, i) : c.F[q]) * inv;
+        if (dD_host) dD_host[q] = 0.25 * c.zz(i, j) * inv;
+      }
+      for (int i = 0; i < N; ++i)
+        if (dh_host) dh_host[i] = c.sz(i) * inv;
+      return ED_OK;
+    }
+    if (rc != ED_ENOMEM && rc != ED_ENOTSUP) return rc;
+  }
   std::vector<int> kinds;
   std::vector<int32_t> ij;
   for (int64_t q = 0; q < nbonds; ++q) {

@@ -21,6 +21,36 @@ int ed_cuda_fail(cudaError_t e, const char* what, const char* file, int line) {
   return e == cudaErrorMemoryAllocation ? ED_ENOMEM : ED_ECUDA;
 }
 
+ed_workspace::ed_workspace(ed_ctx* c, size_t bytes) : ctx(c) {
+  if (bytes <= ED_WS_KEEP && !c->ws_busy) {
+    if (bytes > c->ws_cap) {
+      if (c->ws) cudaFree(c->ws);
+      c->ws = nullptr;
+      c->ws_cap = 0;
+      if (cudaMalloc(&c->ws, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        c->ws = nullptr;
+        return;
+      }
+      c->ws_cap = bytes;
+    }
+    c->ws_busy = true;
+    ptr = c->ws;
+    return;
+  }
+  if (cudaMalloc(&ptr, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    ptr = nullptr;
+    return;
+  }
+  own = true;
+}
+
+ed_workspace::~ed_workspace() {
+  if (own) cudaFree(ptr);
+  else if (ptr) ctx->ws_busy = false;
+}
+
 extern "C" {
 
 int ed_last_error(char* buf, size_t len) {
@@ -91,6 +121,7 @@ int ed_ctx_destroy(ed_ctx* c) {
   clear_profile(c);
   if (c->d_red) cudaFree(c->d_red);
   if (c->h_red) cudaFreeHost(c->h_red);
+  if (c->ws) cudaFree(c->ws);
   if (c->own_stream) cudaStreamDestroy(c->stream);
   delete c;
   return ED_OK;
@@ -200,6 +231,8 @@ int ed_basis_destroy(ed_basis* b) {
   if (b->d_tab) cudaFree(b->d_tab);
   if (b->d_lin_t0) cudaFree(b->d_lin_t0);
   if (b->d_lin_t1) cudaFree(b->d_lin_t1);
+  if (b->d_lin_lows) cudaFree(b->d_lin_lows);
+  if (b->d_lin_highs) cudaFree(b->d_lin_highs);
   delete b;
   return ED_OK;
 }

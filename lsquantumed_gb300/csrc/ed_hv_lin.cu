@@ -92,6 +92,27 @@ int ed_basis_lin_tables(ed_basis* b) {
   if (e1 != cudaSuccess || e2 != cudaSuccess)
     return ed_cuda_fail(e1 != cudaSuccess ? e1 : e2, "rank table upload", __FILE__, __LINE__);
   b->lin_w0 = w0;
+  // the halves by popcount (ascending within): the order of the states of one
+  // high half, and the high halves whose states share it
+  std::vector<uint16_t> lows;
+  std::vector<uint32_t> highs;
+  lows.reserve(t0.size());
+  highs.reserve(t1.size());
+  for (int k = 0; k <= w0; ++k)
+    for (uint32_t c = 0; c < t0.size(); ++c)
+      if (__builtin_popcount(c) == k) lows.push_back((uint16_t)c);
+  for (int k = 0; k <= w1; ++k)
+    for (uint32_t c = 0; c < t1.size(); ++c)
+      if (__builtin_popcount(c) == k) highs.push_back(c);
+  if (cudaMalloc(&b->d_lin_lows, lows.size() * sizeof(uint16_t)) != cudaSuccess ||
+      cudaMalloc(&b->d_lin_highs, highs.size() * sizeof(uint32_t)) != cudaSuccess) {
+    cudaGetLastError();
+    return ed_fail(ED_ENOMEM, "rank tables do not fit in device memory");
+  }
+  e1 = cudaMemcpy(b->d_lin_lows, lows.data(), lows.size() * sizeof(uint16_t), cudaMemcpyHostToDevice);
+  e2 = cudaMemcpy(b->d_lin_highs, highs.data(), highs.size() * sizeof(uint32_t), cudaMemcpyHostToDevice);
+  if (e1 != cudaSuccess || e2 != cudaSuccess)
+    return ed_cuda_fail(e1 != cudaSuccess ? e1 : e2, "rank table upload", __FILE__, __LINE__);
   return ED_OK;
 }
 

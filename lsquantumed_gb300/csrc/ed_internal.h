@@ -92,6 +92,10 @@ struct ed_ctx {
   size_t red_cap = 0;             // doubles
   double* h_red = nullptr;
   int reduce_blocks = 0;
+  // scratch kept between calls (ed_workspace), at most ED_WS_KEEP bytes
+  void* ws = nullptr;
+  size_t ws_cap = 0;
+  bool ws_busy = false;
   // H.v launch timing (events on the stream)
   bool profiling = false;
   std::vector<cudaEvent_t> prof_events;  // pairs (start, stop)
@@ -109,7 +113,45 @@ struct ed_basis {
   int lin_w0 = 0;
   uint16_t* d_lin_t0 = nullptr;
   uint32_t* d_lin_t1 = nullptr;
+  // the halves ordered by popcount, then value
+  uint16_t* d_lin_lows = nullptr;
+  uint32_t* d_lin_highs = nullptr;
 };
+
+// Device scratch of one call, in stream order: the context keeps up to
+// ED_WS_KEEP bytes from call to call (an allocation and its free cost more
+// than a small measurement); a larger request is allocated and freed with
+// the call.  ptr is null when it does not fit.
+#define ED_WS_KEEP ((size_t)512 << 20)
+struct ed_workspace {
+  ed_ctx* ctx;
+  void* ptr = nullptr;
+  bool own = false;
+  ed_workspace(ed_ctx* c, size_t bytes);
+  ~ed_workspace();
+  ed_workspace(const ed_workspace&) = delete;
+  ed_workspace& operator=(const ed_workspace&) = delete;
+};
+
+// Correlations of a real state (ed_corr.cu): the exact S^z moments as
+// integers and the flip sums of the pairs asked for.
+#define ED_CORR_FEW 16  // flip pairs up to here run directly, more as a Gram matrix
+struct ed_corr {
+  bool real = false;
+  int N = 0;
+  double W = 0.0;          // sum psi_r^2
+  double inv_scale = 1.0;  // of the integer sums
+  unsigned __int128 T = 0;               // sum w
+  std::vector<unsigned __int128> P;      // [a (a + 1) / 2 + b], b <= a: sum w over the states with a and b up
+  std::vector<double> F;                 // flip sum per pair of the call (0 for i == j)
+  double zz(int i, int j) const;         // sum w sigma_i sigma_j
+  double up(int i) const;                // sum w over the states with i up
+  double down(int i) const;
+  double sz(int i) const;                // sum w S^z_i
+};
+// ED_ENOTSUP (out.real tells which) when psi is not real or not finite,
+// ED_ENOMEM when the scratch does not fit.
+int ed_corr_real(const ed_basis* b, const double2* psi, bool want_zz, const int32_t* pairs, int64_t np, ed_corr& out);
 
 struct ed_lin;  // two-table fixed-point H.v state (ed_hv_lin.cu)
 
