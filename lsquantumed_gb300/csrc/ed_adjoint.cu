@@ -59,8 +59,13 @@ __device__ __forceinline__ double2 op_apply(int kind, int i, int j, uint32_t s, 
 template <int K>
 __global__ void __launch_bounds__(256) k_expect_mixed(const uint32_t* __restrict__ states, const double2* __restrict__ lam,
                                                       const double2* __restrict__ psi, int64_t dim, const RankTables rt,
-                                                      const TermGroup tg, double* __restrict__ partial, int nblk) {
+                                                      const TermGroup* __restrict__ groups,
+                                                      double* __restrict__ partial, int nblk) {
   extern __shared__ uint32_t stab[];
+  __shared__ TermGroup tg;
+  if (threadIdx.x < sizeof(TermGroup) / sizeof(int))
+    ((int*)&tg)[threadIdx.x] = ((const int*)(groups + blockIdx.y))[threadIdx.x];
+  partial += (size_t)blockIdx.y * 2 * TERM_G * nblk;
   ed_load_tables(stab, rt);
   double acc[2 * TERM_G];
 #pragma unroll
@@ -161,32 +166,87 @@ static int mixed_k(const ed_basis* b, const double2* lam, const double2* psi, co
   ed_ctx* ctx = b->ctx;
   const int64_t dim = b->dim;
   const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>((dim + 255) / 256, (int64_t)ctx->num_sms * 2));
-  ED_TRY(ed_ensure_reduce(ctx, (size_t)2 * TERM_G * nblk + 2 * TERM_G + 8));
   size_t smem = (size_t)b->rt.total * sizeof(uint32_t);
   ED_CUDA(cudaFuncSetAttribute(k_expect_mixed<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(56 * 1024)));
-  double* res = ctx->d_red + (size_t)2 * TERM_G * nblk;
-  for (int64_t t0 = 0; t0 < nt; t0 += TERM_G) {
-    TermGroup tg;
-    memset(&tg, 0, sizeof(tg));
-    tg.n = (int)std::min<int64_t>(TERM_G, nt - t0);
-    for (int g = 0; g < tg.n; ++g) {
-      tg.kind[g] = kinds[t0 + g];
-      tg.i[g] = ij[2 * (t0 + g)];
-      tg.j[g] = ij[2 * (t0 + g) + 1];
+  // the groups of 8 terms side by side in one launch (grid.y) and one
+  // read-back: at 13k rows a group alone leaves the device idle and its
+  // launch and read-back cost more than its work (144 terms at N=16: 18
+  // launches and waits, 770 us, before)
+  const int64_t ngroups = (nt + TERM_G - 1) / TERM_G;
+  std::vector<TermGroup> tgs((size_t)ngroups);
+  memset(tgs.data(), 0, sizeof(TermGroup) * tgs.size());
+  for (int64_t t = 0; t < nt; ++t) {
+    TermGroup& tg = tgs[(size_t)(t / TERM_G)];
+    const int g = tg.n++;
+    tg.kind[g] = kinds[t];
+    tg.i[g] = ij[2 * t];
+    tg.j[g] = ij[2 * t + 1];
+  }
+  int64_t step = 256;  // groups per launch: at most 10 MB of scratch
+  for (int64_t g0 = 0; g0 < ngroups;) {
+    const int ng = (int)std::min(step, ngroups - g0);
+    const size_t o_res = ((size_t)sizeof(TermGroup) * ng + 255) & ~(size_t)255;
+    const size_t o_part = o_res + sizeof(double) * 2 * TERM_G * (size_t)ng;
+    ed_workspace ws(ctx, o_part + sizeof(double) * 2 * TERM_G * (size_t)ng * nblk);
+    if (!ws.ptr && step > 1) {
+      step = 1;
+      continue;
     }
-    k_expect_mixed<K><<<nblk, 256, smem, ctx->stream>>>(b->d_states, lam, psi, dim, b->rt, tg, ctx->d_red, nblk);
+    if (!ws.ptr) return ed_fail(ED_ENOMEM, "scratch of the term expectations does not fit in device memory");
+    char* base = (char*)ws.ptr;
+    ED_CUDA(cudaMemcpyAsync(base, tgs.data() + g0, sizeof(TermGroup) * (size_t)ng, cudaMemcpyHostToDevice,
+                            ctx->stream));
+    k_expect_mixed<K><<<dim3(nblk, ng), 256, smem, ctx->stream>>>(b->d_states, lam, psi, dim, b->rt,
+                                                                  (const TermGroup*)base, (double*)(base + o_part),
+                                                                  nblk);
     ED_CHECK_LAUNCH(ctx);
-    k_sum_items<<<2 * TERM_G, 256, 0, ctx->stream>>>(ctx->d_red, nblk, res);
+    k_sum_items<<<2 * TERM_G * ng, 256, 0, ctx->stream>>>((const double*)(base + o_part), nblk,
+                                                          (double*)(base + o_res));
     ED_CHECK_LAUNCH(ctx);
-    ED_CUDA(cudaMemcpyAsync(ctx->h_red, res, sizeof(double) * 2 * TERM_G, cudaMemcpyDeviceToHost, ctx->stream));
+    std::vector<double2> res((size_t)TERM_G * ng);
+    ED_CUDA(cudaMemcpyAsync(res.data(), base + o_res, sizeof(double2) * res.size(), cudaMemcpyDeviceToHost,
+                            ctx->stream));
     ED_CUDA(cudaStreamSynchronize(ctx->stream));
-    for (int g = 0; g < tg.n; ++g) out[t0 + g] = make_double2(ctx->h_red[2 * g], ctx->h_red[2 * g + 1]);
+    const int64_t n = std::min<int64_t>((int64_t)TERM_G * ng, nt - g0 * TERM_G);
+    std::copy(res.begin(), res.begin() + n, out + g0 * TERM_G);
+    g0 += ng;
   }
   return ED_OK;
 }
 
 static int mixed(const ed_basis* b, const double2* lam, const double2* psi, const int* kinds, const int32_t* ij,
                  int64_t nt, double2* out) {
+  {
+    // real vectors (a real H's eigenvectors and adjoint solutions): the S^z
+    // moments and the flip sums of all terms from a few passes (ed_corr.cu):
+    // 144 terms at N=16 in 44 us of kernels against 0.4 ms for the 18 groups
+    // of the general kernel
+    std::vector<int32_t> flips;
+    bool zz = false;
+    for (int64_t t = 0; t < nt; ++t) {
+      const bool same = ij[2 * t] == ij[2 * t + 1];
+      zz |= kinds[t] == T_ZZ || kinds[t] == T_Z || kinds[t] == T_SISJ || same;
+      if ((kinds[t] == T_XY || kinds[t] == T_SISJ) && !same) {
+        flips.push_back(ij[2 * t]);
+        flips.push_back(ij[2 * t + 1]);
+      }
+    }
+    ed_corr c;
+    const int rc = ed_corr_real(b, lam, psi, zz, flips.data(), (int64_t)flips.size() / 2, c);
+    if (rc == ED_OK) {
+      size_t f = 0;
+      for (int64_t t = 0; t < nt; ++t) {
+        const int i = ij[2 * t], j = ij[2 * t + 1];
+        double v = 0.0;
+        if (kinds[t] == T_Z) v = c.sz(i);
+        if (kinds[t] == T_ZZ || kinds[t] == T_SISJ) v = 0.25 * c.zz(i, j);
+        if (kinds[t] == T_XY || kinds[t] == T_SISJ) v += i == j ? 0.5 * c.zz(i, i) : c.F[f++];
+        out[t] = make_double2(v, 0.0);
+      }
+      return ED_OK;
+    }
+    if (rc != ED_ENOMEM && rc != ED_ENOTSUP) return rc;
+  }
   switch (b->rt.K) {
     case 1: return mixed_k<1>(b, lam, psi, kinds, ij, nt, out);
     case 2: return mixed_k<2>(b, lam, psi, kinds, ij, nt, out);
@@ -244,7 +304,7 @@ int ed_grad_energy(const ed_basis* b, const int32_t* pairs_host, int64_t nbonds,
     // a real psi (the solver's eigenvectors): the S^z moments and flip sums of
     // all bonds at once (ed_corr.cu)
     ed_corr c;
-    const int rc = ed_corr_real(b, (const double2*)psi_dev, true, pairs_host, nbonds, c);
+    const int rc = ed_corr_real(b, (const double2*)psi_dev, (const double2*)psi_dev, true, pairs_host, nbonds, c);
     if (rc == ED_OK) {
       const double inv = 1.0 / c.W;
       for (int64_t q = 0; q < nbonds; ++q) {

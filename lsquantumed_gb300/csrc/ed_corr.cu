@@ -28,6 +28,7 @@
 // 10.9 -> 0.34 ms.
 #include "ed_internal.h"
 #include "ed_device.cuh"
+#include "ed_halves.cuh"
 #include "ed_umma.cuh"
 #include <cuda_fp16.h>
 #include <algorithm>
@@ -38,8 +39,6 @@
 namespace {
 
 constexpr int CR_SITES = 32;      // sites padded to 32
-constexpr int CR_MAXW0 = 14;
-constexpr int CR_CLASSES = CR_MAXW0 + 1;
 
 // 128-bit integer accumulators (two 64-bit words, add with carry)
 __device__ __forceinline__ void add128(unsigned long long& lo, unsigned long long& hi, unsigned long long alo,
@@ -71,34 +70,45 @@ __device__ __forceinline__ void fx128(double w, int S, unsigned long long& lo, u
 
 struct CorrHeader {
   double W;        // sum psi_r^2
+  double Wl;       // sum lam_r^2 (two vectors)
   int imag;        // some imaginary part is not zero
   int emax;        // largest biased exponent of a real part
   int nonfinite;   // some part is not finite
   unsigned done;   // blocks finished
   int err;         // a wait of k_corr_gram ran out
-  int pad;
 };
 
-// One pass over psi: the real parts to pr, their sum of squares, largest
-// exponent and the flags.  Four rows in flight per thread; bound by memory
-// (24 bytes per row).  The last block sums the block partials in order.
-__global__ void __launch_bounds__(256) k_corr_prep(const double2* __restrict__ psi, int64_t n, double* __restrict__ pr,
+// One pass over psi (TWO: and lam): the real parts to pr (pl), their sums of
+// squares, psi's largest exponent and the flags.  Four rows in flight per
+// thread; bound by memory (24 bytes per row and vector).  The last block sums
+// the block partials in order.
+template <bool TWO>
+__global__ void __launch_bounds__(256) k_corr_prep(const double2* __restrict__ psi, const double2* __restrict__ lam,
+                                                   int64_t n, double* __restrict__ pr, double* __restrict__ pl,
                                                    CorrHeader* __restrict__ hdr, double* __restrict__ part) {
-  double acc[1] = {0.0};
+  constexpr int NA = TWO ? 2 : 1;
+  double acc[NA];
+#pragma unroll
+  for (int k = 0; k < NA; ++k) acc[k] = 0.0;
   int im = 0, nf = 0, em = 0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t r0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r0 < n; r0 += 4 * stride) {
-    double2 v[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) v[u] = r0 + u * stride < n ? psi[r0 + u * stride] : make_double2(0.0, 0.0);
+    for (int k = 0; k < NA; ++k) {
+      const double2* src = k ? lam : psi;
+      double* dst = k ? pl : pr;
+      double2 v[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      if (r0 + u * stride < n) pr[r0 + u * stride] = v[u].x;
-      const int e = (int)((__double_as_longlong(v[u].x) >> 52) & 0x7FF);
-      em = max(em, e);
-      nf |= e == 0x7FF;
-      im |= v[u].y != 0.0;  // a NaN counts as not zero
-      acc[0] = fma(v[u].x, v[u].x, acc[0]);
+      for (int u = 0; u < 4; ++u) v[u] = r0 + u * stride < n ? src[r0 + u * stride] : make_double2(0.0, 0.0);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (r0 + u * stride < n) dst[r0 + u * stride] = v[u].x;
+        const int e = (int)((__double_as_longlong(v[u].x) >> 52) & 0x7FF);
+        if (k == 0) em = max(em, e);
+        nf |= e == 0x7FF;
+        im |= v[u].y != 0.0;  // a NaN counts as not zero
+        acc[k] = fma(v[u].x, v[u].x, acc[k]);
+      }
     }
   }
   em = (int)__reduce_max_sync(0xffffffffu, (unsigned)em);
@@ -109,61 +119,82 @@ __global__ void __launch_bounds__(256) k_corr_prep(const double2* __restrict__ p
     if (nf) atomicOr(&hdr->nonfinite, 1);
     if (im) atomicOr(&hdr->imag, 1);
   }
-  __shared__ double sh[32];
+  __shared__ double sh[32 * NA];
   __shared__ bool last;
-  ed_block_reduce<1>(acc, sh);
+  ed_block_reduce<NA>(acc, sh);
   if (threadIdx.x == 0) {
-    part[blockIdx.x] = acc[0];
+#pragma unroll
+    for (int k = 0; k < NA; ++k) part[k * gridDim.x + blockIdx.x] = acc[k];
     __threadfence();
     last = atomicAdd(&hdr->done, 1u) == gridDim.x - 1;
   }
   __syncthreads();
   if (!last) return;
   __threadfence();
-  double t[1] = {0.0};
-  for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) t[0] += __ldcg(part + b);
+  double t[NA];
+#pragma unroll
+  for (int k = 0; k < NA; ++k) {
+    t[k] = 0.0;
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) t[k] += __ldcg(part + k * gridDim.x + b);
+  }
   __syncthreads();  // sh free
-  ed_block_reduce<1>(t, sh);
-  if (threadIdx.x == 0) hdr->W = t[0];
+  ed_block_reduce<NA>(t, sh);
+  if (threadIdx.x == 0) {
+    hdr->W = t[0];
+    if (TWO) hdr->Wl = t[NA - 1];
+  }
 }
 
-// Low halves of one popcount and the high halves that go with them.
-struct CorrGeom {
-  int w0, w1, N;
-  int nlow[CR_CLASSES], low_off[CR_CLASSES];    // low halves of popcount k: lows[low_off[k] ..]
-  int nhigh[CR_CLASSES], high_off[CR_CLASSES];  // high halves of popcount nup - k
-  int chunks[CR_CLASSES];                       // pieces of the low halves
-  int prefix[CR_CLASSES + 1];                   // work items of the classes below k
-};
+// The row's weight w = x y as a signed 128-bit integer (y = x with one vector).
+template <bool TWO>
+__device__ __forceinline__ void weight128(double x, double y, int S, unsigned long long& lo, unsigned long long& hi) {
+  if (!TWO) {
+    fx128(x * x, S, lo, hi);
+    return;
+  }
+  const double w = x * y;
+  fx128(fabs(w), S, lo, hi);
+  if (w < 0.0) {
+    lo = ~lo;
+    hi = ~hi;
+    add128(lo, hi, 1ull, 0ull);
+  }
+}
 
 // W0: thread = one low half, loop over a segment of the high halves of its
 // class: 256 consecutive rows per block and high half, so the reads are
 // coalesced; bound by memory.  The 128-bit sum of a segment is added to the
 // table as four 32-bit limbs in 64-bit integers (order does not matter).
-constexpr int COLS_SEG = 64;
-__global__ void __launch_bounds__(256) k_corr_cols(const double* __restrict__ pr, const CorrGeom g,
+constexpr int COLS_SEG = 64;  // most high halves per block
+template <bool TWO>
+__global__ void __launch_bounds__(256) k_corr_cols(const double* __restrict__ pr, const double* __restrict__ pl,
+                                                   const CorrGeom g,
                                                    const uint16_t* __restrict__ lows,
                                                    const uint32_t* __restrict__ highs,
-                                                   const uint32_t* __restrict__ t1, int S,
+                                                   const uint32_t* __restrict__ t1, int S, int nseg,
                                                    unsigned long long* __restrict__ W0) {
   int k = 0;
   while (k < g.w0 && (int)blockIdx.x >= g.prefix[k + 1]) ++k;
   const int item = (int)blockIdx.x - g.prefix[k];
   const int seg = item / g.chunks[k], o = (item - seg * g.chunks[k]) * 256 + (int)threadIdx.x;
-  const int h0 = seg * COLS_SEG, h1 = min(g.nhigh[k], h0 + COLS_SEG);
+  const int h0 = seg * nseg, h1 = min(g.nhigh[k], h0 + nseg);
   __shared__ uint32_t base[COLS_SEG];
   for (int h = h0 + threadIdx.x; h < h1; h += blockDim.x) base[h - h0] = t1[highs[g.high_off[k] + h]];
   __syncthreads();
   if (o >= g.nlow[k]) return;
   unsigned long long lo = 0ull, hi = 0ull;
   for (int h = 0; h < h1 - h0; h += 4) {
-    double x[4];
+    double x[4], y[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) x[u] = h + u < h1 - h0 ? pr[(size_t)base[h + u] + o] : 0.0;
+    for (int u = 0; u < 4; ++u) {
+      const bool on = h + u < h1 - h0;
+      x[u] = on ? pr[(size_t)base[h + u] + o] : 0.0;
+      y[u] = TWO && on ? pl[(size_t)base[h + u] + o] : 0.0;
+    }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       unsigned long long wl, wh;
-      fx128(x[u] * x[u], S, wl, wh);
+      weight128<TWO>(x[u], y[u], S, wl, wh);
       add128(lo, hi, wl, wh);
     }
   }
@@ -171,7 +202,7 @@ __global__ void __launch_bounds__(256) k_corr_cols(const double* __restrict__ pr
   atomicAdd(d, lo & 0xFFFFFFFFull);
   atomicAdd(d + 1, lo >> 32);
   atomicAdd(d + 2, hi & 0xFFFFFFFFull);
-  atomicAdd(d + 3, hi >> 32);
+  atomicAdd(d + 3, (unsigned long long)((long long)hi >> 32));  // signed
 }
 
 // round(v 2^(54 - E)) for |v| < 2^E, E = emax - 1022, plus 128 in each of
@@ -195,8 +226,9 @@ __device__ __forceinline__ unsigned long long gram_entry(double v, int emax) {
 // the low halves with bit i set (i < w0) and over all.  The bit tests and
 // adds of the 14 low sites (four 32-bit adds each) are most of the work.
 // QUANT: each entry is then replaced by its digits for k_corr_gram.
-template <bool QUANT>
-__global__ void __launch_bounds__(128) k_corr_rows(double* __restrict__ pr, int w0, int w1, int nup,
+template <bool QUANT, bool TWO>
+__global__ void __launch_bounds__(128) k_corr_rows(double* __restrict__ pr, const double* __restrict__ pl, int w0,
+                                                   int w1, int nup,
                                                    const CorrGeom g, const uint16_t* __restrict__ lows,
                                                    const uint32_t* __restrict__ t1, int S, int emax,
                                                    ulonglong2* __restrict__ M) {
@@ -214,17 +246,19 @@ __global__ void __launch_bounds__(128) k_corr_rows(double* __restrict__ pr, int 
     const int n = g.nlow[k];
     const uint16_t* lw = lows + g.low_off[k];
     double* p = pr + t1[c1];
-    double xn = lane < n ? p[lane] : 0.0;
+    const double* py = pl + t1[c1];
+    double xn = lane < n ? p[lane] : 0.0, yn = TWO && lane < n ? py[lane] : 0.0;
     uint32_t cn = lane < n ? lw[lane] : 0u;
     for (int o = lane; o < n; o += 32) {
-      const double x = xn;
+      const double x = xn, y = yn;
       const uint32_t c0 = cn;
       if (o + 32 < n) {
         xn = p[o + 32];
+        if (TWO) yn = py[o + 32];
         cn = lw[o + 32];
       }
       unsigned long long wl, wh;
-      fx128(x * x, S, wl, wh);
+      weight128<TWO>(x, y, S, wl, wh);
 #pragma unroll
       for (int i = 0; i < CR_MAXW0; ++i)
         if ((c0 >> i) & 1u) add128(lo[i], hi[i], wl, wh);
@@ -566,13 +600,14 @@ __global__ void __launch_bounds__(256) k_corr_gram_sum(const long long* __restri
   }
 }
 
-// Flip sums of up to CORR_FEW pairs, directly: every antiparallel row is
-// paired with its partner, so only rows with bit i set and bit j clear
+// Flip sums directly, ED_CORR_FEW pairs per pass (grid.y, masks in fm): every
+// antiparallel row is paired with its partner, so only rows with bit i set and bit j clear
 // contribute.  Lane l of a warp serves pair l / 2: a ballot per pair marks
 // the contributing rows among the warp's 32, and the pair's two lanes take
 // alternate marked rows (state, psi and rank halves by shuffle), four
 // gathers in flight each.  A row and pair that contribute nothing cost no FMA
-// and no gather.  partial[g nblk + blk]: flip sum of pair g (FP64).
+// and no gather.  TWO: sum over the same rows of (lam_r psi_r' + lam_r' psi_r)
+// / 2 with lam in pl.  partial[(pass ED_CORR_FEW + g) nblk + blk] (FP64).
 struct FlipMasks {
   int n;
   uint32_t m[ED_CORR_FEW];   // (1 << i) | (1 << j)
@@ -582,11 +617,16 @@ struct FlipMasks {
 };
 
 constexpr int FL_U = 4;
+template <bool TWO>
 __global__ void __launch_bounds__(256, 3) k_expect_flip_r(const uint32_t* __restrict__ states,
-                                                       const double* __restrict__ pr, int64_t dim,
-                                                       const uint16_t* __restrict__ t0,
-                                                       const uint32_t* __restrict__ t1, int w0, const FlipMasks pm,
+                                                       const double* __restrict__ pr, const double* __restrict__ pl,
+                                                       int64_t dim, const uint16_t* __restrict__ t0,
+                                                       const uint32_t* __restrict__ t1, int w0,
+                                                       const FlipMasks* __restrict__ fm,
                                                        double* __restrict__ partial, int nblk) {
+  __shared__ FlipMasks pm;
+  if (threadIdx.x < sizeof(FlipMasks) / 4) ((uint32_t*)&pm)[threadIdx.x] = ((const uint32_t*)(fm + blockIdx.y))[threadIdx.x];
+  partial += (size_t)blockIdx.y * ED_CORR_FEW * nblk;
   extern __shared__ uint16_t t0s[];
   for (int i = threadIdx.x; i < (1 << w0); i += blockDim.x) t0s[i] = t0[i];
   __syncthreads();
@@ -595,33 +635,41 @@ __global__ void __launch_bounds__(256, 3) k_expect_flip_r(const uint32_t* __rest
   const int gl = lane >> 1, par = lane & 1;  // this lane's pair and its turn
   const bool gl_on = gl < pm.n;
   const uint32_t my_m = pm.m[gl], my_ml = pm.ml[gl], my_mh = pm.mh[gl];
+  uint32_t mm[ED_CORR_FEW], mb[ED_CORR_FEW];
+#pragma unroll
+  for (int g = 0; g < ED_CORR_FEW; ++g) {
+    mm[g] = pm.m[g];
+    mb[g] = g < pm.n ? pm.bi[g] : 0xFFFFFFFFu;  // past the list: never met
+  }
   double fl = 0.0;
   const uint32_t low = (1u << w0) - 1u;
   const int64_t step = (((int64_t)gridDim.x * blockDim.x) >> 5) * 32;
   int64_t base = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32;
   uint32_t s_n = 0u;
-  double x_n = 0.0;
+  double x_n = 0.0, y_n = 0.0;
   if (base + lane < dim) {
     s_n = states[base + lane];
     x_n = pr[base + lane];
+    if (TWO) y_n = pl[base + lane];
   }
   for (; base < dim; base += step) {
     const int64_t r = base + lane;
     const bool valid = r < dim;
     const uint32_t s = s_n;
-    const double x = x_n;
+    const double x = x_n, y = y_n;
     s_n = 0u;  // rows past the end: never marked
     x_n = 0.0;
     if (base + step + lane < dim) {
       s_n = states[base + step + lane];
       x_n = pr[base + step + lane];
+      if (TWO) y_n = pl[base + step + lane];
     }
     const uint32_t r0 = valid ? (uint32_t)t0s[s & low] : 0u;  // rank(s) = r0 + T1[s_hi]
     const uint32_t r1 = (uint32_t)r - r0;                    // = T1[s_hi]
     uint32_t L = 0u;
 #pragma unroll
     for (int g = 0; g < ED_CORR_FEW; ++g) {
-      const bool lead = valid && g < pm.n && (s & pm.m[g]) == pm.bi[g];
+      const bool lead = valid && (s & mm[g]) == mb[g];
       const uint32_t bal = __ballot_sync(FULL, lead);
       L = gl == g ? bal : L;
     }
@@ -639,23 +687,25 @@ __global__ void __launch_bounds__(256, 3) k_expect_flip_r(const uint32_t* __rest
         L &= L - 1u;  // taken
         L &= L - 1u;  // the other lane's
       }
-      double xk[FL_U], q[FL_U];
+      double xk[FL_U], q[FL_U], yk[FL_U], ql[FL_U];
 #pragma unroll
       for (int u = 0; u < FL_U; ++u) {
         const uint32_t sk = __shfl_sync(FULL, s, k[u]);
         const uint32_t r0k = __shfl_sync(FULL, r0, k[u]);
         const uint32_t r1k = __shfl_sync(FULL, r1, k[u]);
         xk[u] = __shfl_sync(FULL, x, k[u]);
-        q[u] = 0.0;
+        if (TWO) yk[u] = __shfl_sync(FULL, y, k[u]);
+        q[u] = ql[u] = 0.0;
         if (has[u]) {
           const uint32_t f = sk ^ my_m;
           const uint32_t c = (my_ml ? (uint32_t)t0s[f & low] : r0k) + (my_mh ? __ldg(&t1[f >> w0]) : r1k);
           q[u] = __ldg(&pr[c]);
+          if (TWO) ql[u] = __ldg(&pl[c]);
         }
       }
 #pragma unroll
       for (int u = 0; u < FL_U; ++u)
-        if (has[u]) fl = fma(xk[u], q[u], fl);
+        if (has[u]) fl = TWO ? fma(yk[u], q[u], fma(xk[u], ql[u], fl)) : fma(xk[u], q[u], fl);
     }
   }
   __shared__ double shf[8 * 32];
@@ -665,7 +715,7 @@ __global__ void __launch_bounds__(256, 3) k_expect_flip_r(const uint32_t* __rest
     const int g = threadIdx.x;
     double a = 0.0;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) a += shf[w * 32 + 2 * g] + shf[w * 32 + 2 * g + 1];
-    partial[(size_t)g * nblk + blockIdx.x] = a;
+    partial[(size_t)g * nblk + blockIdx.x] = TWO ? 0.5 * a : a;
   }
 }
 
@@ -688,36 +738,6 @@ double i128_to_double(u128 z) {
   return neg ? -d : d;
 }
 
-// Classes of low halves with popcount k and the high halves of popcount
-// nup - k; items of class k = chunks * per(k).
-template <typename F>
-CorrGeom corr_geom(const ed_basis* b, int nup, int chunk, F per) {
-  CorrGeom g;
-  memset(&g, 0, sizeof(g));
-  g.w0 = b->lin_w0;
-  g.w1 = b->nspins - b->lin_w0;
-  g.N = b->nspins;
-  int lo = 0, n = 0;
-  for (int k = 0; k < CR_CLASSES; ++k) {
-    g.prefix[k] = n;
-    if (k > g.w0) continue;
-    g.nlow[k] = (int)ed_binom(g.w0, k);
-    g.low_off[k] = lo;
-    lo += g.nlow[k];
-    const int h = nup - k;
-    if (h >= 0 && h <= g.w1) {
-      g.nhigh[k] = (int)ed_binom(g.w1, h);
-      int ho = 0;
-      for (int q = 0; q < h; ++q) ho += (int)ed_binom(g.w1, q);
-      g.high_off[k] = ho;
-      g.chunks[k] = (g.nlow[k] + chunk - 1) / chunk;
-      n += g.chunks[k] * per(g.nhigh[k]);
-    }
-  }
-  g.prefix[CR_CLASSES] = n;
-  return g;
-}
-
 }  // namespace
 
 double ed_corr::zz(int i, int j) const {
@@ -732,7 +752,9 @@ double ed_corr::up(int i) const { return i128_to_double(P[i * (i + 1) / 2 + i]) 
 double ed_corr::down(int i) const { return i128_to_double(T - P[i * (i + 1) / 2 + i]) * inv_scale; }
 double ed_corr::sz(int i) const { return 0.5 * (i128_to_double(2 * P[i * (i + 1) / 2 + i] - T) * inv_scale); }
 
-int ed_corr_real(const ed_basis* b, const double2* psi, bool want_zz, const int32_t* pairs, int64_t np, ed_corr& out) {
+int ed_corr_real(const ed_basis* b, const double2* lam, const double2* psi, bool want_zz, const int32_t* pairs,
+                 int64_t np, ed_corr& out) {
+  const bool two = lam != psi;
   ed_ctx* ctx = b->ctx;
   const int64_t dim = b->dim;
   const int N = b->nspins, w0 = b->lin_w0, w1 = N - w0;
@@ -742,12 +764,18 @@ int ed_corr_real(const ed_basis* b, const double2* psi, bool want_zz, const int3
     if (pairs[2 * p] != pairs[2 * p + 1]) flips.push_back(p);
   // up to 16 pairs are one pass of the direct kernel (1.2 ms at N=28, 0.08 ms
   // at N=24); the Gram kernel serves all pairs for 2.5 and 0.2 ms, so it takes
-  // every longer list
-  const bool gram = (int64_t)flips.size() > ED_CORR_FEW;
+  // every longer list.  Two vectors take direct passes.
+  const bool gram = !two && (int64_t)flips.size() > ED_CORR_FEW;
   const bool few = !gram && !flips.empty();
+  const int64_t npass = few ? ((int64_t)flips.size() + ED_CORR_FEW - 1) / ED_CORR_FEW : 0;
+  if (npass > 65535) return ED_ENOTSUP;  // grid.y
   const int nprep = (int)std::max<int64_t>(1, std::min<int64_t>((dim + 1023) / 1024, (int64_t)ctx->num_sms * 8));
   const int nflip = (int)std::max<int64_t>(1, std::min<int64_t>((dim + 255) / 256, (int64_t)ctx->num_sms * 4));
-  const CorrGeom gc = corr_geom(b, b->nup, 256, [](int nh) { return (nh + COLS_SEG - 1) / COLS_SEG; });
+  // long segments where there is work for every SM (fewer table adds), short
+  // ones below, where the chain of loads is what takes time (21 us at N=16
+  // with 64)
+  const int seg = dim < (int64_t)1 << 20 ? 8 : COLS_SEG;
+  const CorrGeom gc = corr_geom(b, b->nup, 256, [seg](int nh) { return (nh + seg - 1) / seg; });
   const CorrGeom gg = corr_geom(b, b->nup - 1, GRAM_STATES, [](int nh) { return nh; });
   const int nstages = gg.prefix[CR_CLASSES];
   const int ncta = std::max(1, std::min(ctx->num_sms, (nstages + GRAM_GROUP - 1) / GRAM_GROUP));
@@ -764,67 +792,76 @@ int ed_corr_real(const ed_basis* b, const double2* psi, bool want_zz, const int3
   const size_t o_zero = at;  // cleared up to here
   const size_t o_P = take(sizeof(ulonglong2) * (size_t)(npairs + 1));
   const size_t o_G = take(sizeof(ulonglong2) * 2048);
-  const size_t o_f = take(sizeof(double) * ED_CORR_FEW);
+  const size_t o_f = take(sizeof(double) * ED_CORR_FEW * (size_t)npass);
   const size_t o_res = at;  // read back: header .. here
-  const size_t o_part = take(sizeof(double) * (size_t)nprep);
+  const size_t o_part = take(sizeof(double) * 2 * (size_t)nprep);
   const size_t o_M = take((sizeof(ulonglong2) * (size_t)(w0 + 1)) << w1);
-  const size_t o_fp = take(few ? sizeof(double) * (size_t)ED_CORR_FEW * nflip : 0);
+  const size_t o_fm = take(sizeof(FlipMasks) * (size_t)npass);
+  const size_t o_fp = take(sizeof(double) * (size_t)ED_CORR_FEW * (size_t)npass * nflip);
   const size_t o_gp = take(gram ? sizeof(long long) * (size_t)GRAM_ACC * ncta : 0);
   const size_t o_pr = take(sizeof(double) * (size_t)dim);
+  const size_t o_pl = take(two ? sizeof(double) * (size_t)dim : 0);
   ed_workspace ws(ctx, at);
   if (!ws.ptr) return ED_ENOMEM;
   char* base = (char*)ws.ptr;
   CorrHeader* hdr = (CorrHeader*)(base + o_hdr);
   double* pr = (double*)(base + o_pr);
+  double* pl = (double*)(base + o_pl);
   ED_CUDA(cudaMemsetAsync(base, 0, o_zero, ctx->stream));
-  k_corr_prep<<<nprep, 256, 0, ctx->stream>>>(psi, dim, pr, hdr, (double*)(base + o_part));
+  if (two) k_corr_prep<true><<<nprep, 256, 0, ctx->stream>>>(psi, lam, dim, pr, pl, hdr, (double*)(base + o_part));
+  else k_corr_prep<false><<<nprep, 256, 0, ctx->stream>>>(psi, psi, dim, pr, pr, hdr, (double*)(base + o_part));
   ED_CHECK_LAUNCH(ctx);
   CorrHeader hh;
   ED_CUDA(cudaMemcpyAsync(&hh, hdr, sizeof(hh), cudaMemcpyDeviceToHost, ctx->stream));
   ED_CUDA(cudaStreamSynchronize(ctx->stream));
   out.real = hh.imag == 0;
-  if (!out.real || hh.nonfinite || !std::isfinite(hh.W)) return ED_ENOTSUP;
+  // sum_r |w_r| <= B < 2^e (two vectors: Cauchy-Schwarz): every w_r and every
+  // integer sum stays below 2^124 at the scale 2^(124 - e) (the rounding of B
+  // moves it by far less than the spare bits)
+  const double B = two ? std::sqrt(hh.W) * std::sqrt(hh.Wl) : hh.W;
+  if (!out.real || hh.nonfinite || !std::isfinite(B)) return ED_ENOTSUP;
   out.N = N;
   out.W = hh.W;
-  // sum_r psi_r^2 = W < 2^e: every w_r and every integer sum stays below
-  // 2^124 at the scale 2^(124 - e) (the rounding of W moves it by far less
-  // than the spare bits)
   int e = 0;
-  if (hh.W > 0.0) std::frexp(hh.W, &e);
+  if (B > 0.0) std::frexp(B, &e);
   const int S = 124 - e;
   out.inv_scale = std::ldexp(1.0, -S);
   if (want_zz) {
-    k_corr_cols<<<gc.prefix[CR_CLASSES], 256, 0, ctx->stream>>>(pr, gc, b->d_lin_lows, b->d_lin_highs, b->d_lin_t1, S,
-                                                               (unsigned long long*)(base + o_W0));
+    auto kern = two ? k_corr_cols<true> : k_corr_cols<false>;
+    kern<<<gc.prefix[CR_CLASSES], 256, 0, ctx->stream>>>(pr, pl, gc, b->d_lin_lows, b->d_lin_highs, b->d_lin_t1, S,
+                                                         seg, (unsigned long long*)(base + o_W0));
     ED_CHECK_LAUNCH(ctx);
   }
   if (few) {
-    FlipMasks pm;
-    memset(&pm, 0, sizeof(pm));
+    std::vector<FlipMasks> fm((size_t)npass);
+    memset(fm.data(), 0, sizeof(FlipMasks) * fm.size());
     const uint32_t low = (1u << w0) - 1u;
-    pm.n = (int)flips.size();
-    for (int g = 0; g < pm.n; ++g) {
-      const int i = pairs[2 * flips[g]], j = pairs[2 * flips[g] + 1];
+    for (size_t t = 0; t < flips.size(); ++t) {
+      FlipMasks& pm = fm[t / ED_CORR_FEW];
+      const int g = pm.n++;
+      const int i = pairs[2 * flips[t]], j = pairs[2 * flips[t] + 1];
       pm.m[g] = (1u << i) | (1u << j);
       pm.bi[g] = 1u << i;
       pm.ml[g] = pm.m[g] & low;
       pm.mh[g] = pm.m[g] >> w0;
     }
+    ED_CUDA(cudaMemcpyAsync(base + o_fm, fm.data(), sizeof(FlipMasks) * fm.size(), cudaMemcpyHostToDevice,
+                            ctx->stream));
     const size_t smem = sizeof(uint16_t) * ((size_t)1 << w0);
-    k_expect_flip_r<<<nflip, 256, smem, ctx->stream>>>(b->d_states, pr, dim, b->d_lin_t0, b->d_lin_t1, w0, pm,
-                                                       (double*)(base + o_fp), nflip);
+    auto kern = two ? k_expect_flip_r<true> : k_expect_flip_r<false>;
+    kern<<<dim3(nflip, (unsigned)npass), 256, smem, ctx->stream>>>(b->d_states, pr, pl, dim, b->d_lin_t0, b->d_lin_t1,
+                                                                   w0, (const FlipMasks*)(base + o_fm),
+                                                                   (double*)(base + o_fp), nflip);
     ED_CHECK_LAUNCH(ctx);
-    k_flip_sum<<<pm.n, 256, 0, ctx->stream>>>((const double*)(base + o_fp), nflip, (double*)(base + o_f));
+    k_flip_sum<<<(unsigned)flips.size(), 256, 0, ctx->stream>>>((const double*)(base + o_fp), nflip,
+                                                               (double*)(base + o_f));
     ED_CHECK_LAUNCH(ctx);
   }
   if (want_zz || gram) {
     const int gr = std::max(1, std::min((1 << w1) / 4, ctx->num_sms * 16));
-    if (gram)
-      k_corr_rows<true><<<gr, 128, 0, ctx->stream>>>(pr, w0, w1, b->nup, gc, b->d_lin_lows, b->d_lin_t1, S, hh.emax,
-                                                     (ulonglong2*)(base + o_M));
-    else
-      k_corr_rows<false><<<gr, 128, 0, ctx->stream>>>(pr, w0, w1, b->nup, gc, b->d_lin_lows, b->d_lin_t1, S, hh.emax,
-                                                      (ulonglong2*)(base + o_M));
+    auto kern = gram ? k_corr_rows<true, false> : two ? k_corr_rows<false, true> : k_corr_rows<false, false>;
+    kern<<<gr, 128, 0, ctx->stream>>>(pr, pl, w0, w1, b->nup, gc, b->d_lin_lows, b->d_lin_t1, S, hh.emax,
+                                      (ulonglong2*)(base + o_M));
     ED_CHECK_LAUNCH(ctx);
   }
   if (want_zz) {

@@ -151,7 +151,10 @@ struct ed_corr {
 };
 // ED_ENOTSUP (out.real tells which) when psi is not real or not finite,
 // ED_ENOMEM when the scratch does not fit.
-int ed_corr_real(const ed_basis* b, const double2* psi, bool want_zz, const int32_t* pairs, int64_t np, ed_corr& out);
+// lam != psi: the mixed sums of two real vectors, w = lam psi and flip sums
+// (lam_r psi_r' + lam_r' psi_r) / 2 (W is then psi's).
+int ed_corr_real(const ed_basis* b, const double2* lam, const double2* psi, bool want_zz, const int32_t* pairs,
+                 int64_t np, ed_corr& out);
 
 struct ed_lin;  // two-table fixed-point H.v state (ed_hv_lin.cu)
 

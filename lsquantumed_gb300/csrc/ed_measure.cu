@@ -9,6 +9,7 @@
 // convention is kept: ExpectVal = sum_s psi_s * conj((O psi)_s).
 #include "ed_internal.h"
 #include "ed_device.cuh"
+#include "ed_halves.cuh"
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -113,9 +114,10 @@ static int expect_g(const ed_basis* b, int op, const double2* psi, const int32_t
   const int64_t dim = b->dim;
   const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>((dim + 255) / 256, (int64_t)ctx->num_sms * 4));
   const int items = REAL ? G : 2 * G;
-  ED_TRY(ed_ensure_reduce(ctx, (size_t)items * nblk + items + 8));
+  const int64_t groups = (np + G - 1) / G;
+  ED_TRY(ed_ensure_reduce(ctx, (size_t)items * nblk + (size_t)items * groups + 8));
   const size_t smem = sizeof(uint16_t) * ((size_t)1 << b->lin_w0);
-  double* out_dev = ctx->d_red + (size_t)items * nblk;
+  double* out_dev = ctx->d_red + (size_t)items * nblk;  // [group][item], one read-back for all
   for (int64_t p0 = 0; p0 < np; p0 += G) {
     PairGroup pg;
     memset(&pg, 0, sizeof(pg));
@@ -127,14 +129,16 @@ static int expect_g(const ed_basis* b, int op, const double2* psi, const int32_t
     k_expect<G, REAL><<<nblk, 256, smem, ctx->stream>>>(b->d_states, psi, dim, b->d_lin_t0, b->d_lin_t1, b->lin_w0, op,
                                                         pg, ctx->d_red, nblk);
     ED_CHECK_LAUNCH(ctx);
-    k_sum_partials<<<items, 256, 0, ctx->stream>>>(ctx->d_red, nblk, items, out_dev);
+    k_sum_partials<<<items, 256, 0, ctx->stream>>>(ctx->d_red, nblk, items, out_dev + p0 / G * items);
     ED_CHECK_LAUNCH(ctx);
-    ED_CUDA(cudaMemcpyAsync(ctx->h_red, out_dev, sizeof(double) * items, cudaMemcpyDeviceToHost, ctx->stream));
-    ED_CUDA(cudaStreamSynchronize(ctx->stream));
-    for (int g = 0; g < pg.n; ++g) {
-      out[p0 + g].x = REAL ? ctx->h_red[g] : ctx->h_red[2 * g];
-      out[p0 + g].y = REAL ? 0.0 : ctx->h_red[2 * g + 1];
-    }
+  }
+  ED_CUDA(cudaMemcpyAsync(ctx->h_red, out_dev, sizeof(double) * (size_t)(items * groups), cudaMemcpyDeviceToHost,
+                          ctx->stream));
+  ED_CUDA(cudaStreamSynchronize(ctx->stream));
+  for (int64_t p = 0; p < np; ++p) {
+    const double* h = ctx->h_red + p / G * items;
+    const int g = (int)(p % G);
+    out[p] = REAL ? make_double2(h[g], 0.0) : make_double2(h[2 * g], h[2 * g + 1]);
   }
   return ED_OK;
 }
@@ -147,7 +151,7 @@ int ed_launch_expect_pairs(const ed_basis* b, int op, const double2* psi, const 
   bool diag = false;
   for (int64_t p = 0; p < np; ++p) diag |= pairs[2 * p] == pairs[2 * p + 1];
   const bool zz = op == ED_OP_SZSZ || op == ED_OP_SISJ || diag;
-  const int rc = ed_corr_real(b, psi, zz, pairs, op == ED_OP_SZSZ ? 0 : np, c);
+  const int rc = ed_corr_real(b, psi, psi, zz, pairs, op == ED_OP_SZSZ ? 0 : np, c);
   if (rc == ED_OK) {
     for (int64_t p = 0; p < np; ++p) {
       const int i = pairs[2 * p], j = pairs[2 * p + 1];
@@ -233,34 +237,373 @@ static int dsf_k(const ed_basis* b0, const ed_basis* b1, int op, const double2* 
                  double2* c_host) {
   ed_ctx* ctx = b0->ctx;
   const int64_t dim0 = b0->dim, dim1 = b1->dim;
-  const int N = b0->nspins;
+  const int N = b0->nspins, groups = (N + MEAS_G - 1) / MEAS_G;
   const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>((dim0 + 255) / 256, (int64_t)ctx->num_sms * 2));
   const int items = 2 * MEAS_G;
-  ED_TRY(ed_ensure_reduce(ctx, (size_t)items * nblk + items + 8));
+  const size_t total = (size_t)items * groups * nev;
+  ED_TRY(ed_ensure_reduce(ctx, (size_t)items * nblk + total + 8));
   size_t smem = op == 1 ? (size_t)b1->rt.total * sizeof(uint32_t) : 0;
   ED_CUDA(cudaFuncSetAttribute(k_dsf<K1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(56 * 1024)));
-  double* out_dev = ctx->d_red + (size_t)items * nblk;
+  double* out_dev = ctx->d_red + (size_t)items * nblk;  // [n][group][item], one read-back for all
   for (int n = 0; n < nev; ++n) {
     const double2* v = vecs + (size_t)n * dim1;
-    for (int i0 = 0; i0 < N; i0 += MEAS_G) {
-      int ni = std::min(MEAS_G, N - i0);
+    for (int q = 0; q < groups; ++q) {
+      const int i0 = q * MEAS_G, ni = std::min(MEAS_G, N - i0);
       k_dsf<K1><<<nblk, 256, smem, ctx->stream>>>(b0->d_states, psi0, dim0, b1->rt, op, i0, ni, v, ctx->d_red, nblk);
       ED_CHECK_LAUNCH(ctx);
-      k_sum_partials<<<items, 256, 0, ctx->stream>>>(ctx->d_red, nblk, items, out_dev);
+      k_sum_partials<<<items, 256, 0, ctx->stream>>>(ctx->d_red, nblk, items,
+                                                     out_dev + ((size_t)n * groups + q) * items);
       ED_CHECK_LAUNCH(ctx);
-      ED_CUDA(cudaMemcpyAsync(ctx->h_red, out_dev, sizeof(double) * items, cudaMemcpyDeviceToHost, ctx->stream));
-      ED_CUDA(cudaStreamSynchronize(ctx->stream));
-      for (int g = 0; g < ni; ++g) {
-        c_host[(size_t)(i0 + g) * nev + n].x = ctx->h_red[2 * g];
-        c_host[(size_t)(i0 + g) * nev + n].y = ctx->h_red[2 * g + 1];
+    }
+  }
+  ED_CUDA(cudaMemcpyAsync(ctx->h_red, out_dev, sizeof(double) * total, cudaMemcpyDeviceToHost, ctx->stream));
+  ED_CUDA(cudaStreamSynchronize(ctx->stream));
+  for (int n = 0; n < nev; ++n)
+    for (int i = 0; i < N; ++i) {
+      const double* h = ctx->h_red + ((size_t)n * groups + i / MEAS_G) * items + 2 * (i % MEAS_G);
+      c_host[(size_t)i * nev + n] = make_double2(h[0], h[1]);
+    }
+  return ED_OK;
+}
+
+// ---------------------------------------------------------------------------
+// The same coefficients from the runs of the two-table rank.  k_dsf spends an
+// FP64 FMA pair per row and site and reads psi and v once per 8 sites.
+// Sqz: sum_r sigma_i(r) q_r, q = conj(v) psi, needs q summed over the low
+// halves of each c1 (high sites) and over the high halves of each c0 (low
+// sites) only: two FP64 FMAs per row of a real v instead of N pairs.
+//  * k_dsfz_high: a warp takes the run of one c1; lane j keeps site w0 + j's
+//    signed sum;
+//  * k_dsfz_low: a thread owns one low half and loops over a segment of the
+//    high halves; the block then forms the signed sums of the low sites.
+// Both take DZ_V vectors at a time, so psi is read once per DZ_V.
+// Real vectors (eigenvectors of the real H) need only the products of the
+// real parts; any nonzero imaginary part raises *imag and the host runs the
+// complex form.  N=24, ten vectors: 3.78 -> 0.38 ms (k_dsfz_high 0.17,
+// k_dsfz_low 0.15; the two reads of the vectors, 0.95 GB, take 0.14).
+// ---------------------------------------------------------------------------
+#define DZ_V 5
+#define DZ_SEG 32
+
+// partial[(((n * gridDim.x) + blk) * 32 + j) * 2]: re, im of site w0 + j
+template <bool REAL>
+__global__ void __launch_bounds__(128) k_dsfz_high(const double2* __restrict__ psi, const double2* __restrict__ vecs,
+                                                   int64_t dim, int nev, int w0, int w1, int nup, const CorrGeom g,
+                                                   const uint32_t* __restrict__ t1, double* __restrict__ partial,
+                                                   int* __restrict__ imag) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int n0 = blockIdx.y * DZ_V, nv = min(DZ_V, nev - n0);
+  const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
+  double hr[DZ_V], hi[DZ_V];
+#pragma unroll
+  for (int v = 0; v < DZ_V; ++v) hr[v] = hi[v] = 0.0;
+  bool im = false;
+  for (int c1 = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); c1 < (1 << w1); c1 += nwarps) {
+    const int k = nup - __popc(c1);
+    if (k < 0 || k > w0) continue;
+    const int n = g.nlow[k];
+    const double2* p = psi + t1[c1];
+    const double2* q = vecs + (size_t)n0 * dim + t1[c1];
+    double ar[DZ_V], ai[DZ_V];
+#pragma unroll
+    for (int v = 0; v < DZ_V; ++v) ar[v] = ai[v] = 0.0;
+#pragma unroll 2
+    for (int o = lane; o < n; o += 32) {
+      const double2 x = p[o];
+      double2 y[DZ_V];
+#pragma unroll
+      for (int v = 0; v < DZ_V; ++v) y[v] = v < nv ? q[(size_t)v * dim + o] : make_double2(0.0, 0.0);
+      if (REAL) im |= x.y != 0.0;
+#pragma unroll
+      for (int v = 0; v < DZ_V; ++v) {
+        if (REAL) {
+          im |= y[v].y != 0.0;
+          ar[v] = fma(y[v].x, x.x, ar[v]);
+        } else {  // conj(v) psi
+          ar[v] = fma(y[v].x, x.x, fma(y[v].y, x.y, ar[v]));
+          ai[v] = fma(y[v].x, x.y, fma(-y[v].y, x.x, ai[v]));
+        }
+      }
+    }
+    const bool up = (c1 >> lane) & 1;
+#pragma unroll
+    for (int v = 0; v < DZ_V; ++v) {
+#pragma unroll
+      for (int s = 16; s > 0; s >>= 1) {
+        ar[v] += __shfl_xor_sync(0xffffffffu, ar[v], s);
+        if (!REAL) ai[v] += __shfl_xor_sync(0xffffffffu, ai[v], s);
+      }
+      hr[v] += up ? ar[v] : -ar[v];
+      if (!REAL) hi[v] += up ? ai[v] : -ai[v];
+    }
+  }
+  __shared__ double sh[2][DZ_V][4][32];
+#pragma unroll
+  for (int v = 0; v < DZ_V; ++v) {
+    sh[0][v][wid][lane] = hr[v];
+    sh[1][v][wid][lane] = hi[v];
+  }
+  if (REAL && __any_sync(0xffffffffu, im) && lane == 0) atomicOr(imag, 1);
+  __syncthreads();
+  for (int v = wid; v < nv; v += 4) {
+    double* d = partial + (((size_t)(n0 + v) * gridDim.x + blockIdx.x) * 32 + lane) * 2;
+    for (int c = 0; c < 2; ++c) d[c] = (sh[c][v][0][lane] + sh[c][v][1][lane]) + (sh[c][v][2][lane] + sh[c][v][3][lane]);
+  }
+}
+
+// partial[(((n * gridDim.x) + item) * 16 + i) * 2]: re, im of low site i
+template <bool REAL>
+__global__ void __launch_bounds__(256) k_dsfz_low(const double2* __restrict__ psi, const double2* __restrict__ vecs,
+                                                  int64_t dim, int nev, const CorrGeom g,
+                                                  const uint16_t* __restrict__ lows,
+                                                  const uint32_t* __restrict__ highs,
+                                                  const uint32_t* __restrict__ t1, double* __restrict__ partial) {
+  int k = 0;
+  while (k < g.w0 && (int)blockIdx.x >= g.prefix[k + 1]) ++k;
+  const int item = (int)blockIdx.x - g.prefix[k];
+  const int seg = item / g.chunks[k], o = (item - seg * g.chunks[k]) * 256 + (int)threadIdx.x;
+  const int h0 = seg * DZ_SEG, nh = min(DZ_SEG, g.nhigh[k] - h0);
+  const int n0 = blockIdx.y * DZ_V, nv = min(DZ_V, nev - n0);
+  __shared__ uint32_t base[DZ_SEG];
+  __shared__ uint16_t c0[256];
+  __shared__ double sh[REAL ? 1 : 2][DZ_V][256];
+  if (threadIdx.x < nh) base[threadIdx.x] = t1[highs[g.high_off[k] + h0 + threadIdx.x]];
+  const bool on = o < g.nlow[k];
+  c0[threadIdx.x] = on ? lows[g.low_off[k] + o] : (uint16_t)0;
+  __syncthreads();
+  double ar[DZ_V], ai[DZ_V];
+#pragma unroll
+  for (int v = 0; v < DZ_V; ++v) ar[v] = ai[v] = 0.0;
+  if (on) {
+    const double2* q = vecs + (size_t)n0 * dim;
+#pragma unroll 2
+    for (int h = 0; h < nh; ++h) {
+      const size_t r = (size_t)base[h] + o;
+      const double2 x = psi[r];
+      double2 y[DZ_V];
+#pragma unroll
+      for (int v = 0; v < DZ_V; ++v) y[v] = v < nv ? q[(size_t)v * dim + r] : make_double2(0.0, 0.0);
+#pragma unroll
+      for (int v = 0; v < DZ_V; ++v) {
+        if (REAL) {
+          ar[v] = fma(y[v].x, x.x, ar[v]);
+        } else {
+          ar[v] = fma(y[v].x, x.x, fma(y[v].y, x.y, ar[v]));
+          ai[v] = fma(y[v].x, x.y, fma(-y[v].y, x.x, ai[v]));
+        }
       }
     }
   }
+#pragma unroll
+  for (int v = 0; v < DZ_V; ++v) {
+    sh[0][v][threadIdx.x] = ar[v];
+    if (!REAL) sh[REAL ? 0 : 1][v][threadIdx.x] = ai[v];
+  }
+  __syncthreads();
+  // 16 threads per site: signed sums of the 256 columns
+  const int i = threadIdx.x >> 4, l = threadIdx.x & 15;
+  for (int v = 0; v < nv; ++v) {
+    double r = 0.0, m = 0.0;
+    for (int c = l; c < 256; c += 16) {
+      const bool up = (c0[c] >> i) & 1;
+      r += up ? sh[0][v][c] : -sh[0][v][c];
+      if (!REAL) m += up ? sh[REAL ? 0 : 1][v][c] : -sh[REAL ? 0 : 1][v][c];
+    }
+#pragma unroll
+    for (int s = 8; s > 0; s >>= 1) {
+      r += __shfl_down_sync(0xffffffffu, r, s, 16);
+      if (!REAL) m += __shfl_down_sync(0xffffffffu, m, s, 16);
+    }
+    if (l == 0) {
+      double* d = partial + (((size_t)(n0 + v) * gridDim.x + blockIdx.x) * 16 + i) * 2;
+      d[0] = r;
+      d[1] = m;
+    }
+  }
+}
+
+// (h, l) + x as an unevaluated pair (Knuth's TwoSum): the signed sums cancel,
+// so the few large partial sums here decide the rounding of the result
+__device__ __forceinline__ void dsf_add(double& h, double& l, double x, double xl) {
+  const double t = __dadd_rn(h, x), z = __dsub_rn(t, h);
+  l = __dadd_rn(l, __dadd_rn(__dadd_rn(__dsub_rn(h, __dsub_rn(t, z)), __dsub_rn(x, z)), xl));
+  h = t;
+}
+
+// c[n * N + i] = f sum over the blocks of site i's partials (low sites in
+// pl, high in ph); grid (sites, vectors)
+__global__ void __launch_bounds__(128) k_dsf_sum(const double* __restrict__ pl, int nl, int wl,
+                                                 const double* __restrict__ ph, int nh, int w0, double f,
+                                                 double2* __restrict__ c) {
+  const int i = blockIdx.x, n = blockIdx.y;
+  const bool low = i < w0;
+  const double* p = low ? pl + ((size_t)n * nl * wl + i) * 2 : ph + ((size_t)n * nh * 32 + (i - w0)) * 2;
+  const int cnt = low ? nl : nh, ld = (low ? wl : 32) * 2;
+  double h[2] = {0.0, 0.0}, l[2] = {0.0, 0.0};
+#pragma unroll 4
+  for (int b = threadIdx.x; b < cnt; b += 128) {
+    const double2 v = *(const double2*)(p + (size_t)b * ld);
+    dsf_add(h[0], l[0], v.x, 0.0);
+    dsf_add(h[1], l[1], v.y, 0.0);
+  }
+  __shared__ double sh[4][4];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+      const double x = __shfl_down_sync(0xffffffffu, h[k], s), xl = __shfl_down_sync(0xffffffffu, l[k], s);
+      dsf_add(h[k], l[k], x, xl);
+    }
+    if ((threadIdx.x & 31) == 0) {
+      sh[threadIdx.x >> 5][2 * k] = h[k];
+      sh[threadIdx.x >> 5][2 * k + 1] = l[k];
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 4; ++w) {
+      dsf_add(h[0], l[0], sh[w][0], sh[w][1]);
+      dsf_add(h[1], l[1], sh[w][2], sh[w][3]);
+    }
+    c[(size_t)n * gridDim.x + i] = make_double2(f * (h[0] + l[0]), f * (h[1] + l[1]));
+  }
+}
+
+// *any = 1 if some entry has a nonzero imaginary part (two arrays)
+__global__ void k_any_imag(const double2* __restrict__ a, int64_t na, const double2* __restrict__ b, int64_t nb,
+                           int* __restrict__ any) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  bool f = false;
+#pragma unroll 4
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < na; i += stride) f |= a[i].y != 0.0;
+#pragma unroll 4
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += stride) f |= b[i].y != 0.0;
+  if (__any_sync(0xffffffffu, f) && (threadIdx.x & 31) == 0) atomicOr(any, 1);
+}
+
+// Sqp for real vectors: a warp takes the run of one c1 of sector 0; every site
+// that is down adds psi v(s + spin i).  A low site's target lies in the run
+// of c1 in sector 1 at T0[c0 + site]; a high site's is the same offset of
+// the run of c1 + site, so consecutive lanes read consecutive entries.  One
+// pass over psi and v for all sites, one FMA per site that is down; grid.y
+// is the vector.  partial[(((n * gridDim.x) + blk) * 32 + site) * 2].
+__global__ void __launch_bounds__(128) k_dsfp_r(const double2* __restrict__ psi, const double2* __restrict__ vecs,
+                                                int64_t dim1, int w0, int w1, int nup, const CorrGeom g,
+                                                const uint16_t* __restrict__ lows, const uint16_t* __restrict__ t0,
+                                                const uint32_t* __restrict__ t1a, const uint32_t* __restrict__ t1b,
+                                                double* __restrict__ partial) {
+  extern __shared__ uint16_t t0s[];
+  for (int i = threadIdx.x; i < (1 << w0); i += blockDim.x) t0s[i] = t0[i];
+  __syncthreads();
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
+  const double2* v = vecs + (size_t)blockIdx.y * dim1;
+  double acc[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) acc[i] = 0.0;
+  for (int c1 = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); c1 < (1 << w1); c1 += nwarps) {
+    const int k = nup - __popc(c1);
+    if (k < 0 || k > w0) continue;
+    const int n = g.nlow[k];
+    const uint16_t* lw = lows + g.low_off[k];
+    const double2* p = psi + t1a[c1];
+    const uint32_t run = t1b[c1];                                             // low sites
+    const uint32_t hrun = lane < w1 ? t1b[c1 | (1 << lane)] : 0u;  // high site `lane`
+    for (int o = lane; o < ((n + 31) & ~31); o += 32) {
+      const bool on = o < n;
+      const double x = on ? p[o].x : 0.0;
+      const uint32_t c0 = on ? lw[o] : 0xFFFFFFFFu;
+#pragma unroll
+      for (int i = 0; i < CR_MAXW0; ++i)
+        if (i < w0 && !((c0 >> i) & 1u)) acc[i] = fma(__ldg(&v[(size_t)run + t0s[c0 | (1u << i)]].x), x, acc[i]);
+#pragma unroll
+      for (int j = 0; j < 32 - CR_MAXW0; ++j) {
+        if (j < w1 && !((c1 >> j) & 1)) {
+          const uint32_t b = __shfl_sync(0xffffffffu, hrun, j);
+          if (on) acc[CR_MAXW0 + j] = fma(__ldg(&v[(size_t)b + o].x), x, acc[CR_MAXW0 + j]);
+        }
+      }
+    }
+  }
+  __shared__ double sh[4][32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    double a = acc[i];
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) a += __shfl_down_sync(0xffffffffu, a, s);
+    if (lane == 0) sh[wid][i] = a;
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    double* d = partial + (((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 32 + lane) * 2;
+    d[0] = (sh[0][lane] + sh[1][lane]) + (sh[2][lane] + sh[3][lane]);
+    d[1] = 0.0;
+  }
+}
+
+// ED_ENOTSUP (nothing returned): some vector is complex and the form asked
+// for is the real one, or a result is not finite; ED_ENOMEM: no scratch.
+template <bool REAL>
+static int dsf_runs(const ed_basis* b0, const ed_basis* b1, int op, const double2* psi, const double2* vecs, int nev,
+                    double2* c_host) {
+  ed_ctx* ctx = b0->ctx;
+  const int N = b0->nspins, w0 = b0->lin_w0, w1 = N - w0;
+  const int nb = std::max(1, std::min((1 << w1) / 4, ctx->num_sms * 8));
+  const CorrGeom g = corr_geom(b0, b0->nup, 256, [](int nh) { return (nh + DZ_SEG - 1) / DZ_SEG; });
+  const int ni = g.prefix[CR_CLASSES];
+  const size_t o_c = 256, o_h = o_c + ((sizeof(double2) * (size_t)N * nev + 255) & ~(size_t)255);
+  const size_t o_l = o_h + sizeof(double2) * 32 * (size_t)nb * nev;
+  ed_workspace ws(ctx, o_l + sizeof(double2) * 16 * (size_t)ni * nev);
+  if (!ws.ptr) return ED_ENOMEM;
+  char* base = (char*)ws.ptr;
+  int* imag = (int*)base;
+  double2* c = (double2*)(base + o_c);
+  double *ph = (double*)(base + o_h), *pl = (double*)(base + o_l);
+  ED_CUDA(cudaMemsetAsync(imag, 0, sizeof(int), ctx->stream));
+  if (op == 0) {
+    const dim3 gh(nb, (nev + DZ_V - 1) / DZ_V), gl(ni, (nev + DZ_V - 1) / DZ_V);
+    k_dsfz_high<REAL><<<gh, 128, 0, ctx->stream>>>(psi, vecs, b0->dim, nev, w0, w1, b0->nup, g, b0->d_lin_t1, ph, imag);
+    ED_CHECK_LAUNCH(ctx);
+    k_dsfz_low<REAL><<<gl, 256, 0, ctx->stream>>>(psi, vecs, b0->dim, nev, g, b0->d_lin_lows, b0->d_lin_highs,
+                                                  b0->d_lin_t1, pl);
+    ED_CHECK_LAUNCH(ctx);
+    k_dsf_sum<<<dim3(N, nev), 128, 0, ctx->stream>>>(pl, ni, 16, ph, nb, w0, 0.5, c);
+  } else {
+    const int64_t n1 = b1->dim * nev;
+    const int gi = (int)std::max<int64_t>(1, std::min<int64_t>((n1 + 1023) / 1024, (int64_t)ctx->num_sms * 8));
+    k_any_imag<<<gi, 256, 0, ctx->stream>>>(psi, b0->dim, vecs, n1, imag);
+    ED_CHECK_LAUNCH(ctx);
+    const size_t smem = sizeof(uint16_t) * ((size_t)1 << w0);
+    k_dsfp_r<<<dim3(nb, nev), 128, smem, ctx->stream>>>(psi, vecs, b1->dim, w0, w1, b0->nup, g, b0->d_lin_lows,
+                                                        b0->d_lin_t0, b0->d_lin_t1, b1->d_lin_t1, ph);
+    ED_CHECK_LAUNCH(ctx);
+    // all sites in ph, low ones at 0 .., high ones at CR_MAXW0 ..
+    k_dsf_sum<<<dim3(N, nev), 128, 0, ctx->stream>>>(ph, nb, 32, ph + 2 * CR_MAXW0, nb, w0, 1.0, c);
+  }
+  ED_CHECK_LAUNCH(ctx);
+  std::vector<char> res(o_h);
+  ED_CUDA(cudaMemcpyAsync(res.data(), base, o_h, cudaMemcpyDeviceToHost, ctx->stream));
+  ED_CUDA(cudaStreamSynchronize(ctx->stream));
+  int h_imag = 0;
+  memcpy(&h_imag, res.data(), sizeof(int));
+  if (REAL && h_imag) return ED_ENOTSUP;
+  const double2* h = (const double2*)(res.data() + o_c);
+  if (REAL)
+    for (int64_t q = 0; q < (int64_t)N * nev; ++q)
+      if (!std::isfinite(h[q].x)) return ED_ENOTSUP;
+  for (int n = 0; n < nev; ++n)
+    for (int i = 0; i < N; ++i) c_host[(size_t)i * nev + n] = h[(size_t)n * N + i];
   return ED_OK;
 }
 
 int ed_launch_dsf(const ed_basis* b0, const ed_basis* b1, int op, const double2* psi0, const double2* vecs, int nev,
                   double2* c_host) {
+  // the real form serves the solver's eigenvectors; a complex vector or a
+  // non-finite entry takes the complex arithmetic
+  const bool fits = nev <= 65535;  // grid.y
+  int rc = fits ? dsf_runs<true>(b0, b1, op, psi0, vecs, nev, c_host) : ED_ENOTSUP;
+  if (rc == ED_ENOTSUP && op == 0 && fits) rc = dsf_runs<false>(b0, b1, op, psi0, vecs, nev, c_host);
+  if (rc != ED_ENOTSUP && rc != ED_ENOMEM) return rc;
   switch (b1->rt.K) {
     case 1: return dsf_k<1>(b0, b1, op, psi0, vecs, nev, c_host);
     case 2: return dsf_k<2>(b0, b1, op, psi0, vecs, nev, c_host);
