@@ -304,6 +304,11 @@ int ed_scale_copy_r(ed_ctx* ctx, const double* src, double* dst, double s, int64
 // ED_RESTART_EXACT (exact slices on the tensor cores, ed_tc.cu; m <= 32).
 int ed_restart_combine_r(ed_ctx* ctx, const double* const* cols, int m, const double* Y, int ldY, int l,
                          double* const* out, int64_t n, int arith = ED_RESTART_FP64);
+// The FP64 form on the tensor cores in exact 10-bit digits (ed_combine.cu);
+// ED_ENOTSUP (nothing launched) for non-finite coefficients.  Does not wait
+// for the device.
+int ed_combine(ed_ctx* ctx, const double* const* cols, int m, const double* Y, int ldY, int l, double* const* out,
+               int64_t n);
 // h_host[i] = V_i^T w (i < nv) on the tensor cores in exact slices
 // (ed_tc.cu); with vj the local step w <- w - a vj - b vjm1 first (written
 // back).  wbound: an upper bound on max |w| after the local step; ED_ENOTSUP

@@ -666,111 +666,26 @@ int ed_scale_copy_r(ed_ctx* ctx, const double* src, double* dst, double s, int64
   return ED_OK;
 }
 
-// out_c = sum_i V_i * Y[i*ldY + c] for real storage.  GB300 runs FP64 FMA
-// at a small fraction of its other rates, and the combination is bound by it
-// (16 x 8 FMAs per element: 32 ms at N=30).  So the eight outputs of a group
-// are split between two arithmetic units that work side by side: columns
-// 0..3 in FP64 FMA, columns 4..7 in exact integer arithmetic.  For those,
-// every column is a unit vector and Y is orthogonal, so |v|, |Y| <= 1: both
-// become 62-bit fixed point (v in registers, Y on the host), each product is
-// exact in 128 bits (__mul64hi and the low word), each sum is exact (by
-// Cauchy-Schwarz it stays below sqrt(m), far inside 128 bits) and each output
-// is rounded once.  Measured at N=30: 23 ms against 32 ms for all-FP64 and
-// 32 ms for all-integer.  A non-finite input makes its row's integer
-// outputs NaN, as the FP64 ones become.
-__device__ __forceinline__ long long ed_fx62(double v, bool& bad) {
-  const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
-  const int e = (int)((bits >> 52) & 0x7FF);
-  if (e == 0x7FF) { bad = true; return 0; }
-  if (e == 0) return 0;  // |v| < 2^-1022
-  const unsigned long long mant = (bits & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
-  const int sh = e - 1013;  // v * 2^62 = mant * 2^(e - 1023 - 52 + 62)
-  unsigned long long a;
-  if (sh >= 0) a = mant << sh;  // |v| <= 1: sh <= 10, a <= 2^62
-  else if (sh > -63) a = (mant + (1ull << (-sh - 1))) >> (-sh);
-  else a = 0;
-  return (bits >> 63) ? -(long long)a : (long long)a;
-}
-
-// NF outputs of a group in FP64 and the next NI in integers (NF + NI <= 8).
-// A full group of eight takes 4 + 4, which keeps both units busy (3 + 5 and
-// 4 + 4 measured the same; 2 + 6 and fewer FP64 outputs were slower).  A
-// partial last group computes only the outputs it stores: one or two in FP64
-// alone (an integer output of its own would pay the conversion of every input
-// for one product), three or more split as evenly as the FP64 side allows.
-template <int NF, int NI>
-__global__ void __launch_bounds__(256) k_restart_mix(const ColPtrsR cp, int m, const double* __restrict__ Yd,
-                                                     const long long* __restrict__ Yq, int c0,
-                                                     const ColPtrs outp, int64_t n) {
-  static_assert(NF >= 1 && NI >= 0 && NF + NI <= 8, "group of at most eight outputs");
-  __shared__ double shY[128 * 8];     // m x 8 coefficients of this group (FP64 columns)
-  __shared__ long long shQ[128 * 8];  // the same, 62-bit fixed point (integer columns)
-  for (int k = threadIdx.x; k < m * 8; k += blockDim.x) {
-    shY[k] = Yd[k];
-    shQ[k] = Yq[k];
-  }
+// out_c = sum_i V_i Y[i][c] in FP64 FMAs, eight outputs per launch: what
+// non-finite coefficients take (ed_combine.cu serves the others).
+__global__ void __launch_bounds__(256) k_restart_r(const ColPtrsR cp, int m, const double* __restrict__ Y, int c0, int nc,
+                                                   const ColPtrs outp, int64_t n) {
+  __shared__ double shY[128 * 8];
+  for (int k = threadIdx.x; k < m * 8; k += blockDim.x) shY[k] = Y[k];
   __syncthreads();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += stride) {
-    double a[NF];
-    unsigned long long lo[NI > 0 ? NI : 1];
-    long long hi[NI > 0 ? NI : 1];
+    double a[8];
 #pragma unroll
-    for (int c = 0; c < NF; ++c) a[c] = 0.0;
-#pragma unroll
-    for (int c = 0; c < NI; ++c) { lo[c] = 0ull; hi[c] = 0ll; }
-    bool bad = false;
+    for (int c = 0; c < 8; ++c) a[c] = 0.0;
     for (int i = 0; i < m; ++i) {
-      const double vd = cp.p[i][r];
+      const double v = cp.p[i][r];
 #pragma unroll
-      for (int c = 0; c < NF; ++c) a[c] = fma(vd, shY[i * 8 + c], a[c]);
-      if (NI > 0) {
-        const long long v = ed_fx62(vd, bad);
-#pragma unroll
-        for (int c = 0; c < NI; ++c) {
-          const long long y = shQ[i * 8 + NF + c];
-          const unsigned long long pl = (unsigned long long)v * (unsigned long long)y;
-          const long long ph = __mul64hi(v, y);
-          const unsigned long long s = lo[c] + pl;
-          hi[c] += ph + (s < pl ? 1 : 0);
-          lo[c] = s;
-        }
-      }
+      for (int c = 0; c < 8; ++c) a[c] = fma(v, shY[i * 8 + c], a[c]);
     }
 #pragma unroll
-    for (int c = 0; c < NF; ++c) ((double*)outp.p[c0 + c])[r] = a[c];
-#pragma unroll
-    for (int c = 0; c < NI; ++c) {
-      // (hi * 2^64 + lo) * 2^-124
-      double d = fma((double)hi[c], 0x1p-60, (double)lo[c] * 0x1p-124);
-      if (bad) d = __longlong_as_double(0x7FF8000000000000ll);
-      ((double*)outp.p[c0 + NF + c])[r] = d;
-    }
-  }
-}
-
-// One group of nc outputs (1..8) with the split above.
-static int restart_mix_launch(ed_ctx* ctx, const ColPtrsR& cp, int m, const double* dYd, const long long* dYq, int c0,
-                              int nc, const ColPtrs& op, int64_t n) {
-  auto go = [&](auto kern) -> int {
-    int per_sm = 0;
-    ED_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, 0));
-    if (per_sm < 1) per_sm = 1;
-    const int g = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)ctx->num_sms * per_sm));
-    kern<<<g, 256, 0, ctx->stream>>>(cp, m, dYd, dYq, c0, op, n);
-    ED_CHECK_LAUNCH(ctx);
-    return ED_OK;
-  };
-  switch (nc) {
-    case 1: return go(k_restart_mix<1, 0>);
-    case 2: return go(k_restart_mix<2, 0>);
-    case 3: return go(k_restart_mix<2, 1>);
-    case 4: return go(k_restart_mix<2, 2>);
-    case 5: return go(k_restart_mix<3, 2>);
-    case 6: return go(k_restart_mix<3, 3>);
-    case 7: return go(k_restart_mix<4, 3>);
-    case 8: return go(k_restart_mix<4, 4>);
-    default: return ed_fail(ED_EINVAL, "restart group of " + std::to_string(nc) + " outputs");
+    for (int c = 0; c < 8; ++c)
+      if (c < nc) ((double*)outp.p[c0 + c])[r] = a[c];
   }
 }
 
@@ -995,6 +910,10 @@ int ed_restart_combine_r(ed_ctx* ctx, const double* const* cols, int m, const do
                          double* const* out, int64_t n, int arith) {
   if (m > 127) return ed_fail(ED_ENOTSUP, "at most 127 basis vectors");
   if (arith == ED_RESTART_EXACT) return ed_restart_combine_tc(ctx, cols, m, Y, ldY, l, out, n);
+  if (arith == ED_RESTART_FP64) {
+    const int rc = ed_combine(ctx, cols, m, Y, ldY, l, out, n);
+    if (rc != ED_ENOTSUP) return rc;
+  }
   const bool pair = arith == ED_RESTART_PAIR;
   ColPtrsR cp = make_cols_r(cols, m);
   ColPtrs op;
@@ -1027,26 +946,19 @@ int ed_restart_combine_r(ed_ctx* ctx, const double* const* cols, int m, const do
     ED_CUDA(cudaStreamSynchronize(ctx->stream));
     return ED_OK;
   }
-  // coefficients per group of 8 outputs, [group][i][8]: FP64 and 62-bit fixed point
+  // coefficients per group of 8 outputs, [group][i][8]
   std::vector<double> yd(ngroups * per, 0.0);
-  std::vector<long long> yq(ngroups * per, 0);
   for (int gi = 0; gi < ngroups; ++gi)
     for (int i = 0; i < m; ++i)
-      for (int c = 0; c < 8; ++c) {
-        const int col = gi * 8 + c;
-        if (col >= l) continue;
-        const double y = Y[(size_t)i * ldY + col];
-        yd[(gi * m + i) * 8 + c] = y;
-        yq[(gi * m + i) * 8 + c] = std::llround(std::ldexp(y, 62));
-      }
-  ED_TRY(ed_ensure_reduce(ctx, 2 * ngroups * per + 16));
-  double* dYd = ctx->d_red;
-  long long* dYq = (long long*)(ctx->d_red + ngroups * per);
-  ED_CUDA(cudaMemcpyAsync(dYd, yd.data(), sizeof(double) * yd.size(), cudaMemcpyHostToDevice, ctx->stream));
-  ED_CUDA(cudaMemcpyAsync(dYq, yq.data(), sizeof(long long) * yq.size(), cudaMemcpyHostToDevice, ctx->stream));
-  for (int gi = 0; gi < ngroups; ++gi)
-    ED_TRY(restart_mix_launch(ctx, cp, m, dYd + gi * per, dYq + gi * per, gi * 8, std::min(8, l - gi * 8), op, n));
-  // the host coefficients must outlive the copies
+      for (int c = 0; c < 8 && gi * 8 + c < l; ++c) yd[(gi * m + i) * 8 + c] = Y[(size_t)i * ldY + gi * 8 + c];
+  ED_TRY(ed_ensure_reduce(ctx, ngroups * per + 16));
+  ED_CUDA(cudaMemcpyAsync(ctx->d_red, yd.data(), sizeof(double) * yd.size(), cudaMemcpyHostToDevice, ctx->stream));
+  const int g = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)ctx->num_sms * 4));
+  for (int gi = 0; gi < ngroups; ++gi) {
+    k_restart_r<<<g, 256, 0, ctx->stream>>>(cp, m, ctx->d_red + gi * per, gi * 8, std::min(8, l - gi * 8), op, n);
+    ED_CHECK_LAUNCH(ctx);
+  }
+  // the host coefficients must outlive the copy
   ED_CUDA(cudaStreamSynchronize(ctx->stream));
   return ED_OK;
 }
