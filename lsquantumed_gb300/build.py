@@ -18,7 +18,7 @@ BUILD = os.path.join(ROOT, '_build', 'edgb300')
 LIBDIR = os.path.join(HERE, '_lib')
 LIB = os.path.join(LIBDIR, 'libedgb300.so')
 
-SOURCES = ['ed_capi.cu', 'ed_basis.cu', 'ed_hamiltonian.cu', 'ed_linalg.cu', 'ed_eps.cu', 'ed_measure.cu', 'ed_corr.cu', 'ed_combine.cu',
+SOURCES = ['ed_capi.cu', 'ed_basis.cu', 'ed_hamiltonian.cu', 'ed_linalg.cu', 'ed_eps.cu', 'ed_measure.cu', 'ed_corr.cu', 'ed_combine.cu', 'ed_krylov.cu',
            'ed_batch.cu', 'ed_adjoint.cu', 'ed_hv_lin.cu',
            'ed_spectrum.cu', 'ed_hv_jit.cu', 'ed_peaks.cu', 'ed_tc.cu']
 ARCH = ['-gencode', 'arch=compute_103a,code=sm_103a']

@@ -122,6 +122,7 @@ int ed_ctx_destroy(ed_ctx* c) {
   if (c->d_red) cudaFree(c->d_red);
   if (c->h_red) cudaFreeHost(c->h_red);
   if (c->ws) cudaFree(c->ws);
+  if (c->d_counter) cudaFree(c->d_counter);
   if (c->own_stream) cudaStreamDestroy(c->stream);
   delete c;
   return ED_OK;

@@ -74,6 +74,27 @@ __device__ __forceinline__ uint32_t ed_rank_flip(uint32_t r, uint32_t s, const u
   return rr;
 }
 
+// One entry in 64-bit fixed point: v * 2^(sbits - 1 - (emax - 1023)) rounded,
+// or the non-finite sentinel.
+__device__ __forceinline__ long long ed_fx64_entry(double v, int emax, int sbits) {
+  const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
+  const int e = (int)((bits >> 52) & 0x7FF);
+  long long m = 0;
+  if (e == 0x7FF) {
+    m = (long long)0x8000000000000000ull;  // non-finite sentinel
+  } else if (e != 0) {
+    const unsigned long long mant = (bits & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
+    const int sh = e - emax + sbits - 53;
+    unsigned long long a;
+    if (sh >= 0) a = mant << sh;
+    else if (sh > -63) a = (mant + (1ull << (-sh - 1))) >> (-sh);  // round half up in magnitude
+    else a = 0;
+    m = (long long)a;
+    if (bits >> 63) m = -m;
+  }
+  return m;
+}
+
 // Counter-based splitmix64 (deterministic, identical on host and device).
 __device__ __forceinline__ uint64_t ed_splitmix64(uint64_t z) {
   z += 0x9E3779B97F4A7C15ull;
@@ -132,6 +153,19 @@ __device__ __forceinline__ void ed_block_max(double& v, double* sh) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
   }
+}
+
+// The last block of the grid to get here; all threads of every block call it
+// after their block's result is written.  The counter is zero before and after
+// the launch.
+__device__ __forceinline__ bool ed_last_block(unsigned* counter) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicInc(counter, gridDim.x - 1) == gridDim.x - 1;
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
 }
 
 // Load the rank tables into shared memory (block-cooperative).

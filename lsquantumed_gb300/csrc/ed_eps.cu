@@ -101,7 +101,6 @@ static void eps_free(ed_eps* e) {
   if (e->pool) cudaFree(e->pool);
   if (e->w) cudaFree(e->w);
   if (e->pool_r) cudaFree(e->pool_r);
-  if (e->w_r) cudaFree(e->w_r);
   e->pool = nullptr;
   e->w = nullptr;
   e->pool_r = nullptr;
@@ -278,6 +277,88 @@ static int orthogonalize_r(ed_eps* e, int j, double* nw) {
   return ED_OK;
 }
 
+// The end of step j once w is orthogonal to the basis: the next column (w
+// scaled, with its fixed-point copy for the next H.v, or a random vector where
+// the subspace is invariant) and beta_j.
+static int close_step_r(ed_eps* e, int j, int m, double nw, double norig, double wmax, std::vector<double>& beta,
+                        uint64_t* rseed) {
+  ed_ham* H = e->h;
+  ed_ctx* ctx = H->ctx;
+  const int64_t n = H->basis->dim;
+  if (nw <= 1e-13 * norig) {
+    // invariant subspace: continue with a (real) random vector orthogonal to V
+    beta[j] = 0.0;
+    if (j + 1 < m) {
+      ED_TRY(ed_start_vector_r(ctx, (*rseed)++, n, e->w_r));
+      double nw2 = 0.0;
+      ED_TRY(orthogonalize_r(e, j, &nw2));
+      ED_TRY(ed_scale_copy_r(ctx, e->w_r, e->col_r[j + 1], 1.0 / nw2, n));
+    } else {
+      ED_CUDA(cudaMemsetAsync(e->col_r[j + 1], 0, sizeof(double) * (size_t)n, ctx->stream));
+    }
+    H->xq_src = nullptr;
+    return ED_OK;
+  }
+  // the next H.v's input is this vector: its fixed-point copy is made in the
+  // same pass (bit-identical to quantizing it afterwards)
+  const int rq = ed_scale_quantize_r(H, e->w_r, e->col_r[j + 1], 1.0 / nw, wmax);
+  if (rq == ED_ENOTSUP) {
+    H->xq_src = nullptr;
+    ED_TRY(ed_scale_copy_r(ctx, e->w_r, e->col_r[j + 1], 1.0 / nw, n));
+  } else if (rq != ED_OK) {
+    return rq;
+  }
+  beta[j] = nw;
+  return ED_OK;
+}
+
+// Steps k .. m - 1 with the coefficients on the device (ed_krylov.cu): all
+// queued at once, one wait at the end.  A step that needs the host (a
+// refinement pass, an invariant subspace, an undetermined exponent) stops the
+// queue; it is finished here and the rest queued again.
+static int expand_queued(ed_eps* e, KrState* st, int k, int m, std::vector<double>& alpha, std::vector<double>& beta,
+                         uint64_t* rseed) {
+  ed_ham* H = e->h;
+  ed_ctx* ctx = H->ctx;
+  const int64_t n = H->basis->dim;
+  std::vector<double> c;
+  for (int j0 = k; j0 < m;) {
+    for (int j = j0; j < m; ++j) ED_TRY(ed_kr_step(H, e->col_r.data(), j, j > k && j > 0, e->w_r, st));
+    KrState* hs = (KrState*)ctx->h_red;  // at least 64 Ki doubles
+    ED_CUDA(cudaMemcpyAsync(hs, st, sizeof(KrState), cudaMemcpyDeviceToHost, ctx->stream));
+    ED_CUDA(cudaStreamSynchronize(ctx->stream));
+    const KrState s = *hs;
+    const int last = s.stop == KR_RUN ? m - 1 : s.step;
+    for (int j = j0; j <= last; ++j) {
+      alpha[j] = s.alpha[j];
+      beta[j] = s.beta[j];
+      e->nhv++;
+      e->ortho_passes++;
+    }
+    j0 = last + 1;
+    if (s.stop == KR_RUN) continue;
+    const int j = last;
+    H->xq_src = nullptr;  // the queue made no copy for the steps behind
+    ED_CUDA(cudaMemsetAsync(&st->stop, 0, sizeof(int), ctx->stream));
+    ED_CUDA(cudaMemsetAsync(H->d_gmax + ED_HV_SKIP, 0, sizeof(int), ctx->stream));
+    double nw = s.beta[j], wmax = s.wmax;
+    if (s.stop == KR_REFINE) {  // the second pass (DGKS)
+      std::vector<const double*> cols(e->col_r.begin(), e->col_r.begin() + j + 1);
+      c.assign(j + 1, 0.0);
+      double n2 = 0.0;
+      ED_TRY(ed_multidot_r(ctx, cols.data(), j + 1, e->w_r, n, nullptr, 0.0, nullptr, 0.0, c.data(), nullptr));
+      ED_TRY(ed_update_r(ctx, cols.data(), j + 1, c.data(), e->w_r, n, &n2, &wmax, e->restart_mode));
+      alpha[j] += c[j];
+      nw = std::sqrt(n2);
+      e->ortho_passes++;
+    }
+    ED_TRY(close_step_r(e, j, m, nw, std::sqrt(s.y2), wmax, beta, rseed));
+    if (j + 1 < m)  // the next step's local projection reads it
+      ED_CUDA(cudaMemcpyAsync(&st->beta[j], &beta[j], sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+  }
+  return ED_OK;
+}
+
 static int eps_solve_real(ed_eps* e, int* nconv_out, int m, int nev, double tol, int max_it) {
   ed_ham* H = e->h;
   ed_ctx* ctx = H->ctx;
@@ -288,18 +369,25 @@ static int eps_solve_real(ed_eps* e, int* nconv_out, int m, int nev, double tol,
   if (e->restart_mode == ED_RESTART_EXACT && m > 32)
     return ed_fail(ED_ENOTSUP, "the exact tensor-core restart takes at most 32 basis vectors (ncv <= 32)");
   e->pool_cols = 2 * m + 1;
-  if (cudaMalloc(&e->pool_r, sizeof(double) * (size_t)n * e->pool_cols) != cudaSuccess ||
-      cudaMalloc(&e->w_r, sizeof(double) * (size_t)n) != cudaSuccess) {
+  // columns a multiple of 128 bytes apart (16-byte loads of row pairs), the
+  // work vector and the device state behind them
+  const int64_t ld = (n + 15) & ~(int64_t)15;
+  if (cudaMalloc(&e->pool_r, sizeof(double) * (size_t)ld * (e->pool_cols + 1) + sizeof(KrState)) != cudaSuccess) {
     cudaGetLastError();
     eps_free(e);
     return ed_fail(ED_ENOMEM, "Krylov basis does not fit in device memory");
   }
+  e->w_r = e->pool_r + (size_t)e->pool_cols * ld;
+  KrState* d_state = (KrState*)(e->w_r + ld);
+  ED_CUDA(cudaMemsetAsync(d_state, 0, sizeof(KrState), ctx->stream));
+  // the exact and fixed-point arithmetics take their own projections, step by step
+  const bool queued = e->restart_mode == ED_RESTART_FP64 || e->restart_mode == ED_RESTART_PAIR;
   e->real_storage = true;
   e->real_coeffs = true;
   std::vector<double*> freelist;
   e->col_r.assign(m + 1, nullptr);
   for (int i = 0; i < e->pool_cols; ++i) {
-    double* p = e->pool_r + (size_t)i * n;
+    double* p = e->pool_r + (size_t)i * ld;
     if (i <= m) e->col_r[i] = p; else freelist.push_back(p);
   }
   std::vector<double> alpha(m + 1, 0.0), beta(m + 1, 0.0), arrow(m + 1, 0.0);
@@ -318,32 +406,18 @@ static int eps_solve_real(ed_eps* e, int* nconv_out, int m, int nev, double tol,
   bool done = false;
   while (!done) {
     ++its;
-    for (int j = k; j < m; ++j) {
-      double2 pre_a;
-      double pre_y2 = 0.0;
-      ED_TRY(ed_launch_hv_dot_any(H, e->col_r[j], e->w_r, true, &pre_a, &pre_y2));
-      e->nhv++;
-      double nw = 0.0, norig = 0.0, wmax = 0.0;
-      ED_TRY(orthogonalize_lanczos_r(e, j, k, j > 0 ? beta[j - 1] : 0.0, pre_a.x, pre_y2, h, &nw, &norig, &wmax));
-      alpha[j] = h[j];
-      if (nw <= 1e-13 * norig) {
-        // invariant subspace: continue with a (real) random vector orthogonal to V
-        beta[j] = 0.0;
-        if (j + 1 < m) {
-          ED_TRY(ed_start_vector_r(ctx, rseed++, n, e->w_r));
-          double nw2 = 0.0;
-          ED_TRY(orthogonalize_r(e, j, &nw2));
-          ED_TRY(ed_scale_copy_r(ctx, e->w_r, e->col_r[j + 1], 1.0 / nw2, n));
-        } else {
-          ED_CUDA(cudaMemsetAsync(e->col_r[j + 1], 0, sizeof(double) * (size_t)n, ctx->stream));
-        }
-      } else {
-        // the next H.v's input is this vector: its fixed-point copy is made in
-        // the same pass (bit-identical to quantizing it afterwards)
-        const int rq = ed_scale_quantize_r(H, e->w_r, e->col_r[j + 1], 1.0 / nw, wmax);
-        if (rq == ED_ENOTSUP) ED_TRY(ed_scale_copy_r(ctx, e->w_r, e->col_r[j + 1], 1.0 / nw, n));
-        else if (rq != ED_OK) return rq;
-        beta[j] = nw;
+    if (queued) {
+      ED_TRY(expand_queued(e, d_state, k, m, alpha, beta, &rseed));
+    } else {
+      for (int j = k; j < m; ++j) {
+        double2 pre_a;
+        double pre_y2 = 0.0;
+        ED_TRY(ed_launch_hv_dot_any(H, e->col_r[j], e->w_r, true, &pre_a, &pre_y2));
+        e->nhv++;
+        double nw = 0.0, norig = 0.0, wmax = 0.0;
+        ED_TRY(orthogonalize_lanczos_r(e, j, k, j > 0 ? beta[j - 1] : 0.0, pre_a.x, pre_y2, h, &nw, &norig, &wmax));
+        alpha[j] = h[j];
+        ED_TRY(close_step_r(e, j, m, nw, norig, wmax, beta, &rseed));
       }
     }
     std::vector<double> T((size_t)m * m, 0.0);

@@ -588,10 +588,11 @@ static int ensure_fixed_buffers(ed_ham* h) {
   if (!h->d_xq) {
     if (cudaMalloc(&h->d_xq, sizeof(longlong2) * (size_t)dim) != cudaSuccess ||
         cudaMalloc(&h->d_xe, sizeof(uint16_t) * (size_t)((dim + 31) / 32)) != cudaSuccess ||
-        cudaMalloc(&h->d_gmax, 4 * sizeof(int)) != cudaSuccess) {
+        cudaMalloc(&h->d_gmax, ED_GMAX_BYTES) != cudaSuccess) {
       cudaGetLastError();
       return ed_fail(ED_ENOMEM, "H.v scratch does not fit in device memory");
     }
+    ED_CUDA(cudaMemsetAsync(h->d_gmax, 0, ED_GMAX_BYTES, h->ctx->stream));
   }
   return ED_OK;
 }
@@ -644,27 +645,6 @@ __global__ void __launch_bounds__(256) k_max_exponent_r(const double* __restrict
     if (m > 0) atomicMax(gmax, m);
     if (nf) atomicOr(nonfinite, 1);
   }
-}
-
-// One entry in 64-bit fixed point: v * 2^(sbits - 1 - (emax - 1023)) rounded,
-// or the non-finite sentinel.
-__device__ __forceinline__ long long ed_fx64_entry(double v, int emax, int sbits) {
-  const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
-  const int e = (int)((bits >> 52) & 0x7FF);
-  long long m = 0;
-  if (e == 0x7FF) {
-    m = (long long)0x8000000000000000ull;  // non-finite sentinel
-  } else if (e != 0) {
-    const unsigned long long mant = (bits & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
-    const int sh = e - emax + sbits - 53;
-    unsigned long long a;
-    if (sh >= 0) a = mant << sh;
-    else if (sh > -63) a = (mant + (1ull << (-sh - 1))) >> (-sh);  // round half up in magnitude
-    else a = 0;
-    m = (long long)a;
-    if (bits >> 63) m = -m;
-  }
-  return m;
 }
 
 __global__ void __launch_bounds__(256) k_quantize64_r(const double* __restrict__ x, int64_t dim,
@@ -813,9 +793,8 @@ int ed_launch_hv_dot(ed_ham* h, const double2* x, double2* y, double2* dot, doub
   return ed_launch_hv_dot_any(h, x, y, false, dot, y2);
 }
 
-int ed_launch_hv_dot_any(ed_ham* h, const void* x, void* y, bool rio, double2* dot, double* y2) {
+static int launch_hv_dot(ed_ham* h, const void* x, void* y, bool rio) {
   ed_ctx* ctx = h->ctx;
-  if (!ed_lin_supported(h)) return ED_ENOTSUP;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (ctx->profiling) {
     ED_CUDA(cudaEventCreate(&e0));
@@ -829,8 +808,24 @@ int ed_launch_hv_dot_any(ed_ham* h, const void* x, void* y, bool rio, double2* d
     ctx->prof_events.push_back(e0);
     ctx->prof_events.push_back(e1);
   }
-  double out[3];
-  ED_TRY(ed_finish_reduce(ctx, 3, nblk, out));
+  return ED_OK;
+}
+
+int ed_launch_hv_dot_dev(ed_ham* h, const double* x, double* y, const double** sums) {
+  if (!ed_lin_supported(h)) return ED_ENOTSUP;
+  ED_TRY(launch_hv_dot(h, x, y, true));
+  *sums = (const double*)(h->d_gmax + ED_HV_SUMS);
+  return ED_OK;
+}
+
+int ed_launch_hv_dot_any(ed_ham* h, const void* x, void* y, bool rio, double2* dot, double* y2) {
+  ed_ctx* ctx = h->ctx;
+  if (!ed_lin_supported(h)) return ED_ENOTSUP;
+  ED_TRY(launch_hv_dot(h, x, y, rio));
+  // the last block of the H.v left the sums
+  double* out = ctx->h_red;
+  ED_CUDA(cudaMemcpyAsync(out, h->d_gmax + ED_HV_SUMS, 3 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  ED_CUDA(cudaStreamSynchronize(ctx->stream));
   dot->x = out[0];
   dot->y = out[1];
   if (y2) *y2 = out[2];

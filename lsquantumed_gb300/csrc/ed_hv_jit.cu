@@ -115,6 +115,22 @@ struct alignas(16) L2 { i64 x, y; };
 // meet in one bank.  T0[c ^ m] = t0s[SWZ(c) ^ SWZ(m)]: one XOR per row, and
 // SWZ(m) is each bond's immediate.
 #define SWZ(i) ((i) ^ ((((i) >> 6) & 31u) << 1))
+// The last block sums the block partials of the fused dot in order and leaves
+// the three sums after the flags (counter at gmax_p[4], sums from int 16).
+__device__ __forceinline__ void finish(const double* partial, int* gmax_p) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicInc((u32*)gmax_p + 4, gridDim.x - 1) == gridDim.x - 1;
+  __syncthreads();
+  if (!last || threadIdx.x >= 96) return;
+  __threadfence();
+  const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double a = 0.0;
+  for (u32 b = lane; b < gridDim.x; b += 32) a += __ldcg(partial + k * gridDim.x + b);
+  for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+  if (lane == 0) ((double*)(gmax_p + 16))[k] = a;
+}
 // element of the fixed-point input: real parts only (RX) or (re, im) pairs
 template <bool RX> struct XEt { typedef L2 T; };
 template <> struct XEt<true> { typedef i64 T; };
@@ -198,10 +214,11 @@ __device__ __noinline__ void rows_checked(const u32* __restrict__ states, const 
 template <bool DOT, bool RIO>
 __device__ __forceinline__ void body(const u32* __restrict__ states, const double* __restrict__ diag,
                                      const D2* __restrict__ x, const L2* __restrict__ xq,
-                                     const int* __restrict__ gmax_p, int sbits, D2* __restrict__ y, i64 dim,
+                                     int* __restrict__ gmax_p, int sbits, D2* __restrict__ y, i64 dim,
                                      const unsigned short* __restrict__ t0, const u32* __restrict__ t1, const uint4* __restrict__ t1n, double c0c,
                                      double c1c, double* __restrict__ partial) {
   extern __shared__ unsigned short t0s[];
+  if (gmax_p[3]) return;  // skip: a step before this one stopped
   for (int i = threadIdx.x; i < (1 << W0); i += blockDim.x) t0s[i] = t0[SWZ((u32)i)];
   __syncthreads();
   const int e_unit = gmax_p[0] - 1022 - sbits;
@@ -232,12 +249,13 @@ __device__ __forceinline__ void body(const u32* __restrict__ states, const doubl
         if (lane == 0) partial[k * gridDim.x + blockIdx.x] = a;
       }
     }
+    finish(partial, gmax_p);
   }
 }
 
 #define JIT_KERNEL(NAME, DOT, RIO, NT, MINB)                                                              \
   extern "C" __global__ void __launch_bounds__(NT, MINB) NAME(const u32* states, const double* diag,        \
-      const D2* x, const L2* xq, const int* gmax_p, int sbits, D2* y, i64 dim, const unsigned short* t0,     \
+      const D2* x, const L2* xq, int* gmax_p, int sbits, D2* y, i64 dim, const unsigned short* t0,     \
       const u32* t1, const uint4* t1n, double c0c, double c1c, double* partial) {                                             \
     body<DOT, RIO>(states, diag, x, xq, gmax_p, sbits, y, dim, t0, t1, t1n, c0c, c1c, partial);                  \
   }
@@ -389,10 +407,11 @@ __device__ __noinline__ void rows_checked(const u32* __restrict__ states, const 
 template <bool DOT, bool RIO>
 __device__ __forceinline__ void body(const u32* __restrict__ states, const double* __restrict__ diag,
                                      const D2* __restrict__ x, const L2* __restrict__ xq,
-                                     const int* __restrict__ gmax_p, int sbits, D2* __restrict__ y, i64 dim,
+                                     int* __restrict__ gmax_p, int sbits, D2* __restrict__ y, i64 dim,
                                      const unsigned short* __restrict__ t0, const u32* __restrict__ t1, const uint4* __restrict__ t1n, int pbexp,
                                      double* __restrict__ partial, const PBC& pbc, const i64* __restrict__ gcf) {
   extern __shared__ unsigned short t0s[];
+  if (gmax_p[3]) return;  // skip: a step before this one stopped
   for (int i = threadIdx.x; i < (1 << W0); i += blockDim.x) t0s[i] = t0[SWZ((u32)i)];
   __syncthreads();
   const int xexp = gmax_p[0] - 1022 - sbits + pbexp;
@@ -421,12 +440,13 @@ __device__ __forceinline__ void body(const u32* __restrict__ states, const doubl
         if (lane == 0) partial[k * gridDim.x + blockIdx.x] = a;
       }
     }
+    finish(partial, gmax_p);
   }
 }
 
 #define JIT_KERNEL(NAME, DOT, RIO, NT, MINB)                                                              \
   extern "C" __global__ void __launch_bounds__(NT, MINB) NAME(const u32* states, const double* diag,        \
-      const D2* x, const L2* xq, const int* gmax_p, int sbits, D2* y, i64 dim, const unsigned short* t0,     \
+      const D2* x, const L2* xq, int* gmax_p, int sbits, D2* y, i64 dim, const unsigned short* t0,     \
       const u32* t1, const uint4* t1n, int pbexp, double* partial, const __grid_constant__ PBC pbc, const i64* gcf) {         \
     body<DOT, RIO>(states, diag, x, xq, gmax_p, sbits, y, dim, t0, t1, t1n, pbexp, partial, pbc, gcf);           \
   }
@@ -748,7 +768,7 @@ int ed_jit_launch(ed_ham* h, uint64_t signature, int budget, const void* x, void
   const uint32_t* states = b->d_states;
   const double* diag = h->d_diag;
   const longlong2* xq = h->d_xq;
-  const int* gmax = h->d_gmax;
+  int* gmax = h->d_gmax;
   int64_t dim = b->dim;
   const uint16_t* t0 = b->d_lin_t0;
   const uint32_t* t1 = b->d_lin_t1;

@@ -315,11 +315,12 @@ __device__ __forceinline__ void lin_rows(const uint32_t* __restrict__ states, co
 template <bool DOT, int U, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_hv_lin(const uint32_t* __restrict__ states, const double* __restrict__ diag,
                                                 const double2* __restrict__ x, const longlong2* __restrict__ xq,
-                                                const int* __restrict__ gmax_p, int sbits, double2* __restrict__ y,
+                                                int* __restrict__ gmax_p, int sbits, double2* __restrict__ y,
                                                 int64_t dim, const uint16_t* __restrict__ t0,
                                                 const uint32_t* __restrict__ t1, const LinSegs sg, double c0c,
                                                 double c1c, double* __restrict__ partial, int rio_flag) {
   extern __shared__ uint16_t t0s[];
+  if (gmax_p[ED_HV_SKIP]) return;
   const bool rio = rio_flag != 0;
   const int n0 = 1 << sg.w0;
   for (int i = threadIdx.x; i < n0; i += blockDim.x) t0s[i] = t0[i];
@@ -346,6 +347,14 @@ __global__ void __launch_bounds__(256, MINB) k_hv_lin(const uint32_t* __restrict
       partial[gridDim.x + blockIdx.x] = dacc[1];
       partial[2 * gridDim.x + blockIdx.x] = dacc[2];
     }
+    // the last block sums the partials in order: Re, Im x^H y and ||y||^2
+    if (!ed_last_block((unsigned*)gmax_p + ED_HV_COUNT)) return;
+    double t[3] = {0.0, 0.0, 0.0};
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x)
+      for (int k = 0; k < 3; ++k) t[k] += __ldcg(partial + k * gridDim.x + b);
+    ed_block_reduce<3>(t, sh);
+    if (threadIdx.x == 0)
+      for (int k = 0; k < 3; ++k) ((double*)(gmax_p + ED_HV_SUMS))[k] = t[k];
   }
 }
 
@@ -358,7 +367,7 @@ bool ed_lin_supported(const ed_ham* h) {
 
 // Launch variants (same results: the integer sums are exact, so the unroll
 // depth and register budget change only the speed).
-typedef void (*LinKernel)(const uint32_t*, const double*, const double2*, const longlong2*, const int*, int, double2*,
+typedef void (*LinKernel)(const uint32_t*, const double*, const double2*, const longlong2*, int*, int, double2*,
                           int64_t, const uint16_t*, const uint32_t*, const LinSegs, double, double, double*, int);
 struct LinVariant {
   LinKernel plain, dot;
@@ -475,8 +484,7 @@ static int lin_autotune(ed_ham* h, const void* x, void* y, int sbits, bool dot, 
 }
 
 // y = H x through the two-table kernel.  With dot set, the kernel also leaves
-// per-block partials of Re/Im x^H y and ||y||^2 in ctx->d_red (3 items of
-// *nblk_out blocks each, for ed_finish_reduce).
+// Re/Im x^H y and ||y||^2 after the flags (d_gmax + ED_HV_SUMS).
 int ed_launch_hv_lin(ed_ham* h, const void* x, void* y, bool dot, int* nblk_out, bool rio) {
   ED_TRY(lin_prepare(h));
   int sbits = 0;

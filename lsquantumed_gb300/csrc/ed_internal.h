@@ -92,6 +92,9 @@ struct ed_ctx {
   size_t red_cap = 0;             // doubles
   double* h_red = nullptr;
   int reduce_blocks = 0;
+  // blocks-done counter of the kernels whose last block finishes a reduction
+  // (zero between launches)
+  unsigned* d_counter = nullptr;
   // scratch kept between calls (ed_workspace), at most ED_WS_KEEP bytes
   void* ws = nullptr;
   size_t ws_cap = 0;
@@ -190,13 +193,33 @@ struct ed_ham {
   // block floating point copy of the H.v input (integer accumulation path)
   longlong2* d_xq = nullptr;      // 62-bit mantissas, (re, im) per state
   uint16_t* d_xe = nullptr;       // biased exponent per 32-state block
-  int* d_gmax = nullptr;          // largest block exponent
+  // H.v flags, ED_GMAX_BYTES: [0] largest exponent, [1] non-finite input, [2]
+  // imaginary parts, [3] skip (a queued H.v returns at once), [4] blocks-done
+  // counter; from byte 64 the fused dot's three sums
+  int* d_gmax = nullptr;
   // d_xq / d_gmax already hold the fixed-point copy of this real vector
   // (ed_scale_quantize_r); the next two-table H.v of it uses them once
   const void* xq_src = nullptr;
   int hv_kernel = 2;              // 0: FP64, 1: exact 128-bit, 2: 64-bit fixed point
   BondSegments segs{};
   ed_lin* lin = nullptr;          // tables and bond words of the two-table kernel
+};
+
+#define ED_GMAX_BYTES 128
+#define ED_HV_SKIP 3
+#define ED_HV_COUNT 4
+#define ED_HV_SUMS 16  // in ints
+
+// Device state of the expansion steps (ed_krylov.cu).
+enum { KR_RUN = 0, KR_REFINE = 1, KR_INVARIANT = 2, KR_EXPONENT = 3 };
+struct KrState {
+  double c[128];                 // Gram-Schmidt coefficients of the current step
+  double alpha[128], beta[128];  // per step
+  double a, y2, n2, n0, wmax, s; // the last step's: x^T y, ||y||^2, ||w||^2, norm before the update, max |w|, scale
+  int stop;                      // KR_RUN or why the host takes the step over
+  int step;                      // the last step closed
+  int emax;
+  unsigned counter;
 };
 
 // ---------------------------------------------------------------------------
@@ -216,6 +239,9 @@ int ed_launch_hv(ed_ham* h, const double2* x, double2* y);
 int ed_launch_hv_dot(ed_ham* h, const double2* x, double2* y, double2* dot, double* y2);
 // Same for x, y complex (rio false) or real storage double[dim] (rio true).
 int ed_launch_hv_dot_any(ed_ham* h, const void* x, void* y, bool rio, double2* dot, double* y2);
+// Real storage, nothing waits: *sums points at x^T y, 0 and ||y||^2 on the
+// device (valid until the operator's next fused H.v).
+int ed_launch_hv_dot_dev(ed_ham* h, const double* x, double* y, const double** sums);
 // y = H x with real storage (two-table kernel only).
 int ed_launch_hv_r(ed_ham* h, const double* x, double* y);
 // Fixed-point copy of x into h->d_xq: largest exponent, non-finite flag and
@@ -265,6 +291,9 @@ void ed_ham_unique_masks(const ed_ham* h, std::vector<uint32_t>& masks, std::vec
 
 // linear algebra on device vectors (complex128)
 int ed_ensure_reduce(ed_ctx* ctx, size_t doubles);
+int ed_ensure_counter(ed_ctx* ctx);
+// Queue step j of the real-storage expansion (ed_krylov.cu).
+int ed_kr_step(ed_ham* h, double* const* cols, int j, bool three_term, double* w, KrState* st);
 // Sum `items` rows of nblk per-block partials in ctx->d_red (fixed order),
 // copy to host_out and synchronise the stream.
 // The last nmax items are maximised over the blocks instead of summed.

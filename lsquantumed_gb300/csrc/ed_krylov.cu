@@ -1,0 +1,309 @@
+// Expansion steps of the real-storage Krylov-Schur solve.
+//
+// A step is four kernels and no host round trip: H.v with x^T y (ed_hv_lin.cu,
+// ed_hv_jit.cu), the local Lanczos projection with the Gram-Schmidt dots, the
+// update with the new norm, and the scaling with the fixed-point copy for the
+// next H.v.  Every reduction ends in the kernel that needs it: the last block
+// to finish sums the block partials in a fixed order.  The coefficients, the
+// refinement test (DGKS), the test for an invariant subspace and the scale
+// live in device memory (KrState); where a step needs the host (a refinement
+// pass, an invariant subspace, an exponent the high word of max |w| does not
+// determine) it sets `stop`, the kernels queued behind it return at once and
+// the host takes that step over.  Before, each step waited for the host three
+// times and took three reduction kernels: 130 us per step at 13k rows.
+#include "ed_internal.h"
+#include "ed_device.cuh"
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+
+#define KR_THREADS 256
+#define KR_GROUP 16  // columns per dots launch
+
+struct ColPtrsR {
+  const double* p[128];
+};
+
+static ColPtrsR kr_cols(const double* const* cols, int nv) {
+  ColPtrsR c;
+  for (int i = 0; i < 128; ++i) c.p[i] = nullptr;
+  for (int i = 0; i < nv && i < 128; ++i) c.p[i] = cols[i];
+  return c;
+}
+
+// Sums of NI <= 16 items per thread over the block: 16 threads per item add
+// 16 values each from shared memory, then four shuffle steps.  Every FP64 add
+// costs issue slots of GB300's slow FP64 unit, and a shuffle tree over 8 warps
+// spends 5 adds of 32 lanes per warp and item (45 warp adds per item against
+// 10 here).  Threads with (threadIdx.x & 15) == 0 return their item's sum.
+__device__ __forceinline__ double block_sums16(const double (&acc)[KR_GROUP], int ni, double* sh) {
+#pragma unroll
+  for (int k = 0; k < KR_GROUP; ++k)
+    if (k < ni) sh[k * (KR_THREADS + 1) + threadIdx.x] = acc[k];
+  __syncthreads();
+  const int item = threadIdx.x >> 4, l = threadIdx.x & 15;
+  double a = 0.0;
+  if (item < ni) {
+#pragma unroll
+    for (int q = 0; q < 16; ++q) a += sh[item * (KR_THREADS + 1) + l + 16 * q];
+  }
+#pragma unroll
+  for (int s = 8; s > 0; s >>= 1) a += __shfl_down_sync(0xffffffffu, a, s, 16);
+  return a;
+}
+
+// w <- w - a vj - b vjm1 (LOCAL, written back), then out[v0 + i] = V_{v0+i}^T w
+// for i < ng.  a and b from the device where a_dev / b_dev are given.
+template <bool LOCAL>
+__global__ void __launch_bounds__(KR_THREADS) k_kr_dots(const ColPtrsR cp, int v0, int ng, double* __restrict__ w,
+                                                        int64_t n, const double* __restrict__ vj, double a,
+                                                        const double* __restrict__ a_dev,
+                                                        const double* __restrict__ vjm1, double b,
+                                                        const double* __restrict__ b_dev, double* __restrict__ partial,
+                                                        double* __restrict__ out, unsigned* __restrict__ counter,
+                                                        const int* __restrict__ stop) {
+  if (stop && *stop) return;
+  if (LOCAL && a_dev) a = *a_dev;
+  if (LOCAL && b_dev) b = *b_dev;
+  double acc[KR_GROUP];
+#pragma unroll
+  for (int k = 0; k < KR_GROUP; ++k) acc[k] = 0.0;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += stride) {
+    double wv = w[r];
+    if (LOCAL) {
+      wv = fma(-a, vj[r], wv);
+      if (vjm1) wv = fma(-b, vjm1[r], wv);
+      w[r] = wv;
+    }
+#pragma unroll
+    for (int g = 0; g < KR_GROUP; ++g)
+      if (g < ng) acc[g] = fma(cp.p[v0 + g][r], wv, acc[g]);
+  }
+  __shared__ double sh[KR_GROUP * (KR_THREADS + 1)];
+  const int item = threadIdx.x >> 4, l = threadIdx.x & 15;
+  const double s = block_sums16(acc, ng, sh);
+  if (l == 0 && item < ng) partial[(size_t)item * gridDim.x + blockIdx.x] = s;
+  if (!ed_last_block(counter)) return;
+  double t = 0.0;
+  if (item < ng)
+    for (unsigned q = l; q < gridDim.x; q += 16) t += __ldcg(partial + (size_t)item * gridDim.x + q);
+#pragma unroll
+  for (int k = 8; k > 0; k >>= 1) t += __shfl_down_sync(0xffffffffu, t, k, 16);
+  if (l == 0 && item < ng) out[v0 + item] = t;
+}
+
+// ||w||^2, four rows in flight per thread.
+__global__ void __launch_bounds__(KR_THREADS) k_kr_norm2(const double* __restrict__ w, int64_t n,
+                                                         double* __restrict__ partial, double* __restrict__ out,
+                                                         unsigned* __restrict__ counter) {
+  double acc[1] = {0.0};
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += 4 * stride) {
+    double x[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) x[u] = r + u * stride < n ? w[r + u * stride] : 0.0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) acc[0] = fma(x[u], x[u], acc[0]);
+  }
+  __shared__ double sh[32];
+  ed_block_reduce<1>(acc, sh);
+  if (threadIdx.x == 0) partial[blockIdx.x] = acc[0];
+  if (!ed_last_block(counter)) return;
+  double t[1] = {0.0};
+  for (unsigned q = threadIdx.x; q < gridDim.x; q += blockDim.x) t[0] += __ldcg(partial + q);
+  ed_block_reduce<1>(t, sh);
+  if (threadIdx.x == 0) *out = t[0];
+}
+
+// fl(max |w| s) has one biased exponent for every max |w| with this high word,
+// or -1 (ed_fx64_emax_scaled).
+__device__ __forceinline__ int kr_emax_scaled(double absmax_hi, double s) {
+  const double u = __longlong_as_double((long long)((unsigned long long)__double_as_longlong(absmax_hi) | 0xFFFFFFFFull));
+  const double ml = absmax_hi * s, mu = u * s;
+  if (!isfinite(ml) || !isfinite(mu) || !(s > 0.0)) return -1;
+  const int el = (int)(((unsigned long long)__double_as_longlong(ml) >> 52) & 0x7FF);
+  const int eu = (int)(((unsigned long long)__double_as_longlong(mu) >> 52) & 0x7FF);
+  return el == eu ? el : -1;
+}
+
+// w <- w - sum_i V_i c_i with ||w||^2 and the high word of max |w|; the last
+// block then closes the step (see the top of the file).  Two rows per thread,
+// columns unrolled by four.
+__global__ void __launch_bounds__(KR_THREADS) k_kr_update(const ColPtrsR cp, int nv, double* __restrict__ w, int64_t n,
+                                                          double* __restrict__ partial, KrState* __restrict__ st,
+                                                          const double* __restrict__ hv, int j,
+                                                          int* __restrict__ gmax) {
+  if (st->stop) return;
+  __shared__ double sh_h[128];
+  for (int i = threadIdx.x; i < nv; i += blockDim.x) sh_h[i] = st->c[i];
+  __syncthreads();
+  double acc[1] = {0.0};
+  unsigned int amax = 0u;  // high word of max |w|
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t r0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r0 < n; r0 += 2 * stride) {
+    const int64_t r1 = r0 + stride;
+    const bool has1 = r1 < n;
+    double w0 = w[r0];
+    double w1 = has1 ? w[r1] : 0.0;
+#pragma unroll 4
+    for (int i = 0; i < nv; ++i) {
+      const double* col = cp.p[i];
+      const double c = sh_h[i];
+      w0 = fma(-col[r0], c, w0);
+      if (has1) w1 = fma(-col[r1], c, w1);
+    }
+    w[r0] = w0;
+    acc[0] = fma(w0, w0, acc[0]);
+    amax = ed_absmax_hi(amax, w0);
+    if (has1) {
+      w[r1] = w1;
+      acc[0] = fma(w1, w1, acc[0]);
+      amax = ed_absmax_hi(amax, w1);
+    }
+  }
+  __shared__ double sh[32];
+  __shared__ unsigned int shm[8];
+  ed_block_reduce<1>(acc, sh);
+  amax = __reduce_max_sync(0xffffffffu, amax);
+  if ((threadIdx.x & 31) == 0) shm[threadIdx.x >> 5] = amax;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int q = 1; q < KR_THREADS / 32; ++q) amax = max(amax, shm[q]);
+    partial[blockIdx.x] = acc[0];
+    partial[gridDim.x + blockIdx.x] = ed_absmax_hi_value(amax);
+  }
+  if (!ed_last_block(&st->counter)) return;
+  double t[1] = {0.0};
+  amax = 0u;
+  for (unsigned q = threadIdx.x; q < gridDim.x; q += blockDim.x) {
+    t[0] += __ldcg(partial + q);
+    amax = ed_absmax_hi(amax, __ldcg(partial + gridDim.x + q));
+  }
+  __syncthreads();  // sh, shm free
+  ed_block_reduce<1>(t, sh);
+  amax = __reduce_max_sync(0xffffffffu, amax);
+  if ((threadIdx.x & 31) == 0) shm[threadIdx.x >> 5] = amax;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int q = 1; q < KR_THREADS / 32; ++q) amax = max(amax, shm[q]);
+    const double n2 = t[0], nw = sqrt(n2), mx = ed_absmax_hi_value(amax);
+    // the norm before the update (Pythagoras against the orthonormal basis)
+    double s2 = n2;
+    for (int i = 0; i < nv; ++i) s2 += sh_h[i] * sh_h[i];
+    const double n0 = sqrt(s2), norig = sqrt(hv[2]);
+    st->step = j;
+    st->a = hv[0];
+    st->y2 = hv[2];
+    st->n2 = n2;
+    st->n0 = n0;
+    st->wmax = mx;
+    st->alpha[j] = hv[0] + sh_h[j];
+    st->beta[j] = nw;
+    const double s = 1.0 / nw;
+    const int emax = kr_emax_scaled(mx, s);
+    st->s = s;
+    st->emax = emax;
+    int why = KR_RUN;
+    if (!(nw >= 0.7071067811865476 * n0)) why = KR_REFINE;
+    else if (nw <= 1e-13 * norig) why = KR_INVARIANT;
+    else if (emax < 0) why = KR_EXPONENT;
+    if (why != KR_RUN) {
+      st->stop = why;
+      gmax[3] = 1;  // the H.v kernels queued behind return
+    } else {
+      gmax[0] = emax;
+      gmax[1] = 0;
+      gmax[2] = 0;
+    }
+  }
+}
+
+// dst = w s and its fixed-point copy for the next H.v (k_scale_quantize_r with
+// the scale and exponent from the device).
+__global__ void __launch_bounds__(KR_THREADS) k_kr_scale(const double* __restrict__ w, double* __restrict__ dst,
+                                                         int64_t n, const KrState* __restrict__ st, int sbits,
+                                                         long long* __restrict__ xq) {
+  if (st->stop) return;
+  const double s = st->s;
+  const int emax = st->emax;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t r0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r0 < n; r0 += 2 * stride) {
+    const int64_t r1 = r0 + stride;
+    const double v0 = w[r0] * s, v1 = r1 < n ? w[r1] * s : 0.0;
+    dst[r0] = v0;
+    xq[r0] = ed_fx64_entry(v0, emax, sbits);
+    if (r1 < n) {
+      dst[r1] = v1;
+      xq[r1] = ed_fx64_entry(v1, emax, sbits);
+    }
+  }
+}
+
+// Blocks of a pass over n rows: at most per_sm per SM.
+static int kr_blocks(ed_ctx* ctx, int64_t n, int per_sm) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>((n + KR_THREADS - 1) / KR_THREADS, (int64_t)ctx->num_sms * per_sm));
+}
+
+// partials, results and the counter in the reduction buffer:
+// [items][nblk] | out[items] ; the counter is the context's
+static int kr_dots(ed_ctx* ctx, const double* const* cols, int nv, double* w, int64_t n, const double* vj, double a,
+                   const double* a_dev, const double* vjm1, double b, const double* b_dev, double* out, const int* stop) {
+  const int nblk = kr_blocks(ctx, n, 4);
+  ED_TRY(ed_ensure_reduce(ctx, (size_t)KR_GROUP * nblk + 256));
+  ED_TRY(ed_ensure_counter(ctx));
+  double* partial = ctx->d_red;
+  const ColPtrsR cp = kr_cols(cols, nv);
+  for (int v0 = 0; v0 < nv; v0 += KR_GROUP) {
+    const int ng = std::min(KR_GROUP, nv - v0);
+    if (v0 == 0 && vj)
+      k_kr_dots<true><<<nblk, KR_THREADS, 0, ctx->stream>>>(cp, v0, ng, w, n, vj, a, a_dev, vjm1, b, b_dev, partial, out,
+                                                           ctx->d_counter, stop);
+    else
+      k_kr_dots<false><<<nblk, KR_THREADS, 0, ctx->stream>>>(cp, v0, ng, w, n, nullptr, 0.0, nullptr, nullptr, 0.0,
+                                                            nullptr, partial, out, ctx->d_counter, stop);
+    ED_CHECK_LAUNCH(ctx);
+  }
+  return ED_OK;
+}
+
+int ed_multidot_r(ed_ctx* ctx, const double* const* cols, int nv, double* w, int64_t n, const double* vj, double a,
+                  const double* vjm1, double b, double* h_host, double* wnorm2_host) {
+  if (nv > 127) return ed_fail(ED_ENOTSUP, "at most 127 basis vectors");
+  const int nblk = kr_blocks(ctx, n, 4);
+  const size_t part = (size_t)KR_GROUP * nblk;
+  ED_TRY(ed_ensure_reduce(ctx, part + 256));
+  ED_TRY(ed_ensure_counter(ctx));
+  double* out = ctx->d_red + part;
+  if (nv > 0) ED_TRY(kr_dots(ctx, cols, nv, w, n, vj, a, nullptr, vjm1, b, nullptr, out, nullptr));
+  if (wnorm2_host) {
+    k_kr_norm2<<<nblk, KR_THREADS, 0, ctx->stream>>>(w, n, ctx->d_red, out + nv, ctx->d_counter);
+    ED_CHECK_LAUNCH(ctx);
+  }
+  const int items = nv + (wnorm2_host ? 1 : 0);
+  if (items == 0) return ED_OK;
+  ED_CUDA(cudaMemcpyAsync(ctx->h_red, out, sizeof(double) * items, cudaMemcpyDeviceToHost, ctx->stream));
+  ED_CUDA(cudaStreamSynchronize(ctx->stream));
+  for (int i = 0; i < nv; ++i) h_host[i] = ctx->h_red[i];
+  if (wnorm2_host) *wnorm2_host = ctx->h_red[nv];
+  return ED_OK;
+}
+
+// Queues step j: H.v of cols[j] (its fixed-point copy is in place or is made
+// here), projection, update and scaling into cols[j + 1].  Nothing waits.
+int ed_kr_step(ed_ham* h, double* const* cols, int j, bool three_term, double* w, KrState* st) {
+  ed_ctx* ctx = h->ctx;
+  const int64_t n = h->basis->dim;
+  const double* hv = nullptr;
+  ED_TRY(ed_launch_hv_dot_dev(h, cols[j], w, &hv));
+  ED_TRY(kr_dots(ctx, cols, j + 1, w, n, cols[j], 0.0, hv, three_term ? cols[j - 1] : nullptr, 0.0,
+                 three_term ? &st->beta[j - 1] : nullptr, st->c, &st->stop));
+  const int nblk = kr_blocks(ctx, n, 4);
+  k_kr_update<<<nblk, KR_THREADS, 0, ctx->stream>>>(kr_cols(cols, j + 1), j + 1, w, n, ctx->d_red, st, hv, j, h->d_gmax);
+  ED_CHECK_LAUNCH(ctx);
+  k_kr_scale<<<kr_blocks(ctx, n, 8), KR_THREADS, 0, ctx->stream>>>(w, cols[j + 1], n, st, ed_fx64_sbits(h),
+                                                                 (long long*)h->d_xq);
+  ED_CHECK_LAUNCH(ctx);
+  h->xq_src = cols[j + 1];
+  return ED_OK;
+}

@@ -33,6 +33,13 @@ int ed_ensure_reduce(ed_ctx* ctx, size_t doubles) {
   return ED_OK;
 }
 
+int ed_ensure_counter(ed_ctx* ctx) {
+  if (ctx->d_counter) return ED_OK;
+  ED_CUDA(cudaMalloc(&ctx->d_counter, 256));
+  ED_CUDA(cudaMemsetAsync(ctx->d_counter, 0, 256, ctx->stream));
+  return ED_OK;
+}
+
 // partial[item * nblk + blk]
 template <int G, bool REAL>
 __global__ void __launch_bounds__(ED_RED_THREADS) k_multidot(const ColPtrs cp, int v0, int ng, const double2* __restrict__ w,
@@ -444,8 +451,6 @@ int ed_is_real(ed_ctx* ctx, const double2* v, int64_t n, bool* real) {
 // above restricted to those real parts: the products they skip are the
 // exact zeros, so every value equals what the complex kernels give.
 // ---------------------------------------------------------------------------
-#define ED_GROUP_R 16
-
 struct ColPtrsR {
   const double* p[128];
 };
@@ -501,70 +506,6 @@ __global__ void __launch_bounds__(256) k_restart_pair(const ColPtrsR cp, int m, 
     for (int k = 0; k < 8; ++k)
       if (k < nc) ((double*)outp.p[c0 + k])[r] = ed_pair_value(s[k], c[k]);
   }
-}
-
-// partial[item * nblk + blk]: items v0..v0+ng-1 = V_i^T w; item v0+ng = ||w||^2
-// (with_norm).  LOCAL: first w <- w - a vj - b vjm1 (vjm1 may be null),
-// written back.
-template <int G, bool LOCAL>
-__global__ void __launch_bounds__(ED_RED_THREADS) k_multidot_r(const ColPtrsR cp, int v0, int ng, double* __restrict__ w,
-                                                               int64_t n, const double* __restrict__ vj, double a,
-                                                               const double* __restrict__ vjm1, double b, int with_norm,
-                                                               double* __restrict__ partial, int nblk) {
-  double acc[G + 1];
-#pragma unroll
-  for (int k = 0; k <= G; ++k) acc[k] = 0.0;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += stride) {
-    double wv = w[r];
-    if (LOCAL) {
-      wv = fma(-a, vj[r], wv);
-      if (vjm1) wv = fma(-b, vjm1[r], wv);
-      w[r] = wv;
-    }
-#pragma unroll
-    for (int g = 0; g < G; ++g)
-      if (g < ng) acc[g] = fma(cp.p[v0 + g][r], wv, acc[g]);
-    if (with_norm) acc[G] = fma(wv, wv, acc[G]);
-  }
-  __shared__ double sh[(G + 1) * 32];
-  ed_block_reduce<G + 1>(acc, sh);
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int g = 0; g < G; ++g)
-      if (g < ng) partial[(size_t)(v0 + g) * nblk + blockIdx.x] = acc[g];
-    if (with_norm) partial[(size_t)(v0 + ng) * nblk + blockIdx.x] = acc[G];
-  }
-}
-
-// h_host[i] = V_i^T w (i < nv), *wnorm2_host = ||w||^2 (after the local step
-// when vj is given: w <- w - a vj - b vjm1 first, in the same pass as the
-// first group of dots).
-int ed_multidot_r(ed_ctx* ctx, const double* const* cols, int nv, double* w, int64_t n, const double* vj, double a,
-                  const double* vjm1, double b, double* h_host, double* wnorm2_host) {
-  if (nv > 127) return ed_fail(ED_ENOTSUP, "at most 127 basis vectors");
-  const int nblk = red_blocks(ctx, n);
-  const int items = nv + 1;
-  ED_TRY(ed_ensure_reduce(ctx, (size_t)items * nblk + items));
-  ColPtrsR cp = make_cols_r(cols, nv);
-  const int ngroups = std::max(1, (nv + ED_GROUP_R - 1) / ED_GROUP_R);
-  for (int gidx = 0; gidx < ngroups; ++gidx) {
-    const int v0 = gidx * ED_GROUP_R;
-    const int ng = std::max(0, std::min(ED_GROUP_R, nv - v0));
-    const int last = gidx == ngroups - 1 && wnorm2_host != nullptr;  // the norm costs one FP64 FMA per row
-    if (gidx == 0 && vj)
-      k_multidot_r<ED_GROUP_R, true><<<nblk, ED_RED_THREADS, 0, ctx->stream>>>(cp, v0, ng, w, n, vj, a, vjm1, b, last,
-                                                                              ctx->d_red, nblk);
-    else
-      k_multidot_r<ED_GROUP_R, false><<<nblk, ED_RED_THREADS, 0, ctx->stream>>>(cp, v0, ng, w, n, nullptr, 0.0, nullptr,
-                                                                               0.0, last, ctx->d_red, nblk);
-    ED_CHECK_LAUNCH(ctx);
-  }
-  std::vector<double> out(items);
-  ED_TRY(ed_finish_reduce(ctx, items, nblk, out.data()));
-  for (int i = 0; i < nv; ++i) h_host[i] = out[i];
-  if (wnorm2_host) *wnorm2_host = out[nv];
-  return ED_OK;
 }
 
 // w <- w - sum_i V_i h_i; partial ||w||^2.  Two rows per thread, columns
