@@ -45,40 +45,56 @@ struct ed_eps {
   int restart_mode = ED_RESTART_FP64;   // the form this real-storage solve uses
 };
 
-void ed_jacobi_eig(int m, std::vector<double>& A, std::vector<double>& theta, std::vector<double>& Y) {
-  Y.assign((size_t)m * m, 0.0);
-  for (int i = 0; i < m; ++i) Y[(size_t)i * m + i] = 1.0;
+// Cyclic Jacobi.  A rotation acts on rows p and q (contiguous) and is mirrored
+// into the columns; the vectors are kept as rows.  From the fifth sweep on an
+// entry that is below the rounding of both diagonal entries is dropped instead
+// of rotated: without it the sweeps of a 25 x 25 problem never met the
+// off-diagonal bound and ran to the limit of 100 (4.6 ms per restart).
+__attribute__((optimize("O3"))) void ed_jacobi_eig(int m, std::vector<double>& A, std::vector<double>& theta, std::vector<double>& Y) {
+  std::vector<double> V((size_t)m * m, 0.0);  // row c: vector c
+  for (int i = 0; i < m; ++i) V[(size_t)i * m + i] = 1.0;
   for (int sweep = 0; sweep < 100; ++sweep) {
     double off = 0, tot = 0;
-    for (int i = 0; i < m; ++i)
-      for (int j = 0; j < m; ++j) {
-        double a = A[(size_t)i * m + j] * A[(size_t)i * m + j];
-        tot += a;
-        if (i != j) off += a;
-      }
+    for (int i = 0; i < m; ++i) {
+      const double* a = &A[(size_t)i * m];
+      for (int j = 0; j < i; ++j) off += 2.0 * a[j] * a[j];
+      tot += a[i] * a[i];
+    }
+    tot += off;
     if (off <= 1e-32 * tot || off == 0.0) break;
     for (int p = 0; p < m - 1; ++p)
       for (int q = p + 1; q < m; ++q) {
-        double apq = A[(size_t)p * m + q];
+        double* ap = &A[(size_t)p * m];
+        double* aq = &A[(size_t)q * m];
+        const double apq = ap[q];
         if (apq == 0.0) continue;
-        double app = A[(size_t)p * m + p], aqq = A[(size_t)q * m + q];
-        double tau = (aqq - app) / (2.0 * apq);
-        double t = (tau >= 0 ? 1.0 : -1.0) / (std::fabs(tau) + std::sqrt(1.0 + tau * tau));
-        double c = 1.0 / std::sqrt(1.0 + t * t), s = t * c;
-        for (int k = 0; k < m; ++k) {
-          double akp = A[(size_t)k * m + p], akq = A[(size_t)k * m + q];
-          A[(size_t)k * m + p] = c * akp - s * akq;
-          A[(size_t)k * m + q] = s * akp + c * akq;
+        const double app = ap[p], aqq = aq[q];
+        const double g = 100.0 * std::fabs(apq);
+        if (sweep > 3 && std::fabs(app) + g == std::fabs(app) && std::fabs(aqq) + g == std::fabs(aqq)) {
+          ap[q] = aq[p] = 0.0;
+          continue;
         }
+        const double tau = (aqq - app) / (2.0 * apq);
+        const double t = (tau >= 0 ? 1.0 : -1.0) / (std::fabs(tau) + std::sqrt(1.0 + tau * tau));
+        const double c = 1.0 / std::sqrt(1.0 + t * t), s = t * c;
         for (int k = 0; k < m; ++k) {
-          double apk = A[(size_t)p * m + k], aqk = A[(size_t)q * m + k];
-          A[(size_t)p * m + k] = c * apk - s * aqk;
-          A[(size_t)q * m + k] = s * apk + c * aqk;
+          const double x = ap[k], y = aq[k];
+          ap[k] = c * x - s * y;
+          aq[k] = s * x + c * y;
         }
+        ap[p] = app - t * apq;
+        aq[q] = aqq + t * apq;
+        ap[q] = aq[p] = 0.0;
         for (int k = 0; k < m; ++k) {
-          double ykp = Y[(size_t)k * m + p], ykq = Y[(size_t)k * m + q];
-          Y[(size_t)k * m + p] = c * ykp - s * ykq;
-          Y[(size_t)k * m + q] = s * ykp + c * ykq;
+          A[(size_t)k * m + p] = ap[k];
+          A[(size_t)k * m + q] = aq[k];
+        }
+        double* vp = &V[(size_t)p * m];
+        double* vq = &V[(size_t)q * m];
+        for (int k = 0; k < m; ++k) {
+          const double x = vp[k], y = vq[k];
+          vp[k] = c * x - s * y;
+          vq[k] = s * x + c * y;
         }
       }
   }
@@ -87,12 +103,11 @@ void ed_jacobi_eig(int m, std::vector<double>& A, std::vector<double>& theta, st
   std::stable_sort(idx.begin(), idx.end(),
                    [&](int a, int b) { return A[(size_t)a * m + a] < A[(size_t)b * m + b]; });
   theta.resize(m);
-  std::vector<double> Ys((size_t)m * m);
+  Y.resize((size_t)m * m);
   for (int c = 0; c < m; ++c) {
     theta[c] = A[(size_t)idx[c] * m + idx[c]];
-    for (int r = 0; r < m; ++r) Ys[(size_t)r * m + c] = Y[(size_t)r * m + idx[c]];
+    for (int r = 0; r < m; ++r) Y[(size_t)r * m + c] = V[(size_t)idx[c] * m + r];
   }
-  Y.swap(Ys);
 }
 
 static void eps_free(ed_eps* e) {

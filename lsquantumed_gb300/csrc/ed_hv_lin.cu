@@ -309,11 +309,35 @@ __device__ __forceinline__ void lin_rows(const uint32_t* __restrict__ states, co
   }
 }
 
+// Sums of three values over the block, in thread 0 (a warp per item adds the
+// NT values: NT / 32 + 5 FP64 adds per item instead of five per warp).
+template <int NT>
+__device__ __forceinline__ void lin_sums(double (&v)[3], double* sh) {
+  const int lane = threadIdx.x & 31;
+  __syncthreads();  // sh free
+#pragma unroll
+  for (int k = 0; k < 3; ++k) sh[k * NT + threadIdx.x] = v[k];
+  __syncthreads();
+  for (int k = threadIdx.x >> 5; k < 3; k += NT / 32) {
+    double a = 0.0;
+#pragma unroll
+    for (int q = 0; q < NT / 32; ++q) a += sh[k * NT + lane + 32 * q];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+    __syncwarp();
+    if (lane == 0) sh[k * NT] = a;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 3; ++k) v[k] = sh[k * NT];
+}
+
 // DOT: partial[item * gridDim.x + block] for item 0/1 = Re/Im x^H y, 2 = ||y||^2.
 // U: bonds per unrolled batch (gathers in flight per thread); MINB: blocks
 // per SM the register allocation must allow.
-template <bool DOT, int U, int MINB>
-__global__ void __launch_bounds__(256, MINB) k_hv_lin(const uint32_t* __restrict__ states, const double* __restrict__ diag,
+// NT: threads per block.
+template <bool DOT, int U, int MINB, int NT = 256>
+__global__ void __launch_bounds__(NT, MINB) k_hv_lin(const uint32_t* __restrict__ states, const double* __restrict__ diag,
                                                 const double2* __restrict__ x, const longlong2* __restrict__ xq,
                                                 int* __restrict__ gmax_p, int sbits, double2* __restrict__ y,
                                                 int64_t dim, const uint16_t* __restrict__ t0,
@@ -340,8 +364,8 @@ __global__ void __launch_bounds__(256, MINB) k_hv_lin(const uint32_t* __restrict
     else lin_rows<false, DOT, U, false>(states, diag, x, xq, y, dim, t0s, t1, sg, c0c, c1c, s1, s2, dacc, rio);
   }
   if (DOT) {
-    __shared__ double sh[3 * 32];
-    ed_block_reduce<3>(dacc, sh);
+    __shared__ double sh[3 * NT];
+    lin_sums<NT>(dacc, sh);
     if (threadIdx.x == 0) {
       partial[blockIdx.x] = dacc[0];
       partial[gridDim.x + blockIdx.x] = dacc[1];
@@ -352,7 +376,7 @@ __global__ void __launch_bounds__(256, MINB) k_hv_lin(const uint32_t* __restrict
     double t[3] = {0.0, 0.0, 0.0};
     for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x)
       for (int k = 0; k < 3; ++k) t[k] += __ldcg(partial + k * gridDim.x + b);
-    ed_block_reduce<3>(t, sh);
+    lin_sums<NT>(t, sh);
     if (threadIdx.x == 0)
       for (int k = 0; k < 3; ++k) ((double*)(gmax_p + ED_HV_SUMS))[k] = t[k];
   }
@@ -379,6 +403,9 @@ static const LinVariant kLinVariants[] = {
     {k_hv_lin<false, 8, 4>, k_hv_lin<true, 8, 4>, "u8-b4"},
     {k_hv_lin<false, 8, 1>, k_hv_lin<true, 8, 1>, "u8-b1"},
 };
+// Fewer rows than 256 threads per SM: blocks of 64, so that every SM takes
+// part (the FP64 work of a row and the sums are what a block waits for).
+static const LinKernel kLinSmall[2] = {k_hv_lin<false, 8, 1, 64>, k_hv_lin<true, 8, 1, 64>};
 static const int kNumLinVariants = (int)(sizeof(kLinVariants) / sizeof(kLinVariants[0]));
 
 // Variants kNumLinVariants + 0 .. 4 are the run-time specialised kernel
@@ -397,15 +424,17 @@ static int lin_launch(ed_ham* h, int v, const void* x, void* y, bool dot, int sb
     return ed_jit_launch(h, lin_signature(h), v - kJitVariant, x, y, dot, sbits, nblk_out, L->segs.word, L->segs.seg,
                          L->segs.w0, rio, L->per_bond ? L->coef.data() : nullptr, L->d_coef, L->pbexp);
   const size_t smem = sizeof(uint16_t) * ((size_t)1 << b->lin_w0);
-  LinKernel k = dot ? kLinVariants[v].dot : kLinVariants[v].plain;
+  const bool small = b->dim < (int64_t)ctx->num_sms * 256;
+  const int nt = small ? 64 : 256;
+  LinKernel k = small ? kLinSmall[dot ? 1 : 0] : dot ? kLinVariants[v].dot : kLinVariants[v].plain;
   int per_sm = 0;
-  ED_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 256, smem));
+  ED_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, nt, smem));
   if (per_sm < 1) per_sm = 1;
-  int64_t g = (b->dim + 255) / 256;
+  int64_t g = (b->dim + nt - 1) / nt;
   g = std::max<int64_t>(1, std::min<int64_t>(g, (int64_t)ctx->num_sms * per_sm));
   const int nblk = (int)g;
   if (dot) ED_TRY(ed_ensure_reduce(ctx, (size_t)3 * nblk + 8));
-  k<<<nblk, 256, smem, ctx->stream>>>(b->d_states, h->d_diag, (const double2*)x, h->d_xq, h->d_gmax, sbits,
+  k<<<nblk, nt, smem, ctx->stream>>>(b->d_states, h->d_diag, (const double2*)x, h->d_xq, h->d_gmax, sbits,
                                       (double2*)y, b->dim, b->d_lin_t0, b->d_lin_t1, L->segs, h->bs.chalf[0],
                                       h->bs.chalf[1], dot ? ctx->d_red : nullptr, rio ? 1 : 0);
   ED_CHECK_LAUNCH(ctx);

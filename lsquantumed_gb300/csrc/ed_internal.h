@@ -215,7 +215,7 @@ enum { KR_RUN = 0, KR_REFINE = 1, KR_INVARIANT = 2, KR_EXPONENT = 3 };
 struct KrState {
   double c[128];                 // Gram-Schmidt coefficients of the current step
   double alpha[128], beta[128];  // per step
-  double a, y2, n2, n0, wmax, s; // the last step's: x^T y, ||y||^2, ||w||^2, norm before the update, max |w|, scale
+  double y2, wmax, s;            // the last step's: ||H v||^2, high word of max |w|, scale 1 / ||w||
   int stop;                      // KR_RUN or why the host takes the step over
   int step;                      // the last step closed
   int emax;

@@ -52,6 +52,22 @@ __device__ __forceinline__ double block_sums16(const double (&acc)[KR_GROUP], in
   return a;
 }
 
+// Sum over the block's 256 threads (all threads call it; thread 0 has it): 32
+// lanes add 8 values each, then one shuffle tree.
+__device__ __forceinline__ double block_sum256(double v, double* sh) {
+  __syncthreads();  // sh free
+  sh[threadIdx.x] = v;
+  __syncthreads();
+  double a = 0.0;
+  if (threadIdx.x < 32) {
+#pragma unroll
+    for (int q = 0; q < KR_THREADS / 32; ++q) a += sh[threadIdx.x + 32 * q];
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1) a += __shfl_down_sync(0xffffffffu, a, k);
+  }
+  return a;
+}
+
 // w <- w - a vj - b vjm1 (LOCAL, written back), then out[v0 + i] = V_{v0+i}^T w
 // for i < ng.  a and b from the device where a_dev / b_dev are given.
 template <bool LOCAL>
@@ -106,14 +122,14 @@ __global__ void __launch_bounds__(KR_THREADS) k_kr_norm2(const double* __restric
 #pragma unroll
     for (int u = 0; u < 4; ++u) acc[0] = fma(x[u], x[u], acc[0]);
   }
-  __shared__ double sh[32];
-  ed_block_reduce<1>(acc, sh);
-  if (threadIdx.x == 0) partial[blockIdx.x] = acc[0];
+  __shared__ double sh[KR_THREADS];
+  const double bs = block_sum256(acc[0], sh);
+  if (threadIdx.x == 0) partial[blockIdx.x] = bs;
   if (!ed_last_block(counter)) return;
-  double t[1] = {0.0};
-  for (unsigned q = threadIdx.x; q < gridDim.x; q += blockDim.x) t[0] += __ldcg(partial + q);
-  ed_block_reduce<1>(t, sh);
-  if (threadIdx.x == 0) *out = t[0];
+  double t = 0.0;
+  for (unsigned q = threadIdx.x; q < gridDim.x; q += blockDim.x) t += __ldcg(partial + q);
+  t = block_sum256(t, sh);
+  if (threadIdx.x == 0) *out = t;
 }
 
 // fl(max |w| s) has one biased exponent for every max |w| with this high word,
@@ -162,55 +178,56 @@ __global__ void __launch_bounds__(KR_THREADS) k_kr_update(const ColPtrsR cp, int
       amax = ed_absmax_hi(amax, w1);
     }
   }
-  __shared__ double sh[32];
+  __shared__ double sh[KR_THREADS];
   __shared__ unsigned int shm[8];
-  ed_block_reduce<1>(acc, sh);
+  double bs = block_sum256(acc[0], sh);
   amax = __reduce_max_sync(0xffffffffu, amax);
   if ((threadIdx.x & 31) == 0) shm[threadIdx.x >> 5] = amax;
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int q = 1; q < KR_THREADS / 32; ++q) amax = max(amax, shm[q]);
-    partial[blockIdx.x] = acc[0];
+    partial[blockIdx.x] = bs;
     partial[gridDim.x + blockIdx.x] = ed_absmax_hi_value(amax);
   }
   if (!ed_last_block(&st->counter)) return;
-  double t[1] = {0.0};
+  double t = 0.0;
   amax = 0u;
   for (unsigned q = threadIdx.x; q < gridDim.x; q += blockDim.x) {
-    t[0] += __ldcg(partial + q);
+    t += __ldcg(partial + q);
     amax = ed_absmax_hi(amax, __ldcg(partial + gridDim.x + q));
   }
-  __syncthreads();  // sh, shm free
-  ed_block_reduce<1>(t, sh);
+  const double n2 = block_sum256(t, sh);
   amax = __reduce_max_sync(0xffffffffu, amax);
   if ((threadIdx.x & 31) == 0) shm[threadIdx.x >> 5] = amax;
   __syncthreads();
+  if (threadIdx.x >= 32) return;
+  // one warp closes the step; FP64 instructions are slow, so as few in a row
+  // as possible: the tests compare squares
+  amax = __reduce_max_sync(0xffffffffu, threadIdx.x < KR_THREADS / 32 ? shm[threadIdx.x] : 0u);
+  double c2 = 0.0;
+  for (int i = threadIdx.x; i < nv; i += 32) c2 = fma(sh_h[i], sh_h[i], c2);
+#pragma unroll
+  for (int k = 16; k > 0; k >>= 1) c2 += __shfl_down_sync(0xffffffffu, c2, k);
   if (threadIdx.x == 0) {
-    for (int q = 1; q < KR_THREADS / 32; ++q) amax = max(amax, shm[q]);
-    const double n2 = t[0], nw = sqrt(n2), mx = ed_absmax_hi_value(amax);
-    // the norm before the update (Pythagoras against the orthonormal basis)
-    double s2 = n2;
-    for (int i = 0; i < nv; ++i) s2 += sh_h[i] * sh_h[i];
-    const double n0 = sqrt(s2), norig = sqrt(hv[2]);
+    const double nw = sqrt(n2), mx = ed_absmax_hi_value(amax), y2 = hv[2];
+    const double s = 1.0 / nw;
+    const int emax = kr_emax_scaled(mx, s);
     st->step = j;
-    st->a = hv[0];
-    st->y2 = hv[2];
-    st->n2 = n2;
-    st->n0 = n0;
+    st->y2 = y2;
     st->wmax = mx;
     st->alpha[j] = hv[0] + sh_h[j];
     st->beta[j] = nw;
-    const double s = 1.0 / nw;
-    const int emax = kr_emax_scaled(mx, s);
     st->s = s;
     st->emax = emax;
     int why = KR_RUN;
-    if (!(nw >= 0.7071067811865476 * n0)) why = KR_REFINE;
-    else if (nw <= 1e-13 * norig) why = KR_INVARIANT;
+    // the squared norm before the update is n2 + sum c_i^2 (Pythagoras against
+    // the orthonormal basis): refine below 1/sqrt(2) of it
+    if (!(n2 >= 0.5 * (n2 + c2))) why = KR_REFINE;
+    else if (n2 <= 1e-26 * y2) why = KR_INVARIANT;
     else if (emax < 0) why = KR_EXPONENT;
     if (why != KR_RUN) {
       st->stop = why;
-      gmax[3] = 1;  // the H.v kernels queued behind return
+      gmax[ED_HV_SKIP] = 1;  // the H.v kernels queued behind return
     } else {
       gmax[0] = emax;
       gmax[1] = 0;
