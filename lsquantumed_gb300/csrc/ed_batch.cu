@@ -341,59 +341,87 @@ struct BCols {
 #define BU_REG 16  // k_batch_update_norm keeps up to this many coefficients in registers
 // With vj: first w <- w - a_b vj - bet_b vjm1 (coef = [a][B], [bet][B]),
 // written back, in the same pass (the local Lanczos projection).
-__global__ void __launch_bounds__(256) k_batch_dots(const BCols V, int nv, double* __restrict__ w, int64_t dim,
-                                                    int B, int with_norm, double* __restrict__ partial, int nblk,
+// One instance per column count NI (0: the norm alone): the loads of a row are
+// issued together, without a test per column.  More than BD_MAXV columns: the
+// first BD_MAXV here, the others by the caller's next launches (item0).
+template <int NI>
+__global__ void __launch_bounds__(256) k_batch_dots(const BCols V, int item0, double* __restrict__ w, int64_t dim,
+                                                    int B, int norm_item, double* __restrict__ partial, int nblk,
                                                     const double* __restrict__ vj, const double* __restrict__ vjm1,
                                                     const double* __restrict__ coef, const int* __restrict__ pred) {
   if (pred && *pred == 0) return;  // a pass the device decided to skip (uniform over the grid)
-  __shared__ double sh[256 * (BD_MAXV + 1)];
+  __shared__ double sh[256 * (NI + 1)];
   const int Bp = B >= 256 ? 256 : ((B + 31) / 32) * 32;
   const int S = 256 / Bp;  // row lanes
   const int lane_b = threadIdx.x % Bp, lane_r = threadIdx.x / Bp;
   const int64_t rows_per = (dim + gridDim.x - 1) / gridDim.x;
   const int64_t r0 = (int64_t)blockIdx.x * rows_per, r1 = min(dim, r0 + rows_per);
+  const bool norm = norm_item >= 0;
   for (int b0 = 0; b0 < B; b0 += Bp) {
     const int b = b0 + lane_b;
-    const bool act = lane_r < S && b < B;
-    for (int i0 = 0; i0 < max(nv, 1); i0 += BD_MAXV) {
-      const int ni = max(0, min(BD_MAXV, nv - i0));
-      const bool norm = with_norm && i0 == 0;
-      double acc[BD_MAXV + 1];
+    double acc[NI + 1];
 #pragma unroll
-      for (int i = 0; i <= BD_MAXV; ++i) acc[i] = 0.0;
-      if (act) {
-        const bool local = vj && i0 == 0;
-        const double ca = local ? coef[b] : 0.0, cb = local ? coef[B + b] : 0.0;
-        for (int64_t r = r0 + lane_r; r < r1; r += S) {
-          const size_t k = (size_t)r * B + b;
-          double wv = w[k];
-          if (local) {
-            wv = fma(-ca, vj[k], wv);
-            if (vjm1) wv = fma(-cb, vjm1[k], wv);
-            w[k] = wv;
-          }
+    for (int i = 0; i <= NI; ++i) acc[i] = 0.0;
+    if (lane_r < S && b < B) {
+      const double ca = vj ? coef[b] : 0.0, cb = vj ? coef[B + b] : 0.0;
+      for (int64_t r = r0 + lane_r; r < r1; r += S) {
+        const size_t k = (size_t)r * B + b;
+        double wv = w[k], p = 0.0, q = 0.0, v[NI + 1];
+        if (vj) p = vj[k];
+        if (vjm1) q = vjm1[k];
 #pragma unroll
-          for (int i = 0; i < BD_MAXV; ++i)
-            if (i < ni) acc[i] = fma(V.p[i0 + i][k], wv, acc[i]);
-          if (norm) acc[BD_MAXV] = fma(wv, wv, acc[BD_MAXV]);
+        for (int i = 0; i < NI; ++i) v[i] = V.p[i][k];
+        if (vj) {
+          wv = fma(-ca, p, wv);
+          if (vjm1) wv = fma(-cb, q, wv);
+          w[k] = wv;
         }
-      }
-      __syncthreads();  // sh free
 #pragma unroll
-      for (int i = 0; i <= BD_MAXV; ++i) sh[i * 256 + threadIdx.x] = acc[i];
-      __syncthreads();
-      if (lane_r == 0 && b < B) {
-        for (int i = 0; i <= BD_MAXV; ++i) {
-          if (i < ni || (i == BD_MAXV && norm)) {
-            double t = 0.0;
-            for (int q = 0; q < S; ++q) t += sh[i * 256 + q * Bp + lane_b];
-            const int item = i < BD_MAXV ? i0 + i : nv;
-            partial[((size_t)item * B + b) * nblk + blockIdx.x] = t;
-          }
-        }
+        for (int i = 0; i < NI; ++i) acc[i] = fma(v[i], wv, acc[i]);
+        if (norm) acc[NI] = fma(wv, wv, acc[NI]);
       }
     }
+    __syncthreads();  // sh free
+#pragma unroll
+    for (int i = 0; i <= NI; ++i) sh[i * 256 + threadIdx.x] = acc[i];
+    __syncthreads();
+    // the items over all threads: thread = (item group, column)
+    if (b < B)
+      for (int i = lane_r; i <= NI; i += S) {
+        if (i == NI && !norm) break;
+        double t = 0.0;
+        for (int q = 0; q < S; ++q) t += sh[i * 256 + q * Bp + lane_b];
+        partial[((size_t)(i < NI ? item0 + i : norm_item) * B + b) * nblk + blockIdx.x] = t;
+      }
   }
+}
+
+// partials of the dots of nv columns (and the norm where norm_item >= 0)
+static int batch_dots_launch(ed_ctx* ctx, int nblk, const std::vector<const double*>& V, double* w, int64_t dim, int B,
+                             int norm_item, double* partial, const double* vj, const double* vjm1, const double* coef,
+                             const int* pred) {
+  const int nv = (int)V.size();
+  for (int i0 = 0; i0 < std::max(nv, 1); i0 += BD_MAXV) {
+    const int ni = std::min(BD_MAXV, nv - i0);
+    BCols vc;
+    memset(&vc, 0, sizeof(vc));
+    for (int i = 0; i < ni; ++i) vc.p[i] = V[i0 + i];
+    auto go = [&](auto kern) {
+      kern<<<nblk, 256, 0, ctx->stream>>>(vc, i0, w, dim, B, i0 == 0 ? norm_item : -1, partial, nblk,
+                                          i0 == 0 ? vj : nullptr, i0 == 0 ? vjm1 : nullptr, coef, pred);
+    };
+#define BD_CASE(NI)         \
+  case NI:                  \
+    go(k_batch_dots<NI>);   \
+    break;
+    switch (ni) {
+      BD_CASE(0) BD_CASE(1) BD_CASE(2) BD_CASE(3) BD_CASE(4) BD_CASE(5) BD_CASE(6) BD_CASE(7) BD_CASE(8)
+      BD_CASE(9) BD_CASE(10) BD_CASE(11) BD_CASE(12) BD_CASE(13) BD_CASE(14) BD_CASE(15) BD_CASE(16)
+    }
+#undef BD_CASE
+    ED_CHECK_LAUNCH(ctx);
+  }
+  return ED_OK;
 }
 
 // out[item] = sum_k partial[item * nblk + k]: one warp per item, lanes over k
@@ -787,12 +815,7 @@ static int batch_dots(ed_batch* bt, int B, const std::vector<const double*>& V, 
   const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>(bt->dim / 64 + 1, (int64_t)ctx->num_sms * 4));
   const int64_t items = (int64_t)(nv + 1) * B;
   ED_TRY(batch_reduce_buf(bt, (size_t)items * nblk + (size_t)items));
-  BCols vc;
-  memset(&vc, 0, sizeof(vc));
-  for (int i = 0; i < nv && i < 64; ++i) vc.p[i] = V[i];
-  k_batch_dots<<<nblk, 256, 0, ctx->stream>>>(vc, nv, w, bt->dim, B, norm ? 1 : 0, bt->d_red, nblk, vj, vjm1, coef,
-                                              nullptr);
-  ED_CHECK_LAUNCH(ctx);
+  ED_TRY(batch_dots_launch(ctx, nblk, V, w, bt->dim, B, norm ? nv : -1, bt->d_red, vj, vjm1, coef, nullptr));
   double* res = bt->d_red + (size_t)items * nblk;
   k_batch_reduce<<<grid_n(ctx, items * 32, 8), 256, 0, ctx->stream>>>(bt->d_red, nblk, items, res, items);
   ED_CHECK_LAUNCH(ctx);
@@ -812,11 +835,7 @@ static int batch_dots_dev(ed_batch* bt, int B, const std::vector<const double*>&
   const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>(bt->dim / 64 + 1, (int64_t)ctx->num_sms * 4));
   const int64_t items = (int64_t)nv * B;
   ED_TRY(batch_reduce_buf(bt, (size_t)(items + B) * nblk + (size_t)items));
-  BCols vc;
-  memset(&vc, 0, sizeof(vc));
-  for (int i = 0; i < nv && i < 64; ++i) vc.p[i] = V[i];
-  k_batch_dots<<<nblk, 256, 0, ctx->stream>>>(vc, nv, w, bt->dim, B, 0, bt->d_red, nblk, vj, vjm1, coef, pred);
-  ED_CHECK_LAUNCH(ctx);
+  ED_TRY(batch_dots_launch(ctx, nblk, V, w, bt->dim, B, -1, bt->d_red, vj, vjm1, coef, pred));
   k_batch_reduce<<<grid_n(ctx, items * 32, 8), 256, 0, ctx->stream>>>(bt->d_red, nblk, items, out_dev, items, pred);
   ED_CHECK_LAUNCH(ctx);
   return ED_OK;

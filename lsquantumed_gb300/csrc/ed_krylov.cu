@@ -24,6 +24,10 @@ struct ColPtrsR {
   const double* p[128];
 };
 
+struct KrCols {
+  const double* p[KR_GROUP];
+};
+
 static ColPtrsR kr_cols(const double* const* cols, int nv) {
   ColPtrsR c;
   for (int i = 0; i < 128; ++i) c.p[i] = nullptr;
@@ -68,16 +72,24 @@ __device__ __forceinline__ double block_sum256(double v, double* sh) {
   return a;
 }
 
-// w <- w - a vj - b vjm1 (LOCAL, written back), then out[v0 + i] = V_{v0+i}^T w
-// for i < ng.  a and b from the device where a_dev / b_dev are given.
-template <bool LOCAL>
-__global__ void __launch_bounds__(KR_THREADS) k_kr_dots(const ColPtrsR cp, int v0, int ng, double* __restrict__ w,
-                                                        int64_t n, const double* __restrict__ vj, double a,
-                                                        const double* __restrict__ a_dev,
-                                                        const double* __restrict__ vjm1, double b,
-                                                        const double* __restrict__ b_dev, double* __restrict__ partial,
-                                                        double* __restrict__ out, unsigned* __restrict__ counter,
-                                                        const int* __restrict__ stop) {
+// Blocks per SM of k_kr_dots: registers for the loads of a row in flight.
+__host__ __device__ constexpr int kr_dots_per_sm(int ng) { return ng > 8 ? 2 : 3; }
+
+// w <- w - a vj - b vjm1 (LOCAL, written back), then out[i] = V_i^T w for the
+// NG columns of cp.  a and b from the device where a_dev / b_dev are given.
+// One instance per column count: the loads of a row (of several rows for few
+// columns) are then issued together, without a test per column; bound by the
+// FP64 unit (NG + 2 FMAs per row) from about 6 columns on, by memory below.
+template <int NG, bool LOCAL>
+__global__ void __launch_bounds__(KR_THREADS, kr_dots_per_sm(NG)) k_kr_dots(const __grid_constant__ KrCols cp, double* __restrict__ w,
+                                                           int64_t n, const double* __restrict__ vj, double a,
+                                                           const double* __restrict__ a_dev,
+                                                           const double* __restrict__ vjm1, double b,
+                                                           const double* __restrict__ b_dev,
+                                                           double* __restrict__ partial, double* __restrict__ out,
+                                                           unsigned* __restrict__ counter,
+                                                           const int* __restrict__ stop) {
+  constexpr int U = NG <= 3 ? 4 : NG <= 8 ? 2 : 1;  // rows in flight per thread
   if (stop && *stop) return;
   if (LOCAL && a_dev) a = *a_dev;
   if (LOCAL && b_dev) b = *b_dev;
@@ -85,28 +97,52 @@ __global__ void __launch_bounds__(KR_THREADS) k_kr_dots(const ColPtrsR cp, int v
 #pragma unroll
   for (int k = 0; k < KR_GROUP; ++k) acc[k] = 0.0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += stride) {
-    double wv = w[r];
-    if (LOCAL) {
-      wv = fma(-a, vj[r], wv);
-      if (vjm1) wv = fma(-b, vjm1[r], wv);
-      w[r] = wv;
+  int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (; r + (U - 1) * stride < n; r += U * stride) {
+    double v[U][NG], wv[U], p[U], q[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t ru = r + u * stride;
+      wv[u] = w[ru];
+      p[u] = LOCAL ? vj[ru] : 0.0;
+      q[u] = LOCAL && vjm1 ? vjm1[ru] : 0.0;
+#pragma unroll
+      for (int g = 0; g < NG; ++g) v[u][g] = cp.p[g][ru];
     }
 #pragma unroll
-    for (int g = 0; g < KR_GROUP; ++g)
-      if (g < ng) acc[g] = fma(cp.p[v0 + g][r], wv, acc[g]);
+    for (int u = 0; u < U; ++u) {
+      if (LOCAL) {
+        wv[u] = fma(-a, p[u], wv[u]);
+        if (vjm1) wv[u] = fma(-b, q[u], wv[u]);
+        w[r + u * stride] = wv[u];
+      }
+#pragma unroll
+      for (int g = 0; g < NG; ++g) acc[g] = fma(v[u][g], wv[u], acc[g]);
+    }
   }
-  __shared__ double sh[KR_GROUP * (KR_THREADS + 1)];
+  if (U > 1) {
+    for (; r < n; r += stride) {
+      double wv = w[r];
+      if (LOCAL) {
+        wv = fma(-a, vj[r], wv);
+        if (vjm1) wv = fma(-b, vjm1[r], wv);
+        w[r] = wv;
+      }
+#pragma unroll
+      for (int g = 0; g < NG; ++g) acc[g] = fma(cp.p[g][r], wv, acc[g]);
+    }
+  }
+  __shared__ double sh[NG * (KR_THREADS + 1)];
   const int item = threadIdx.x >> 4, l = threadIdx.x & 15;
-  const double s = block_sums16(acc, ng, sh);
-  if (l == 0 && item < ng) partial[(size_t)item * gridDim.x + blockIdx.x] = s;
+  const double s = block_sums16(acc, NG, sh);
+  if (l == 0 && item < NG) partial[(size_t)item * gridDim.x + blockIdx.x] = s;
   if (!ed_last_block(counter)) return;
   double t = 0.0;
-  if (item < ng)
+  if (item < NG)
     for (unsigned q = l; q < gridDim.x; q += 16) t += __ldcg(partial + (size_t)item * gridDim.x + q);
 #pragma unroll
   for (int k = 8; k > 0; k >>= 1) t += __shfl_down_sync(0xffffffffu, t, k, 16);
-  if (l == 0 && item < ng) out[v0 + item] = t;
+  if (l == 0 && item < NG) out[item] = t;
 }
 
 // ||w||^2, four rows in flight per thread.
@@ -270,15 +306,25 @@ static int kr_dots(ed_ctx* ctx, const double* const* cols, int nv, double* w, in
   ED_TRY(ed_ensure_reduce(ctx, (size_t)KR_GROUP * nblk + 256));
   ED_TRY(ed_ensure_counter(ctx));
   double* partial = ctx->d_red;
-  const ColPtrsR cp = kr_cols(cols, nv);
   for (int v0 = 0; v0 < nv; v0 += KR_GROUP) {
-    const int ng = std::min(KR_GROUP, nv - v0);
-    if (v0 == 0 && vj)
-      k_kr_dots<true><<<nblk, KR_THREADS, 0, ctx->stream>>>(cp, v0, ng, w, n, vj, a, a_dev, vjm1, b, b_dev, partial, out,
-                                                           ctx->d_counter, stop);
-    else
-      k_kr_dots<false><<<nblk, KR_THREADS, 0, ctx->stream>>>(cp, v0, ng, w, n, nullptr, 0.0, nullptr, nullptr, 0.0,
-                                                            nullptr, partial, out, ctx->d_counter, stop);
+    KrCols cp;
+    for (int i = 0; i < KR_GROUP; ++i) cp.p[i] = v0 + i < nv ? cols[v0 + i] : nullptr;
+    const bool local = v0 == 0 && vj;
+    if (!local) a_dev = b_dev = vjm1 = nullptr;
+    const int nb = kr_blocks(ctx, n, kr_dots_per_sm(std::min(KR_GROUP, nv - v0)));
+    auto go = [&](auto kern) {
+      kern<<<nb, KR_THREADS, 0, ctx->stream>>>(cp, w, n, local ? vj : nullptr, a, a_dev, vjm1, b, b_dev, partial,
+                                                 out + v0, ctx->d_counter, stop);
+    };
+#define KR_DOTS(NG)                                             \
+  case NG:                                                      \
+    local ? go(k_kr_dots<NG, true>) : go(k_kr_dots<NG, false>); \
+    break;
+    switch (std::min(KR_GROUP, nv - v0)) {
+      KR_DOTS(1) KR_DOTS(2) KR_DOTS(3) KR_DOTS(4) KR_DOTS(5) KR_DOTS(6) KR_DOTS(7) KR_DOTS(8)
+      KR_DOTS(9) KR_DOTS(10) KR_DOTS(11) KR_DOTS(12) KR_DOTS(13) KR_DOTS(14) KR_DOTS(15) KR_DOTS(16)
+    }
+#undef KR_DOTS
     ED_CHECK_LAUNCH(ctx);
   }
   return ED_OK;
