@@ -338,6 +338,9 @@ struct BCols {
 // lanes (consecutive b: coalesced) times 256 / Bp row lanes, and the row
 // lanes are summed in shared memory in a fixed order at the end.
 #define BD_MAXV 16
+// blocks per SM of the column-wise kernels: all resident at once (with four
+// and room for three, the fourth ran as a second, mostly empty wave)
+#define BD_PER_SM 3
 #define BU_REG 16  // k_batch_update_norm keeps up to this many coefficients in registers
 // With vj: first w <- w - a_b vj - bet_b vjm1 (coef = [a][B], [bet][B]),
 // written back, in the same pass (the local Lanczos projection).
@@ -345,7 +348,7 @@ struct BCols {
 // issued together, without a test per column.  More than BD_MAXV columns: the
 // first BD_MAXV here, the others by the caller's next launches (item0).
 template <int NI>
-__global__ void __launch_bounds__(256) k_batch_dots(const BCols V, int item0, double* __restrict__ w, int64_t dim,
+__global__ void __launch_bounds__(256, BD_PER_SM) k_batch_dots(const BCols V, int item0, double* __restrict__ w, int64_t dim,
                                                     int B, int norm_item, double* __restrict__ partial, int nblk,
                                                     const double* __restrict__ vj, const double* __restrict__ vjm1,
                                                     const double* __restrict__ coef, const int* __restrict__ pred) {
@@ -466,7 +469,7 @@ __global__ void __launch_bounds__(256) k_batch_update(const BCols V, int nv, con
 // partial[b * nblk + blk] (blocks over row ranges, lanes as in k_batch_dots).
 // partial[(B + b) * nblk + blk]: max_r |w[r, b]| over the block's rows.
 template <bool REG>
-__global__ void __launch_bounds__(256) k_batch_update_norm(const BCols V, int nv, const double* __restrict__ h,
+__global__ void __launch_bounds__(256, BD_PER_SM) k_batch_update_norm(const BCols V, int nv, const double* __restrict__ h,
                                                            double* __restrict__ w, int64_t dim, int B,
                                                            double* __restrict__ partial, int nblk,
                                                            const int* __restrict__ pred = nullptr) {
@@ -793,6 +796,10 @@ static int grid_n(ed_ctx* ctx, int64_t n, int per_sm = 8) {
   return (int)std::max<int64_t>(1, std::min(g, cap));
 }
 
+static int batch_blocks(ed_ctx* ctx, int64_t dim) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>(dim / 64 + 1, (int64_t)ctx->num_sms * BD_PER_SM));
+}
+
 static int batch_reduce_buf(ed_batch* bt, size_t doubles) {
   if (doubles <= bt->red_cap) return ED_OK;
   if (bt->d_red) cudaFree(bt->d_red);
@@ -812,7 +819,7 @@ static int batch_dots(ed_batch* bt, int B, const std::vector<const double*>& V, 
                       const double* coef = nullptr) {
   ed_ctx* ctx = bt->h->ctx;
   const int nv = (int)V.size();
-  const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>(bt->dim / 64 + 1, (int64_t)ctx->num_sms * 4));
+  const int nblk = batch_blocks(ctx, bt->dim);
   const int64_t items = (int64_t)(nv + 1) * B;
   ED_TRY(batch_reduce_buf(bt, (size_t)items * nblk + (size_t)items));
   ED_TRY(batch_dots_launch(ctx, nblk, V, w, bt->dim, B, norm ? nv : -1, bt->d_red, vj, vjm1, coef, nullptr));
@@ -832,7 +839,7 @@ static int batch_dots_dev(ed_batch* bt, int B, const std::vector<const double*>&
                           const double* vj, const double* vjm1, const double* coef, const int* pred) {
   ed_ctx* ctx = bt->h->ctx;
   const int nv = (int)V.size();
-  const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>(bt->dim / 64 + 1, (int64_t)ctx->num_sms * 4));
+  const int nblk = batch_blocks(ctx, bt->dim);
   const int64_t items = (int64_t)nv * B;
   ED_TRY(batch_reduce_buf(bt, (size_t)(items + B) * nblk + (size_t)items));
   ED_TRY(batch_dots_launch(ctx, nblk, V, w, bt->dim, B, -1, bt->d_red, vj, vjm1, coef, pred));
@@ -1223,7 +1230,7 @@ static int batch_solve_impl(ed_batch* bt, int nev, int ncv, double tol, int max_
     // sizes the buffers) are captured in a CUDA graph and replayed once.
     bool capture = bt->graphs && its > 1;
     if (capture) {
-      const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>(dim / 64 + 1, (int64_t)ctx->num_sms * 4));
+      const int nblk = batch_blocks(ctx, dim);
       const size_t nd = (size_t)m * A;
       const size_t need = std::max({(nd + A) * nblk + nd, (size_t)2 * A * nblk + 2 * (size_t)A,
                                     (size_t)2 * A * ((size_t)ctx->num_sms * 64) + 2 * (size_t)A});
@@ -1247,7 +1254,7 @@ static int batch_solve_impl(ed_batch* bt, int nev, int ncv, double tol, int max_
       BCols vc;
       memset(&vc, 0, sizeof(vc));
       for (int i = 0; i <= j; ++i) vc.p[i] = col[i];
-      const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>(dim / 64 + 1, (int64_t)ctx->num_sms * 4));
+      const int nblk = batch_blocks(ctx, dim);
       {
         // room for the dots' and the update's partials at once, so that no
         // call below moves the reduce buffer while res_upd points into it
