@@ -338,8 +338,13 @@ struct BCols {
 // lanes (consecutive b: coalesced) times 256 / Bp row lanes, and the row
 // lanes are summed in shared memory in a fixed order at the end.
 #define BD_MAXV 16
-// blocks per SM of the column-wise kernels: all resident at once (with four
-// and room for three, the fourth ran as a second, mostly empty wave)
+// Blocks per SM of the column-wise kernels, launched and resident.  Three leave
+// a thread up to 80 registers.  With four launched and no bound, the dots of 12
+// to 15 columns took 76-80 registers, so their fourth block waited for a second
+// wave; the other dots and the updates took at most 64 and all four fitted, but
+// the compiler had fewer registers to keep loads in flight with.  64 solves at
+// N=20, both trees in turn: 237.1 -> 231.2 ms (runs of one side within 0.1%),
+// again 242.6 -> 234.6 (within 2.9%).
 #define BD_PER_SM 3
 #define BU_REG 16  // k_batch_update_norm keeps up to this many coefficients in registers
 // With vj: first w <- w - a_b vj - bet_b vjm1 (coef = [a][B], [bet][B]),
