@@ -24,8 +24,8 @@
 // As FP64 FMAs it would be bound by the FP64 unit (7.4 ms at N=28), so it
 // runs on the tensor cores in exact 8-bit digits (k_corr_gram): 2.5 ms at
 // N=28 instead of 31.6 ms for 26 passes of 16 pairs before.  All S.S of the
-// N=28 state: 47.5 -> 3.2 ms; the energy gradient over 96 bonds at N=24:
-// 10.9 -> 0.34 ms.
+// N=28 state: 47.5 -> 2.9 ms; the energy gradient over 96 bonds at N=24:
+// 10.9 -> 0.30 ms.
 #include "ed_internal.h"
 #include "ed_device.cuh"
 #include "ed_halves.cuh"
@@ -427,7 +427,28 @@ __global__ void __launch_bounds__(GRAM_THREADS, 1) k_corr_gram(const unsigned lo
   // this CTA's stages: a contiguous piece, high halves innermost
   const int s0 = (int)((int64_t)nstages * blockIdx.x / gridDim.x);
   const int s1 = (int)((int64_t)nstages * (blockIdx.x + 1) / gridDim.x);
-  if (warp < GRAM_PROD) {
+  if (warp < GRAM_PROD && 2 * warp >= g.N) {
+    // Both sites lie past the last one: their digits are zero in every stage,
+    // so both buffers get them once.  The wait for empty stays: without it a
+    // warp could arrive twice in one phase of full.
+    // All pairs at N=28 (2 of 16 warps): 2.95 -> 2.88 ms; all bonds at N=24
+    // (4 of 16): 308 -> 295 us (the whole call).
+    const int site = 2 * warp + (lane >> 4), l = lane & 15;
+    for (int b = 0; b < 2; ++b)
+      for (int d = 0; d < GRAM_DIG; ++d)
+        *reinterpret_cast<uint4*>(smem + b * GRAM_STAGE + l * GRAM_LBO + site * 16 + d * (CR_SITES * 16)) =
+            make_uint4(0u, 0u, 0u, 0u);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    for (int s = s0; s < s1; ++s) {
+      const int it = s - s0, st = it & 1;
+      if (!mbar_wait(smem_u32(&S.empty[st]), ((it >> 1) & 1) ^ 1, TC_WAIT_POLLS)) {
+        atomicExch(err, 1);
+        break;
+      }
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&S.full[st])) : "memory");
+    }
+  } else if (warp < GRAM_PROD) {
     const int site = 2 * warp + (lane >> 4), l = lane & 15;
     const bool low = site < g.w0, high = !low && site < g.N;
     const uint32_t jbit = high ? 1u << (site - g.w0) : 0u;
