@@ -180,9 +180,14 @@ __device__ __forceinline__ int kr_emax_scaled(double absmax_hi, double s) {
 }
 
 // w <- w - sum_i V_i c_i with ||w||^2 and the high word of max |w|; the last
-// block then closes the step (see the top of the file).  Two rows per thread,
-// columns unrolled by four.
-__global__ void __launch_bounds__(KR_THREADS) k_kr_update(const ColPtrsR cp, int nv, double* __restrict__ w, int64_t n,
+// block then closes the step (see the top of the file).  One instance per
+// column count up to KR_GROUP: the loads of a row are issued together.  NV = 0:
+// any count, two rows per thread, columns unrolled by four.  Bound by the FP64
+// unit for large n, by the chain of latencies for small n: against NV = 0 for
+// every count, a solve of the 16-site chain (13k rows) 3.00 -> 2.93 ms, of the
+// N=28 lattice 476.9 -> 470.9 ms.
+template <int NV>
+__global__ void __launch_bounds__(KR_THREADS, NV > 8 ? 3 : 4) k_kr_update(const ColPtrsR cp, int nv, double* __restrict__ w, int64_t n,
                                                           double* __restrict__ partial, KrState* __restrict__ st,
                                                           const double* __restrict__ hv, int j,
                                                           int* __restrict__ gmax) {
@@ -193,25 +198,50 @@ __global__ void __launch_bounds__(KR_THREADS) k_kr_update(const ColPtrsR cp, int
   double acc[1] = {0.0};
   unsigned int amax = 0u;  // high word of max |w|
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t r0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r0 < n; r0 += 2 * stride) {
-    const int64_t r1 = r0 + stride;
-    const bool has1 = r1 < n;
-    double w0 = w[r0];
-    double w1 = has1 ? w[r1] : 0.0;
-#pragma unroll 4
-    for (int i = 0; i < nv; ++i) {
-      const double* col = cp.p[i];
-      const double c = sh_h[i];
-      w0 = fma(-col[r0], c, w0);
-      if (has1) w1 = fma(-col[r1], c, w1);
+  if (NV > 0) {
+    constexpr int U = NV <= 3 ? 4 : NV <= 8 ? 2 : 1;  // rows in flight per thread
+    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += U * stride) {
+      double v[U][NV + 1], x[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int64_t ru = r + u * stride;
+        const bool in = ru < n;
+        x[u] = in ? w[ru] : 0.0;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) v[u][i] = in ? cp.p[i][ru] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) x[u] = fma(-v[u][i], sh_h[i], x[u]);
+        if (r + u * stride < n) {
+          w[r + u * stride] = x[u];
+          acc[0] = fma(x[u], x[u], acc[0]);
+          amax = ed_absmax_hi(amax, x[u]);
+        }
+      }
     }
-    w[r0] = w0;
-    acc[0] = fma(w0, w0, acc[0]);
-    amax = ed_absmax_hi(amax, w0);
-    if (has1) {
-      w[r1] = w1;
-      acc[0] = fma(w1, w1, acc[0]);
-      amax = ed_absmax_hi(amax, w1);
+  } else {
+    for (int64_t r0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r0 < n; r0 += 2 * stride) {
+      const int64_t r1 = r0 + stride;
+      const bool has1 = r1 < n;
+      double w0 = w[r0];
+      double w1 = has1 ? w[r1] : 0.0;
+#pragma unroll 4
+      for (int i = 0; i < nv; ++i) {
+        const double* col = cp.p[i];
+        const double c = sh_h[i];
+        w0 = fma(-col[r0], c, w0);
+        if (has1) w1 = fma(-col[r1], c, w1);
+      }
+      w[r0] = w0;
+      acc[0] = fma(w0, w0, acc[0]);
+      amax = ed_absmax_hi(amax, w0);
+      if (has1) {
+        w[r1] = w1;
+        acc[0] = fma(w1, w1, acc[0]);
+        amax = ed_absmax_hi(amax, w1);
+      }
     }
   }
   __shared__ double sh[KR_THREADS];
@@ -361,8 +391,22 @@ int ed_kr_step(ed_ham* h, double* const* cols, int j, bool three_term, double* w
   ED_TRY(ed_launch_hv_dot_dev(h, cols[j], w, &hv));
   ED_TRY(kr_dots(ctx, cols, j + 1, w, n, cols[j], 0.0, hv, three_term ? cols[j - 1] : nullptr, 0.0,
                  three_term ? &st->beta[j - 1] : nullptr, st->c, &st->stop));
-  const int nblk = kr_blocks(ctx, n, 4);
-  k_kr_update<<<nblk, KR_THREADS, 0, ctx->stream>>>(kr_cols(cols, j + 1), j + 1, w, n, ctx->d_red, st, hv, j, h->d_gmax);
+  const int nv = j + 1;
+  const int nblk = kr_blocks(ctx, n, nv > 8 && nv <= KR_GROUP ? 3 : 4);  // all resident
+  auto update = [&](auto kern) {
+    kern<<<nblk, KR_THREADS, 0, ctx->stream>>>(kr_cols(cols, nv), nv, w, n, ctx->d_red, st, hv, j, h->d_gmax);
+  };
+#define KR_UPDATE(NV)         \
+  case NV:                    \
+    update(k_kr_update<NV>);  \
+    break;
+  switch (nv) {
+    KR_UPDATE(1) KR_UPDATE(2) KR_UPDATE(3) KR_UPDATE(4) KR_UPDATE(5) KR_UPDATE(6) KR_UPDATE(7) KR_UPDATE(8)
+    KR_UPDATE(9) KR_UPDATE(10) KR_UPDATE(11) KR_UPDATE(12) KR_UPDATE(13) KR_UPDATE(14) KR_UPDATE(15) KR_UPDATE(16)
+    default:
+      update(k_kr_update<0>);
+  }
+#undef KR_UPDATE
   ED_CHECK_LAUNCH(ctx);
   k_kr_scale<<<kr_blocks(ctx, n, 8), KR_THREADS, 0, ctx->stream>>>(w, cols[j + 1], n, st, ed_fx64_sbits(h),
                                                                  (long long*)h->d_xq);
