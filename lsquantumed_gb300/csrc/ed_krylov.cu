@@ -28,6 +28,50 @@ struct KrCols {
   const double* p[KR_GROUP];
 };
 
+// For short vectors (kr_dependent; DEP) the kernels of a step are launched as
+// programmatic dependents: the blocks of one become resident while the one
+// before drains.  A solve of the 16-site chain 2.91 -> 2.52 ms.  Each begins with kr_wait,
+// before it reads or writes any memory: it returns when the grid before has
+// completed and its writes are visible, so the order of the stream is kept.
+// Every block runs it, so a grid completes only after the one before it.
+__device__ __forceinline__ void kr_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Reads in these kernels go through kr_ld: the kernel before may still write
+// when a block becomes resident, so a read-only (.nc) load, which the compiler
+// may choose for a const restrict pointer and move above the wait, is not
+// allowed.  volatile keeps the order against kr_wait, .cg reads from L2.
+template <bool DEP>
+__device__ __forceinline__ double kr_ld(const double* p) {
+  if (!DEP) return *p;
+  double v;
+  asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+template <bool DEP>
+__device__ __forceinline__ int kr_ld(const int* p) {
+  if (!DEP) return *p;
+  int v;
+  asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+// lets the next grid's blocks become resident (they wait in kr_wait)
+__device__ __forceinline__ void kr_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... K, typename... A>
+static int kr_launch(ed_ctx* ctx, bool dep, void (*kern)(K...), int nblk, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)nblk);
+  cfg.blockDim = dim3(KR_THREADS);
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = dep ? 1 : 0;
+  ED_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<K>(args)...));
+  ctx->kernels++;
+  return ED_OK;
+}
+
 static ColPtrsR kr_cols(const double* const* cols, int nv) {
   ColPtrsR c;
   for (int i = 0; i < 128; ++i) c.p[i] = nullptr;
@@ -80,7 +124,7 @@ __host__ __device__ constexpr int kr_dots_per_sm(int ng) { return ng > 8 ? 2 : 3
 // One instance per column count: the loads of a row (of several rows for few
 // columns) are then issued together, without a test per column; bound by the
 // FP64 unit (NG + 2 FMAs per row) from about 6 columns on, by memory below.
-template <int NG, bool LOCAL>
+template <int NG, bool LOCAL, bool DEP>
 __global__ void __launch_bounds__(KR_THREADS, kr_dots_per_sm(NG)) k_kr_dots(const __grid_constant__ KrCols cp, double* __restrict__ w,
                                                            int64_t n, const double* __restrict__ vj, double a,
                                                            const double* __restrict__ a_dev,
@@ -90,9 +134,13 @@ __global__ void __launch_bounds__(KR_THREADS, kr_dots_per_sm(NG)) k_kr_dots(cons
                                                            unsigned* __restrict__ counter,
                                                            const int* __restrict__ stop) {
   constexpr int U = NG <= 3 ? 4 : NG <= 8 ? 2 : 1;  // rows in flight per thread
-  if (stop && *stop) return;
-  if (LOCAL && a_dev) a = *a_dev;
-  if (LOCAL && b_dev) b = *b_dev;
+  if (DEP) {
+    kr_next();
+    kr_wait();
+  }
+  if (stop && kr_ld<DEP>(stop)) return;
+  if (LOCAL && a_dev) a = kr_ld<DEP>(a_dev);
+  if (LOCAL && b_dev) b = kr_ld<DEP>(b_dev);
   double acc[KR_GROUP];
 #pragma unroll
   for (int k = 0; k < KR_GROUP; ++k) acc[k] = 0.0;
@@ -103,11 +151,11 @@ __global__ void __launch_bounds__(KR_THREADS, kr_dots_per_sm(NG)) k_kr_dots(cons
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int64_t ru = r + u * stride;
-      wv[u] = w[ru];
-      p[u] = LOCAL ? vj[ru] : 0.0;
-      q[u] = LOCAL && vjm1 ? vjm1[ru] : 0.0;
+      wv[u] = kr_ld<DEP>(w + ru);
+      p[u] = LOCAL ? kr_ld<DEP>(vj + ru) : 0.0;
+      q[u] = LOCAL && vjm1 ? kr_ld<DEP>(vjm1 + ru) : 0.0;
 #pragma unroll
-      for (int g = 0; g < NG; ++g) v[u][g] = cp.p[g][ru];
+      for (int g = 0; g < NG; ++g) v[u][g] = kr_ld<DEP>(cp.p[g] + ru);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -122,14 +170,14 @@ __global__ void __launch_bounds__(KR_THREADS, kr_dots_per_sm(NG)) k_kr_dots(cons
   }
   if (U > 1) {
     for (; r < n; r += stride) {
-      double wv = w[r];
+      double wv = kr_ld<DEP>(w + r);
       if (LOCAL) {
-        wv = fma(-a, vj[r], wv);
-        if (vjm1) wv = fma(-b, vjm1[r], wv);
+        wv = fma(-a, kr_ld<DEP>(vj + r), wv);
+        if (vjm1) wv = fma(-b, kr_ld<DEP>(vjm1 + r), wv);
         w[r] = wv;
       }
 #pragma unroll
-      for (int g = 0; g < NG; ++g) acc[g] = fma(cp.p[g][r], wv, acc[g]);
+      for (int g = 0; g < NG; ++g) acc[g] = fma(kr_ld<DEP>(cp.p[g] + r), wv, acc[g]);
     }
   }
   __shared__ double sh[NG * (KR_THREADS + 1)];
@@ -186,14 +234,18 @@ __device__ __forceinline__ int kr_emax_scaled(double absmax_hi, double s) {
 // unit for large n, by the chain of latencies for small n: against NV = 0 for
 // every count, a solve of the 16-site chain (13k rows) 3.00 -> 2.93 ms, of the
 // N=28 lattice 476.9 -> 470.9 ms.
-template <int NV>
+template <int NV, bool DEP>
 __global__ void __launch_bounds__(KR_THREADS, NV > 8 ? 3 : 4) k_kr_update(const ColPtrsR cp, int nv, double* __restrict__ w, int64_t n,
                                                           double* __restrict__ partial, KrState* __restrict__ st,
                                                           const double* __restrict__ hv, int j,
                                                           int* __restrict__ gmax) {
-  if (st->stop) return;
+  if (DEP) {
+    kr_next();
+    kr_wait();
+  }
+  if (kr_ld<DEP>(&st->stop)) return;
   __shared__ double sh_h[128];
-  for (int i = threadIdx.x; i < nv; i += blockDim.x) sh_h[i] = st->c[i];
+  for (int i = threadIdx.x; i < nv; i += blockDim.x) sh_h[i] = kr_ld<DEP>(&st->c[i]);
   __syncthreads();
   double acc[1] = {0.0};
   unsigned int amax = 0u;  // high word of max |w|
@@ -206,9 +258,9 @@ __global__ void __launch_bounds__(KR_THREADS, NV > 8 ? 3 : 4) k_kr_update(const 
       for (int u = 0; u < U; ++u) {
         const int64_t ru = r + u * stride;
         const bool in = ru < n;
-        x[u] = in ? w[ru] : 0.0;
+        x[u] = in ? kr_ld<DEP>(w + ru) : 0.0;
 #pragma unroll
-        for (int i = 0; i < NV; ++i) v[u][i] = in ? cp.p[i][ru] : 0.0;
+        for (int i = 0; i < NV; ++i) v[u][i] = in ? kr_ld<DEP>(cp.p[i] + ru) : 0.0;
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -225,14 +277,14 @@ __global__ void __launch_bounds__(KR_THREADS, NV > 8 ? 3 : 4) k_kr_update(const 
     for (int64_t r0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r0 < n; r0 += 2 * stride) {
       const int64_t r1 = r0 + stride;
       const bool has1 = r1 < n;
-      double w0 = w[r0];
-      double w1 = has1 ? w[r1] : 0.0;
+      double w0 = kr_ld<DEP>(w + r0);
+      double w1 = has1 ? kr_ld<DEP>(w + r1) : 0.0;
 #pragma unroll 4
       for (int i = 0; i < nv; ++i) {
         const double* col = cp.p[i];
         const double c = sh_h[i];
-        w0 = fma(-col[r0], c, w0);
-        if (has1) w1 = fma(-col[r1], c, w1);
+        w0 = fma(-kr_ld<DEP>(col + r0), c, w0);
+        if (has1) w1 = fma(-kr_ld<DEP>(col + r1), c, w1);
       }
       w[r0] = w0;
       acc[0] = fma(w0, w0, acc[0]);
@@ -275,13 +327,13 @@ __global__ void __launch_bounds__(KR_THREADS, NV > 8 ? 3 : 4) k_kr_update(const 
 #pragma unroll
   for (int k = 16; k > 0; k >>= 1) c2 += __shfl_down_sync(0xffffffffu, c2, k);
   if (threadIdx.x == 0) {
-    const double nw = sqrt(n2), mx = ed_absmax_hi_value(amax), y2 = hv[2];
+    const double nw = sqrt(n2), mx = ed_absmax_hi_value(amax), y2 = kr_ld<DEP>(hv + 2);
     const double s = 1.0 / nw;
     const int emax = kr_emax_scaled(mx, s);
     st->step = j;
     st->y2 = y2;
     st->wmax = mx;
-    st->alpha[j] = hv[0] + sh_h[j];
+    st->alpha[j] = kr_ld<DEP>(hv) + sh_h[j];
     st->beta[j] = nw;
     st->s = s;
     st->emax = emax;
@@ -304,16 +356,21 @@ __global__ void __launch_bounds__(KR_THREADS, NV > 8 ? 3 : 4) k_kr_update(const 
 
 // dst = w s and its fixed-point copy for the next H.v (k_scale_quantize_r with
 // the scale and exponent from the device).
+template <bool DEP>
 __global__ void __launch_bounds__(KR_THREADS) k_kr_scale(const double* __restrict__ w, double* __restrict__ dst,
                                                          int64_t n, const KrState* __restrict__ st, int sbits,
                                                          long long* __restrict__ xq) {
-  if (st->stop) return;
-  const double s = st->s;
-  const int emax = st->emax;
+  if (DEP) {
+    kr_next();
+    kr_wait();
+  }
+  if (kr_ld<DEP>(&st->stop)) return;
+  const double s = kr_ld<DEP>(&st->s);
+  const int emax = kr_ld<DEP>(&st->emax);
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t r0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r0 < n; r0 += 2 * stride) {
     const int64_t r1 = r0 + stride;
-    const double v0 = w[r0] * s, v1 = r1 < n ? w[r1] * s : 0.0;
+    const double v0 = kr_ld<DEP>(w + r0) * s, v1 = r1 < n ? kr_ld<DEP>(w + r1) * s : 0.0;
     dst[r0] = v0;
     xq[r0] = ed_fx64_entry(v0, emax, sbits);
     if (r1 < n) {
@@ -328,11 +385,20 @@ static int kr_blocks(ed_ctx* ctx, int64_t n, int per_sm) {
   return (int)std::max<int64_t>(1, std::min<int64_t>((n + KR_THREADS - 1) / KR_THREADS, (int64_t)ctx->num_sms * per_sm));
 }
 
+// Dependent launches pay where a kernel is hardly longer than the gap before
+// it; with long passes the L2 loads they need cost more than the gap.  Per step
+// of a 16-column solve on 152 SMs, plain -> dependent: 3432 rows 41.3 -> 35.2
+// us, 12870 45.7 -> 39.6, 48620 51.4 -> 47.1, 184756 69.2 -> 67.7, 705432 143.3
+// -> 144.1, 2704156 313-316 either way.  The line, 311296 rows there, is eight
+// rows per thread of one block per SM.
+static bool kr_dependent(const ed_ctx* ctx, int64_t n) { return n <= (int64_t)ctx->num_sms * KR_THREADS * 8; }
+
 // partials, results and the counter in the reduction buffer:
 // [items][nblk] | out[items] ; the counter is the context's
 static int kr_dots(ed_ctx* ctx, const double* const* cols, int nv, double* w, int64_t n, const double* vj, double a,
                    const double* a_dev, const double* vjm1, double b, const double* b_dev, double* out, const int* stop) {
   const int nblk = kr_blocks(ctx, n, 4);
+  const bool dep = kr_dependent(ctx, n);
   ED_TRY(ed_ensure_reduce(ctx, (size_t)KR_GROUP * nblk + 256));
   ED_TRY(ed_ensure_counter(ctx));
   double* partial = ctx->d_red;
@@ -342,20 +408,22 @@ static int kr_dots(ed_ctx* ctx, const double* const* cols, int nv, double* w, in
     const bool local = v0 == 0 && vj;
     if (!local) a_dev = b_dev = vjm1 = nullptr;
     const int nb = kr_blocks(ctx, n, kr_dots_per_sm(std::min(KR_GROUP, nv - v0)));
+    int rc = ED_OK;
     auto go = [&](auto kern) {
-      kern<<<nb, KR_THREADS, 0, ctx->stream>>>(cp, w, n, local ? vj : nullptr, a, a_dev, vjm1, b, b_dev, partial,
-                                                 out + v0, ctx->d_counter, stop);
+      rc = kr_launch(ctx, dep, kern, nb, cp, w, n, local ? vj : nullptr, a, a_dev, vjm1, b, b_dev, partial, out + v0,
+                     ctx->d_counter, stop);
     };
-#define KR_DOTS(NG)                                             \
-  case NG:                                                      \
-    local ? go(k_kr_dots<NG, true>) : go(k_kr_dots<NG, false>); \
+#define KR_DOTS(NG)                                                                 \
+  case NG:                                                                          \
+    if (dep) local ? go(k_kr_dots<NG, true, true>) : go(k_kr_dots<NG, false, true>); \
+    else local ? go(k_kr_dots<NG, true, false>) : go(k_kr_dots<NG, false, false>);   \
     break;
     switch (std::min(KR_GROUP, nv - v0)) {
       KR_DOTS(1) KR_DOTS(2) KR_DOTS(3) KR_DOTS(4) KR_DOTS(5) KR_DOTS(6) KR_DOTS(7) KR_DOTS(8)
       KR_DOTS(9) KR_DOTS(10) KR_DOTS(11) KR_DOTS(12) KR_DOTS(13) KR_DOTS(14) KR_DOTS(15) KR_DOTS(16)
     }
 #undef KR_DOTS
-    ED_CHECK_LAUNCH(ctx);
+    ED_TRY(rc);
   }
   return ED_OK;
 }
@@ -392,25 +460,25 @@ int ed_kr_step(ed_ham* h, double* const* cols, int j, bool three_term, double* w
   ED_TRY(kr_dots(ctx, cols, j + 1, w, n, cols[j], 0.0, hv, three_term ? cols[j - 1] : nullptr, 0.0,
                  three_term ? &st->beta[j - 1] : nullptr, st->c, &st->stop));
   const int nv = j + 1;
+  const bool dep = kr_dependent(ctx, n);
   const int nblk = kr_blocks(ctx, n, nv > 8 && nv <= KR_GROUP ? 3 : 4);  // all resident
+  int rc = ED_OK;
   auto update = [&](auto kern) {
-    kern<<<nblk, KR_THREADS, 0, ctx->stream>>>(kr_cols(cols, nv), nv, w, n, ctx->d_red, st, hv, j, h->d_gmax);
+    rc = kr_launch(ctx, dep, kern, nblk, kr_cols(cols, nv), nv, w, n, ctx->d_red, st, hv, j, h->d_gmax);
   };
-#define KR_UPDATE(NV)         \
-  case NV:                    \
-    update(k_kr_update<NV>);  \
+#define KR_UPDATE(NV)                                                    \
+  case NV:                                                               \
+    dep ? update(k_kr_update<NV, true>) : update(k_kr_update<NV, false>); \
     break;
   switch (nv) {
     KR_UPDATE(1) KR_UPDATE(2) KR_UPDATE(3) KR_UPDATE(4) KR_UPDATE(5) KR_UPDATE(6) KR_UPDATE(7) KR_UPDATE(8)
     KR_UPDATE(9) KR_UPDATE(10) KR_UPDATE(11) KR_UPDATE(12) KR_UPDATE(13) KR_UPDATE(14) KR_UPDATE(15) KR_UPDATE(16)
     default:
-      update(k_kr_update<0>);
+      dep ? update(k_kr_update<0, true>) : update(k_kr_update<0, false>);
   }
 #undef KR_UPDATE
-  ED_CHECK_LAUNCH(ctx);
-  k_kr_scale<<<kr_blocks(ctx, n, 8), KR_THREADS, 0, ctx->stream>>>(w, cols[j + 1], n, st, ed_fx64_sbits(h),
-                                                                 (long long*)h->d_xq);
-  ED_CHECK_LAUNCH(ctx);
+  ED_TRY(rc);
+  ED_TRY(kr_launch(ctx, dep, dep ? k_kr_scale<true> : k_kr_scale<false>, kr_blocks(ctx, n, 8), w, cols[j + 1], n, st, ed_fx64_sbits(h), (long long*)h->d_xq));
   h->xq_src = cols[j + 1];
   return ED_OK;
 }

@@ -22,8 +22,11 @@ def ed():
     return ed
 
 
-@pytest.mark.parametrize('lx,ly,mag', [(2, 4, 0), (4, 3, 0), (4, 3, 2), (4, 4, 0)])
-@pytest.mark.parametrize('ncv', [6, 8, 9, 10, 15, 16, 17, 18, 24, 40])
+# the last two: 319770 and 170544 rows, plain and dependent launches
+@pytest.mark.parametrize('lx,ly,mag,ncv', [
+    (lx, ly, mag, ncv) for lx, ly, mag in [(2, 4, 0), (4, 3, 0), (4, 3, 2), (4, 4, 0)]
+    for ncv in [6, 8, 9, 10, 15, 16, 17, 18, 24, 40]
+] + [(2, 11, 3, 16), (2, 11, 3, 18), (2, 11, 4, 16), (2, 11, 4, 18)])
 def test_ground_state_over_subspace_sizes(ed, lx, ly, mag, ncv):
     import oracle
     N = lx * ly
