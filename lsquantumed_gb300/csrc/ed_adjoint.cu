@@ -239,8 +239,9 @@ static int mixed(const ed_basis* b, const double2* lam, const double2* psi, cons
         const int i = ij[2 * t], j = ij[2 * t + 1];
         double v = 0.0;
         if (kinds[t] == T_Z) v = c.sz(i);
-        if (kinds[t] == T_ZZ || kinds[t] == T_SISJ) v = 0.25 * c.zz(i, j);
-        if (kinds[t] == T_XY || kinds[t] == T_SISJ) v += i == j ? 0.5 * c.zz(i, i) : c.F[f++];
+        if (kinds[t] == T_ZZ) v = 0.25 * c.zz(i, j);
+        if (kinds[t] == T_XY) v = i == j ? 0.5 * c.zz(i, i) : c.F[f++];
+        if (kinds[t] == T_SISJ) v = i == j ? 0.75 * c.zz(i, i) : c.sisj(i, j, (int64_t)f++);
         out[t] = make_double2(v, 0.0);
       }
       return ED_OK;

@@ -791,14 +791,36 @@ double i128_to_double(u128 z) {
   return neg ? -d : d;
 }
 
+// The nearest double and what is left of z, as a double (|z| below 2^126).
+double i128_split(u128 z, double& rest) {
+  const double d = (double)(__int128)z;
+  rest = (double)((__int128)z - (__int128)d);
+  return d;
+}
+
+// T - 2 A, A = the weight of the antiparallel states of (i, j)
+u128 zz_sum(const ed_corr& c, int i, int j) {
+  const int a = std::max(i, j), b = std::min(i, j);
+  const u128 A = c.P[a * (a + 1) / 2 + a] + c.P[b * (b + 1) / 2 + b] - 2 * c.P[a * (a + 1) / 2 + b];
+  return c.T - 2 * A;
+}
+
 }  // namespace
 
 double ed_corr::zz(int i, int j) const {
   if (i == j) return i128_to_double(T) * inv_scale;
-  const int a = std::max(i, j), b = std::min(i, j);
-  // T - 2 A, A = the weight of the antiparallel states
-  const u128 A = P[a * (a + 1) / 2 + a] + P[b * (b + 1) / 2 + b] - 2 * P[a * (a + 1) / 2 + b];
-  return i128_to_double(T - 2 * A) * inv_scale;
+  return i128_to_double(zz_sum(*this, i, j)) * inv_scale;
+}
+
+// Both parts are exact integers (Gram form).  Rounded apart and then added, the
+// root mean square error at N=20 was 6% above that of an FP64 flip sum; rounded
+// once it is 1.62e-17 of the largest value, as with the FP64 sum.
+double ed_corr::sisj(int i, int j, int64_t q) const {
+  double zl;
+  const double f = 0.25 * inv_scale, z = i128_split(zz_sum(*this, i, j), zl) * f;
+  const double s = z + F[q], t = s - z;
+  const double e = (z - (s - t)) + (F[q] - t);  // z + F = s + e (Knuth's TwoSum)
+  return s + (e + (zl * f + Fl[q]));
 }
 
 double ed_corr::up(int i) const { return i128_to_double(P[i * (i + 1) / 2 + i]) * inv_scale; }
@@ -949,6 +971,7 @@ int ed_corr_real(const ed_basis* b, const double2* lam, const double2* psi, bool
     out.T = get(o_P + 16 * (size_t)npairs);
   }
   out.F.assign(np, 0.0);
+  out.Fl.assign(np, 0.0);
   for (size_t t = 0; t < flips.size(); ++t) {
     const int i = pairs[2 * flips[t]], j = pairs[2 * flips[t] + 1];
     if (few) {
@@ -957,7 +980,10 @@ int ed_corr_real(const ed_basis* b, const double2* lam, const double2* psi, bool
       // F 2^(2 (54 - E) - 24), E = emax - 1022
       const u128 x = get(o_G + 16 * (size_t)(i * 32 + j)) + get(o_G + 16 * (size_t)(1024 + i * 32 + j)) +
                      get(o_G + 16 * (size_t)(1024 + j * 32 + i));
-      out.F[flips[t]] = std::ldexp((double)(__int128)x, 2 * (hh.emax - 1022) - 108 + 24);
+      const int sh = 2 * (hh.emax - 1022) - 108 + 24;
+      double rest;
+      out.F[flips[t]] = std::ldexp(i128_split(x, rest), sh);
+      out.Fl[flips[t]] = std::ldexp(rest, sh);
     }
   }
   return ED_OK;

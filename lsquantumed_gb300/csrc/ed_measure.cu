@@ -156,8 +156,8 @@ int ed_launch_expect_pairs(const ed_basis* b, int op, const double2* psi, const 
     for (int64_t p = 0; p < np; ++p) {
       const int i = pairs[2 * p], j = pairs[2 * p + 1];
       double v = 0.0;
-      if (op == ED_OP_SZSZ || op == ED_OP_SISJ) v = 0.25 * c.zz(i, j);
-      if (op == ED_OP_SISJ) v += i == j ? 0.5 * c.zz(i, i) : c.F[p];  // (S+S- + S-S+) / 2
+      if (op == ED_OP_SZSZ) v = 0.25 * c.zz(i, j);
+      if (op == ED_OP_SISJ) v = i == j ? 0.75 * c.zz(i, i) : c.sisj(i, j, p);  // + (S+S- + S-S+) / 2
       if (op == ED_OP_SPSM) v = i == j ? c.up(i) : c.F[p];
       if (op == ED_OP_SMSP) v = i == j ? c.down(i) : c.F[p];
       out[p] = make_double2(v, 0.0);
