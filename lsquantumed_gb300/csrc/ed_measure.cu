@@ -588,9 +588,9 @@ static int dsf_runs(const ed_basis* b0, const ed_basis* b1, int op, const double
   memcpy(&h_imag, res.data(), sizeof(int));
   if (REAL && h_imag) return ED_ENOTSUP;
   const double2* h = (const double2*)(res.data() + o_c);
-  if (REAL)
-    for (int64_t q = 0; q < (int64_t)N * nev; ++q)
-      if (!std::isfinite(h[q].x)) return ED_ENOTSUP;
+  // compensated sums make NaN of an infinity: the general kernel answers
+  for (int64_t q = 0; q < (int64_t)N * nev; ++q)
+    if (!std::isfinite(h[q].x) || !std::isfinite(h[q].y)) return ED_ENOTSUP;
   for (int n = 0; n < nev; ++n)
     for (int i = 0; i < N; ++i) c_host[(size_t)i * nev + n] = h[(size_t)n * N + i];
   return ED_OK;

@@ -84,3 +84,26 @@ def test_expect_mixed_groups(ed, N, nterms, cplx):
         o = {ed.Adjoint.XY: 0.5 * flip, ed.Adjoint.ZZ: zz, ed.Adjoint.Z: np.where(bi, 0.5, -0.5) * psi,
              ed.Adjoint.SISJ: zz + 0.5 * flip}[kind]
         assert abs(got[t] - np.vdot(lam, o)) <= 2.0 ** -52 * b.size, (t, terms[t])
+
+
+@pytest.mark.parametrize('cplx', [False, True])
+def test_dsf_infinite_entry(ed, cplx):
+    """An infinite amplitude in row r gives sign(bit i of r) * conj(v_r) * inf
+    at every site i, not NaN (real part; the imaginary part too where v and
+    psi are complex with finite, nonzero parts)."""
+    import torch
+    N, r = 12, 7
+    env = ed.Environment(nspins=N)
+    b = ed.Basis(env, 0)
+    g = np.random.default_rng(3)
+    psi = g.standard_normal(b.size) + (1j * g.standard_normal(b.size) if cplx else 0j)
+    V = g.standard_normal((2, b.size)) + (1j * g.standard_normal((2, b.size)) if cplx else 0j)
+    psi[r] = complex(np.inf, psi[r].imag)
+    c = ed.Phys.dsf_coefficients(env, b, b, 0, torch.tensor(psi, device='cuda'), torch.tensor(V, device='cuda'))
+    s = int(b.int_basis[r])
+    for i in range(N):
+        sg = 1.0 if (s >> i) & 1 else -1.0
+        for n in range(2):
+            assert c[i, n].real == sg * np.sign(V[n, r].real) * np.inf
+            if cplx:
+                assert c[i, n].imag == -sg * np.sign(V[n, r].imag) * np.inf
