@@ -279,11 +279,28 @@ static int dsf_k(const ed_basis* b0, const ed_basis* b1, int op, const double2* 
 // Both take DZ_V vectors at a time, so psi is read once per DZ_V.
 // Real vectors (eigenvectors of the real H) need only the products of the
 // real parts; any nonzero imaginary part raises *imag and the host runs the
-// complex form.  N=24, ten vectors: 3.78 -> 0.38 ms (k_dsfz_high 0.17,
-// k_dsfz_low 0.15; the two reads of the vectors, 0.95 GB, take 0.14).
+// complex form.
+// The signed sums cancel, so the large unsigned ones may not round: the warps'
+// sums are joined as pairs, a column's rows in chains of DZ_ROWS joined as
+// pairs, and the 256 columns of a block as exact integers.  With plain FP64
+// there the root mean square error against quad sums was up to 18% above
+// k_dsf's; with it, N=20, 12 real / complex states: 0.66-0.74e-16 / 0.92-1.0e-16
+// of the largest value against 0.92-0.97e-16 / 1.0-1.2e-16.  N=24, ten vectors:
+// 3.8 ms with k_dsf, 0.374 with plain sums, 0.394 so (the two reads of the
+// vectors, 0.95 GB, take 0.14).
 // ---------------------------------------------------------------------------
 #define DZ_V 5
 #define DZ_SEG 32
+#define DZ_BITS 54
+#define DZ_ROWS 16  // rows of k_dsfz_low per plain FP64 chain
+
+// (h, l) + x as an unevaluated pair (Knuth's TwoSum): the signed sums cancel,
+// so the few large partial sums here decide the rounding of the result
+__device__ __forceinline__ void dsf_add(double& h, double& l, double x, double xl) {
+  const double t = __dadd_rn(h, x), z = __dsub_rn(t, h);
+  l = __dadd_rn(l, __dadd_rn(__dadd_rn(__dsub_rn(h, __dsub_rn(t, z)), __dsub_rn(x, z)), xl));
+  h = t;
+}
 
 // partial[(((n * gridDim.x) + blk) * 32 + j) * 2]: re, im of site w0 + j
 template <bool REAL>
@@ -347,7 +364,11 @@ __global__ void __launch_bounds__(128) k_dsfz_high(const double2* __restrict__ p
   __syncthreads();
   for (int v = wid; v < nv; v += 4) {
     double* d = partial + (((size_t)(n0 + v) * gridDim.x + blockIdx.x) * 32 + lane) * 2;
-    for (int c = 0; c < 2; ++c) d[c] = (sh[c][v][0][lane] + sh[c][v][1][lane]) + (sh[c][v][2][lane] + sh[c][v][3][lane]);
+    for (int c = 0; c < 2; ++c) {
+      double h = sh[c][v][0][lane], l = 0.0;
+      for (int w = 1; w < 4; ++w) dsf_add(h, l, sh[c][v][w][lane], 0.0);
+      d[c] = h + l;
+    }
   }
 }
 
@@ -366,7 +387,9 @@ __global__ void __launch_bounds__(256) k_dsfz_low(const double2* __restrict__ ps
   const int n0 = blockIdx.y * DZ_V, nv = min(DZ_V, nev - n0);
   __shared__ uint32_t base[DZ_SEG];
   __shared__ uint16_t c0[256];
-  __shared__ double sh[REAL ? 1 : 2][DZ_V][256];
+  __shared__ double sh[REAL ? 1 : 2][DZ_V][256];  // then the same as fixed point
+  __shared__ int emax[REAL ? 1 : 2][DZ_V];
+  if (threadIdx.x < (REAL ? 1 : 2) * DZ_V) (&emax[0][0])[threadIdx.x] = 0;
   if (threadIdx.x < nh) base[threadIdx.x] = t1[highs[g.high_off[k] + h0 + threadIdx.x]];
   const bool on = o < g.nlow[k];
   c0[threadIdx.x] = on ? lows[g.low_off[k] + o] : (uint16_t)0;
@@ -376,8 +399,20 @@ __global__ void __launch_bounds__(256) k_dsfz_low(const double2* __restrict__ ps
   for (int v = 0; v < DZ_V; ++v) ar[v] = ai[v] = 0.0;
   if (on) {
     const double2* q = vecs + (size_t)n0 * dim;
+    double sr[DZ_V], si[DZ_V], lr[DZ_V], li[DZ_V];  // chains of DZ_ROWS joined as pairs
+#pragma unroll
+    for (int v = 0; v < DZ_V; ++v) sr[v] = si[v] = lr[v] = li[v] = 0.0;
+    auto join = [&]() {
+#pragma unroll
+      for (int v = 0; v < DZ_V; ++v) {
+        dsf_add(sr[v], lr[v], ar[v], 0.0);
+        if (!REAL) dsf_add(si[v], li[v], ai[v], 0.0);
+        ar[v] = ai[v] = 0.0;
+      }
+    };
 #pragma unroll 2
     for (int h = 0; h < nh; ++h) {
+      if (h > 0 && h % DZ_ROWS == 0) join();
       const size_t r = (size_t)base[h] + o;
       const double2 x = psi[r];
       double2 y[DZ_V];
@@ -393,41 +428,61 @@ __global__ void __launch_bounds__(256) k_dsfz_low(const double2* __restrict__ ps
         }
       }
     }
-  }
+    join();
 #pragma unroll
-  for (int v = 0; v < DZ_V; ++v) {
-    sh[0][v][threadIdx.x] = ar[v];
-    if (!REAL) sh[REAL ? 0 : 1][v][threadIdx.x] = ai[v];
+    for (int v = 0; v < DZ_V; ++v) {
+      ar[v] = sr[v] + lr[v];
+      ai[v] = si[v] + li[v];
+    }
   }
+  // The signed sums cancel: exact, as 54-bit integers against the block's
+  // largest column (256 of them stay below 2^62), rounded once.  FP64 adds are
+  // the scarcer unit too.  A column that is not finite: in FP64, as it was.
+#pragma unroll
+  for (int v = 0; v < DZ_V; ++v)
+#pragma unroll
+    for (int c = 0; c < (REAL ? 1 : 2); ++c) {
+      const int e = (int)(((unsigned long long)__double_as_longlong(c ? ai[v] : ar[v]) >> 52) & 0x7FF);
+      const int m = (int)__reduce_max_sync(0xffffffffu, (unsigned)e);
+      if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(&emax[c][v], m);
+    }
+  __syncthreads();
+#pragma unroll
+  for (int v = 0; v < DZ_V; ++v)
+#pragma unroll
+    for (int c = 0; c < (REAL ? 1 : 2); ++c) {
+      const double x = c ? ai[v] : ar[v];
+      sh[c][v][threadIdx.x] =
+          emax[c][v] == 0x7FF ? x : __longlong_as_double(ed_fx64_entry(x, emax[c][v], DZ_BITS));
+    }
   __syncthreads();
   // 16 threads per site: signed sums of the 256 columns
   const int i = threadIdx.x >> 4, l = threadIdx.x & 15;
   for (int v = 0; v < nv; ++v) {
-    double r = 0.0, m = 0.0;
-    for (int c = l; c < 256; c += 16) {
-      const bool up = (c0[c] >> i) & 1;
-      r += up ? sh[0][v][c] : -sh[0][v][c];
-      if (!REAL) m += up ? sh[REAL ? 0 : 1][v][c] : -sh[REAL ? 0 : 1][v][c];
-    }
+    double rm[2] = {0.0, 0.0};
 #pragma unroll
-    for (int s = 8; s > 0; s >>= 1) {
-      r += __shfl_down_sync(0xffffffffu, r, s, 16);
-      if (!REAL) m += __shfl_down_sync(0xffffffffu, m, s, 16);
+    for (int p = 0; p < (REAL ? 1 : 2); ++p) {
+      if (emax[p][v] == 0x7FF) {
+        for (int c = l; c < 256; c += 16) rm[p] += ((c0[c] >> i) & 1) ? sh[p][v][c] : -sh[p][v][c];
+#pragma unroll
+        for (int s = 8; s > 0; s >>= 1) rm[p] += __shfl_down_sync(0xffffffffu, rm[p], s, 16);
+      } else {
+        long long q = 0;
+        for (int c = l; c < 256; c += 16) {
+          const long long x = __double_as_longlong(sh[p][v][c]);
+          q += ((c0[c] >> i) & 1) ? x : -x;
+        }
+#pragma unroll
+        for (int s = 8; s > 0; s >>= 1) q += __shfl_down_sync(0xffffffffu, q, s, 16);
+        rm[p] = ldexp((double)q, emax[p][v] - 1022 - DZ_BITS);
+      }
     }
     if (l == 0) {
       double* d = partial + (((size_t)(n0 + v) * gridDim.x + blockIdx.x) * 16 + i) * 2;
-      d[0] = r;
-      d[1] = m;
+      d[0] = rm[0];
+      d[1] = rm[1];
     }
   }
-}
-
-// (h, l) + x as an unevaluated pair (Knuth's TwoSum): the signed sums cancel,
-// so the few large partial sums here decide the rounding of the result
-__device__ __forceinline__ void dsf_add(double& h, double& l, double x, double xl) {
-  const double t = __dadd_rn(h, x), z = __dsub_rn(t, h);
-  l = __dadd_rn(l, __dadd_rn(__dadd_rn(__dsub_rn(h, __dsub_rn(t, z)), __dsub_rn(x, z)), xl));
-  h = t;
 }
 
 // c[n * N + i] = f sum over the blocks of site i's partials (low sites in
