@@ -504,7 +504,10 @@ int ed_bv_mult_real(ed_ctx* ctx, const double* const* V_dev, int m, const double
     return ed_fail(ED_EINVAL, "unknown restart arithmetic");
   if (arith == ED_RESTART_EXACT && m > 32) return ed_fail(ED_ENOTSUP, "the exact restart takes at most 32 vectors");
   ED_CUDA(cudaSetDevice(ctx->device));
-  return ed_restart_combine_r(ctx, V_dev, m, Y_host, ldY, l, out_dev, n, arith);
+  ED_TRY(ed_restart_combine_r(ctx, V_dev, m, Y_host, ldY, l, out_dev, n, arith));
+  // not every form waits; the solver's own calls need no wait, this one promises it
+  ED_CUDA(cudaStreamSynchronize(ctx->stream));
+  return ED_OK;
 }
 
 int ed_bv_dot_real(ed_ctx* ctx, const double* const* V_dev, int m, const double* w_dev, int64_t n, int arith,
