@@ -355,7 +355,6 @@ static int expand_queued(ed_eps* e, KrState* st, int k, int m, std::vector<doubl
     const int j = last;
     H->xq_src = nullptr;  // the queue made no copy for the steps behind
     ED_CUDA(cudaMemsetAsync(&st->stop, 0, sizeof(int), ctx->stream));
-    ED_CUDA(cudaMemsetAsync(H->d_gmax + ED_HV_SKIP, 0, sizeof(int), ctx->stream));
     double nw = s.beta[j], wmax = s.wmax;
     if (s.stop == KR_REFINE) {  // the second pass (DGKS)
       std::vector<const double*> cols(e->col_r.begin(), e->col_r.begin() + j + 1);

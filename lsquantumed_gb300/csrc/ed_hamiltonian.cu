@@ -890,7 +890,7 @@ int ed_launch_hv_dot(ed_ham* h, const double2* x, double2* y, double2* dot, doub
   return ed_launch_hv_dot_any(h, x, y, false, dot, y2);
 }
 
-static int launch_hv_dot(ed_ham* h, const void* x, void* y, bool rio) {
+static int launch_hv_dot(ed_ham* h, const void* x, void* y, bool rio, const int* skip = nullptr) {
   ed_ctx* ctx = h->ctx;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (ctx->profiling) {
@@ -899,7 +899,7 @@ static int launch_hv_dot(ed_ham* h, const void* x, void* y, bool rio) {
     ED_CUDA(cudaEventRecord(e0, ctx->stream));
   }
   int nblk = 0;
-  ED_TRY(ed_launch_hv_lin(h, x, y, true, &nblk, rio));
+  ED_TRY(ed_launch_hv_lin(h, x, y, true, &nblk, rio, skip));
   if (ctx->profiling) {
     ED_CUDA(cudaEventRecord(e1, ctx->stream));
     ctx->prof_events.push_back(e0);
@@ -908,9 +908,9 @@ static int launch_hv_dot(ed_ham* h, const void* x, void* y, bool rio) {
   return ED_OK;
 }
 
-int ed_launch_hv_dot_dev(ed_ham* h, const double* x, double* y, const double** sums) {
+int ed_launch_hv_dot_dev(ed_ham* h, const double* x, double* y, const int* skip, const double** sums) {
   if (!ed_lin_supported(h)) return ED_ENOTSUP;
-  ED_TRY(launch_hv_dot(h, x, y, true));
+  ED_TRY(launch_hv_dot(h, x, y, true, skip));
   *sums = (const double*)(h->d_gmax + ED_HV_SUMS);
   return ED_OK;
 }

@@ -216,9 +216,9 @@ __device__ __forceinline__ void body(const u32* __restrict__ states, const doubl
                                      const D2* __restrict__ x, const L2* __restrict__ xq,
                                      int* __restrict__ gmax_p, int sbits, D2* __restrict__ y, i64 dim,
                                      const unsigned short* __restrict__ t0, const u32* __restrict__ t1, const uint4* __restrict__ t1n, double c0c,
-                                     double c1c, double* __restrict__ partial) {
+                                     double c1c, double* __restrict__ partial, const int* __restrict__ skip) {
   extern __shared__ unsigned short t0s[];
-  if (gmax_p[3]) return;  // skip: a step before this one stopped
+  if (skip && *skip) return;  // a step before this one stopped
   for (int i = threadIdx.x; i < (1 << W0); i += blockDim.x) t0s[i] = t0[SWZ((u32)i)];
   __syncthreads();
   const int e_unit = gmax_p[0] - 1022 - sbits;
@@ -256,8 +256,8 @@ __device__ __forceinline__ void body(const u32* __restrict__ states, const doubl
 #define JIT_KERNEL(NAME, DOT, RIO, NT, MINB)                                                              \
   extern "C" __global__ void __launch_bounds__(NT, MINB) NAME(const u32* states, const double* diag,        \
       const D2* x, const L2* xq, int* gmax_p, int sbits, D2* y, i64 dim, const unsigned short* t0,     \
-      const u32* t1, const uint4* t1n, double c0c, double c1c, double* partial) {                                             \
-    body<DOT, RIO>(states, diag, x, xq, gmax_p, sbits, y, dim, t0, t1, t1n, c0c, c1c, partial);                  \
+      const u32* t1, const uint4* t1n, double c0c, double c1c, double* partial, const int* skip) {                            \
+    body<DOT, RIO>(states, diag, x, xq, gmax_p, sbits, y, dim, t0, t1, t1n, c0c, c1c, partial, skip);            \
   }
 // register budgets: 2, 3 or 4 blocks of 256 per SM (128, 80 or 64 registers);
 // _r: real storage of x and y
@@ -409,9 +409,10 @@ __device__ __forceinline__ void body(const u32* __restrict__ states, const doubl
                                      const D2* __restrict__ x, const L2* __restrict__ xq,
                                      int* __restrict__ gmax_p, int sbits, D2* __restrict__ y, i64 dim,
                                      const unsigned short* __restrict__ t0, const u32* __restrict__ t1, const uint4* __restrict__ t1n, int pbexp,
-                                     double* __restrict__ partial, const PBC& pbc, const i64* __restrict__ gcf) {
+                                     double* __restrict__ partial, const PBC& pbc, const i64* __restrict__ gcf,
+                                     const int* __restrict__ skip) {
   extern __shared__ unsigned short t0s[];
-  if (gmax_p[3]) return;  // skip: a step before this one stopped
+  if (skip && *skip) return;  // a step before this one stopped
   for (int i = threadIdx.x; i < (1 << W0); i += blockDim.x) t0s[i] = t0[SWZ((u32)i)];
   __syncthreads();
   const int xexp = gmax_p[0] - 1022 - sbits + pbexp;
@@ -447,8 +448,9 @@ __device__ __forceinline__ void body(const u32* __restrict__ states, const doubl
 #define JIT_KERNEL(NAME, DOT, RIO, NT, MINB)                                                              \
   extern "C" __global__ void __launch_bounds__(NT, MINB) NAME(const u32* states, const double* diag,        \
       const D2* x, const L2* xq, int* gmax_p, int sbits, D2* y, i64 dim, const unsigned short* t0,     \
-      const u32* t1, const uint4* t1n, int pbexp, double* partial, const __grid_constant__ PBC pbc, const i64* gcf) {         \
-    body<DOT, RIO>(states, diag, x, xq, gmax_p, sbits, y, dim, t0, t1, t1n, pbexp, partial, pbc, gcf);           \
+      const u32* t1, const uint4* t1n, int pbexp, double* partial, const __grid_constant__ PBC pbc, const i64* gcf,           \
+      const int* skip) {                                                                                       \
+    body<DOT, RIO>(states, diag, x, xq, gmax_p, sbits, y, dim, t0, t1, t1n, pbexp, partial, pbc, gcf, skip);     \
   }
 JIT_KERNEL(k_hv_jit_b2, false, false, 256, 2)
 JIT_KERNEL(k_hv_jit_dot_b2, true, false, 256, 2)
@@ -609,7 +611,7 @@ bool ed_jit_available() {
 // Signature of the operator's bond words (the same hash the autotuner keys on).
 int ed_jit_launch(ed_ham* h, uint64_t signature, int budget, const void* x, void* y, bool dot, int sbits,
                   int* nblk_out, const unsigned long long* words, const int* seg, int w0, bool rio,
-                  const long long* coef, const long long* coef_dev, int pbexp) {
+                  const long long* coef, const long long* coef_dev, int pbexp, const int* skip) {
   ed_ctx* ctx = h->ctx;
   const ed_basis* b = h->basis;
   JitModule* mod = nullptr;
@@ -775,11 +777,11 @@ int ed_jit_launch(ed_ham* h, uint64_t signature, int budget, const void* x, void
   double c0c = h->bs.chalf[0], c1c = h->bs.chalf[1];
   double* partial = dot ? ctx->d_red : nullptr;
   const void* t1n = h->jit_t1n;
-  void* args_u[] = {&states, &diag, &x, &xq, &gmax, &sbits, &y, &dim, &t0, &t1, &t1n, &c0c, &c1c, &partial};
+  void* args_u[] = {&states, &diag, &x, &xq, &gmax, &sbits, &y, &dim, &t0, &t1, &t1n, &c0c, &c1c, &partial, &skip};
   std::vector<long long> pbc(coef ? std::max(1, seg[6]) : 0, 0ll);  // the PBC parameter's bytes
   if (coef) std::copy(coef, coef + seg[6], pbc.begin());
   void* args_pb[] = {&states, &diag, &x, &xq, &gmax, &sbits, &y, &dim, &t0, &t1, &t1n, &pbexp, &partial, pbc.data(),
-                     &coef_dev};
+                     &coef_dev, &skip};
   void** args = coef ? args_pb : args_u;
   CUresult r = g_drv.launch(mod->fn[bg][kd][ri], (unsigned)nblk, 1, 1, (unsigned)nt, 1, 1, (unsigned)smem,
                             (CUstream)ctx->stream, args, nullptr);

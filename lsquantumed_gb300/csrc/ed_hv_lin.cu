@@ -342,9 +342,10 @@ __global__ void __launch_bounds__(NT, MINB) k_hv_lin(const uint32_t* __restrict_
                                                 int* __restrict__ gmax_p, int sbits, double2* __restrict__ y,
                                                 int64_t dim, const uint16_t* __restrict__ t0,
                                                 const uint32_t* __restrict__ t1, const LinSegs sg, double c0c,
-                                                double c1c, double* __restrict__ partial, int rio_flag) {
+                                                double c1c, double* __restrict__ partial, int rio_flag,
+                                                const int* __restrict__ skip) {
   extern __shared__ uint16_t t0s[];
-  if (gmax_p[ED_HV_SKIP]) return;
+  if (skip && *skip) return;
   const bool rio = rio_flag != 0;
   const int n0 = 1 << sg.w0;
   for (int i = threadIdx.x; i < n0; i += blockDim.x) t0s[i] = t0[i];
@@ -392,7 +393,7 @@ bool ed_lin_supported(const ed_ham* h) {
 // Launch variants (same results: the integer sums are exact, so the unroll
 // depth and register budget change only the speed).
 typedef void (*LinKernel)(const uint32_t*, const double*, const double2*, const longlong2*, int*, int, double2*,
-                          int64_t, const uint16_t*, const uint32_t*, const LinSegs, double, double, double*, int);
+                          int64_t, const uint16_t*, const uint32_t*, const LinSegs, double, double, double*, int, const int*);
 struct LinVariant {
   LinKernel plain, dot;
   const char* name;
@@ -415,14 +416,15 @@ static const int kNumAllVariants = kNumLinVariants + 5;
 static const char* const kJitNames[5] = {"jit", "jit-b4", "jit-b3", "jit-w3", "jit-w4"};
 static uint64_t lin_signature(const ed_ham* h);
 
-static int lin_launch(ed_ham* h, int v, const void* x, void* y, bool dot, int sbits, int* nblk_out, bool rio) {
+static int lin_launch(ed_ham* h, int v, const void* x, void* y, bool dot, int sbits, int* nblk_out, bool rio,
+                      const int* skip) {
   ed_ctx* ctx = h->ctx;
   const ed_basis* b = h->basis;
   const ed_lin* L = h->lin;
   if (L->per_bond && v < kJitVariant) v = kJitVariant + 1;  // no static per-bond form
   if (v >= kJitVariant)
     return ed_jit_launch(h, lin_signature(h), v - kJitVariant, x, y, dot, sbits, nblk_out, L->segs.word, L->segs.seg,
-                         L->segs.w0, rio, L->per_bond ? L->coef.data() : nullptr, L->d_coef, L->pbexp);
+                         L->segs.w0, rio, L->per_bond ? L->coef.data() : nullptr, L->d_coef, L->pbexp, skip);
   const size_t smem = sizeof(uint16_t) * ((size_t)1 << b->lin_w0);
   const bool small = b->dim < (int64_t)ctx->num_sms * 256;
   const int nt = small ? 64 : 256;
@@ -436,7 +438,7 @@ static int lin_launch(ed_ham* h, int v, const void* x, void* y, bool dot, int sb
   if (dot) ED_TRY(ed_ensure_reduce(ctx, (size_t)3 * nblk + 8));
   k<<<nblk, nt, smem, ctx->stream>>>(b->d_states, h->d_diag, (const double2*)x, h->d_xq, h->d_gmax, sbits,
                                       (double2*)y, b->dim, b->d_lin_t0, b->d_lin_t1, L->segs, h->bs.chalf[0],
-                                      h->bs.chalf[1], dot ? ctx->d_red : nullptr, rio ? 1 : 0);
+                                      h->bs.chalf[1], dot ? ctx->d_red : nullptr, rio ? 1 : 0, skip);
   ED_CHECK_LAUNCH(ctx);
   if (nblk_out) *nblk_out = nblk;
   return ED_OK;
@@ -463,7 +465,7 @@ static uint64_t lin_signature(const ed_ham* h) {
 // First H.v (and first fused H.v + dot) of a large operator: time each
 // variant (two launches after one warm-up, CUDA events on the context's
 // stream) and keep the fastest.  The timing synchronises the stream once.
-static int lin_autotune(ed_ham* h, const void* x, void* y, int sbits, bool dot, bool rio) {
+static int lin_autotune(ed_ham* h, const void* x, void* y, int sbits, bool dot, bool rio, const int* skip) {
   ed_lin* L = h->lin;
   ed_ctx* ctx = h->ctx;
   int& chosen = L->variant[2 * (dot ? 1 : 0) + (rio ? 1 : 0)];
@@ -486,13 +488,13 @@ static int lin_autotune(ed_ham* h, const void* x, void* y, int sbits, bool dot, 
   int rc = ED_OK;
   bool first = true;
   for (int v = L->per_bond ? kJitVariant : 0; v < kNumAllVariants && rc == ED_OK; ++v) {
-    rc = lin_launch(h, v, x, y, dot, sbits, nullptr, rio);
+    rc = lin_launch(h, v, x, y, dot, sbits, nullptr, rio, skip);
     if (v >= kJitVariant && rc == ED_ENOTSUP) {  // no run-time compiler here: keep the static choice
       rc = ED_OK;
       break;
     }
     if (rc == ED_OK && cudaEventRecord(e0, ctx->stream) != cudaSuccess) rc = ed_fail(ED_ECUDA, "event record");
-    for (int it = 0; it < 2 && rc == ED_OK; ++it) rc = lin_launch(h, v, x, y, dot, sbits, nullptr, rio);
+    for (int it = 0; it < 2 && rc == ED_OK; ++it) rc = lin_launch(h, v, x, y, dot, sbits, nullptr, rio, skip);
     if (rc == ED_OK && cudaEventRecord(e1, ctx->stream) != cudaSuccess) rc = ed_fail(ED_ECUDA, "event record");
     float ms = 0.0f;
     if (rc == ED_OK && (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess))
@@ -514,7 +516,7 @@ static int lin_autotune(ed_ham* h, const void* x, void* y, int sbits, bool dot, 
 
 // y = H x through the two-table kernel.  With dot set, the kernel also leaves
 // Re/Im x^H y and ||y||^2 after the flags (d_gmax + ED_HV_SUMS).
-int ed_launch_hv_lin(ed_ham* h, const void* x, void* y, bool dot, int* nblk_out, bool rio) {
+int ed_launch_hv_lin(ed_ham* h, const void* x, void* y, bool dot, int* nblk_out, bool rio, const int* skip) {
   ED_TRY(lin_prepare(h));
   int sbits = 0;
   if (rio && h->xq_src == x) {
@@ -527,8 +529,8 @@ int ed_launch_hv_lin(ed_ham* h, const void* x, void* y, bool dot, int* nblk_out,
     ED_TRY(ed_fx64_quantize(h, (const double2*)x, &sbits));
   }
   const int which = 2 * (dot ? 1 : 0) + (rio ? 1 : 0);
-  if (h->lin->variant[which] < 0) ED_TRY(lin_autotune(h, x, y, sbits, dot, rio));
-  return lin_launch(h, h->lin->variant[which], x, y, dot, sbits, nblk_out, rio);
+  if (h->lin->variant[which] < 0) ED_TRY(lin_autotune(h, x, y, sbits, dot, rio, skip));
+  return lin_launch(h, h->lin->variant[which], x, y, dot, sbits, nblk_out, rio, skip);
 }
 
 // Force a launch variant by name ("auto" re-enables the autotuner); for tests

@@ -196,8 +196,8 @@ struct ed_ham {
   longlong2* d_xq = nullptr;      // 62-bit mantissas, (re, im) per state
   uint16_t* d_xe = nullptr;       // biased exponent per 32-state block
   // H.v flags, ED_GMAX_BYTES: [0] largest exponent, [1] non-finite input, [2]
-  // imaginary parts, [3] skip (a queued H.v returns at once), [4] blocks-done
-  // counter; from byte 64 the fused dot's three sums
+  // imaginary parts, [4] blocks-done counter; from byte 64 the fused dot's
+  // three sums
   int* d_gmax = nullptr;
   // d_xq / d_gmax already hold the fixed-point copy of this real vector
   // (ed_scale_quantize_r); the next two-table H.v of it uses them once
@@ -208,7 +208,6 @@ struct ed_ham {
 };
 
 #define ED_GMAX_BYTES 128
-#define ED_HV_SKIP 3
 #define ED_HV_COUNT 4
 #define ED_HV_SUMS 16  // in ints
 
@@ -242,8 +241,9 @@ int ed_launch_hv_dot(ed_ham* h, const double2* x, double2* y, double2* dot, doub
 // Same for x, y complex (rio false) or real storage double[dim] (rio true).
 int ed_launch_hv_dot_any(ed_ham* h, const void* x, void* y, bool rio, double2* dot, double* y2);
 // Real storage, nothing waits: *sums points at x^T y, 0 and ||y||^2 on the
-// device (valid until the operator's next fused H.v).
-int ed_launch_hv_dot_dev(ed_ham* h, const double* x, double* y, const double** sums);
+// device (valid until the operator's next fused H.v).  skip: on the device; the
+// product and the sums are left out when *skip is set by then.
+int ed_launch_hv_dot_dev(ed_ham* h, const double* x, double* y, const int* skip, const double** sums);
 // y = H x with real storage (two-table kernel only).
 int ed_launch_hv_r(ed_ham* h, const double* x, double* y);
 // Fixed-point copy of x into h->d_xq: largest exponent, non-finite flag and
@@ -266,7 +266,7 @@ int ed_scale_quantize_r(ed_ham* h, const double* src, double* dst, double s, dou
 int ed_fx64_sbits(const ed_ham* h);
 bool ed_lin_supported(const ed_ham* h);
 // rio: x and y are real storage (double[dim]) instead of complex128.
-int ed_launch_hv_lin(ed_ham* h, const void* x, void* y, bool dot, int* nblk_out, bool rio);
+int ed_launch_hv_lin(ed_ham* h, const void* x, void* y, bool dot, int* nblk_out, bool rio, const int* skip = nullptr);
 // The two-table H.v compiled at run time for one operator's bond words
 // (ed_hv_jit.cu); ED_ENOTSUP where no run-time compiler is available.
 // budget 0, 1, 2: register budget for 2, 4 or 3 blocks of 256 per SM; 3, 4:
@@ -276,7 +276,8 @@ int ed_launch_hv_lin(ed_ham* h, const void* x, void* y, bool dot, int* nblk_out,
 // read by the checked path); the row sums are then scaled by 2^pbexp.
 int ed_jit_launch(ed_ham* h, uint64_t signature, int budget, const void* x, void* y, bool dot, int sbits,
                   int* nblk_out, const unsigned long long* words, const int* seg, int w0, bool rio,
-                  const long long* coef = nullptr, const long long* coef_dev = nullptr, int pbexp = 0);
+                  const long long* coef = nullptr, const long long* coef_dev = nullptr, int pbexp = 0,
+                  const int* skip = nullptr);
 // NVRTC and the driver entry points can be loaded (the run-time compiled
 // kernels can exist at all).
 bool ed_jit_available();

@@ -344,8 +344,7 @@ __global__ void __launch_bounds__(KR_THREADS, NV > 8 ? 3 : 4) k_kr_update(const 
     else if (n2 <= 1e-26 * y2) why = KR_INVARIANT;
     else if (emax < 0) why = KR_EXPONENT;
     if (why != KR_RUN) {
-      st->stop = why;
-      gmax[ED_HV_SKIP] = 1;  // the H.v kernels queued behind return
+      st->stop = why;  // the kernels queued behind, H.v among them, return
     } else {
       gmax[0] = emax;
       gmax[1] = 0;
@@ -456,7 +455,7 @@ int ed_kr_step(ed_ham* h, double* const* cols, int j, bool three_term, double* w
   ed_ctx* ctx = h->ctx;
   const int64_t n = h->basis->dim;
   const double* hv = nullptr;
-  ED_TRY(ed_launch_hv_dot_dev(h, cols[j], w, &hv));
+  ED_TRY(ed_launch_hv_dot_dev(h, cols[j], w, &st->stop, &hv));
   ED_TRY(kr_dots(ctx, cols, j + 1, w, n, cols[j], 0.0, hv, three_term ? cols[j - 1] : nullptr, 0.0,
                  three_term ? &st->beta[j - 1] : nullptr, st->c, &st->stop));
   const int nv = j + 1;
