@@ -70,7 +70,7 @@ __device__ __forceinline__ void fx128(double w, int S, unsigned long long& lo, u
 
 struct CorrHeader {
   double W;        // sum psi_r^2
-  double Wl;       // sum lam_r^2 (two vectors)
+  double B;        // sum |w_r| (two vectors; with one it is W)
   int imag;        // some imaginary part is not zero
   int emax;        // largest biased exponent of a real part
   int nonfinite;   // some part is not finite
@@ -78,10 +78,10 @@ struct CorrHeader {
   int err;         // a wait of k_corr_gram ran out
 };
 
-// One pass over psi (TWO: and lam): the real parts to pr (pl), their sums of
-// squares, psi's largest exponent and the flags.  Four rows in flight per
-// thread; bound by memory (24 bytes per row and vector).  The last block sums
-// the block partials in order.
+// One pass over psi (TWO: and lam): the real parts to pr (pl), the sum of
+// squares of psi (TWO: and sum |lam psi|), psi's largest exponent and the
+// flags.  Four rows in flight per thread; bound by memory (24 bytes per row and
+// vector).  The last block sums the block partials in order.
 template <bool TWO>
 __global__ void __launch_bounds__(256) k_corr_prep(const double2* __restrict__ psi, const double2* __restrict__ lam,
                                                    int64_t n, double* __restrict__ pr, double* __restrict__ pl,
@@ -93,6 +93,7 @@ __global__ void __launch_bounds__(256) k_corr_prep(const double2* __restrict__ p
   int im = 0, nf = 0, em = 0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t r0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r0 < n; r0 += 4 * stride) {
+    double xa[4];
 #pragma unroll
     for (int k = 0; k < NA; ++k) {
       const double2* src = k ? lam : psi;
@@ -107,7 +108,8 @@ __global__ void __launch_bounds__(256) k_corr_prep(const double2* __restrict__ p
         if (k == 0) em = max(em, e);
         nf |= e == 0x7FF;
         im |= v[u].y != 0.0;  // a NaN counts as not zero
-        acc[k] = fma(v[u].x, v[u].x, acc[k]);
+        if (k == 0) xa[u] = v[u].x;
+        acc[k] = fma(fabs(v[u].x), fabs(xa[u]), acc[k]);
       }
     }
   }
@@ -141,7 +143,7 @@ __global__ void __launch_bounds__(256) k_corr_prep(const double2* __restrict__ p
   ed_block_reduce<NA>(t, sh);
   if (threadIdx.x == 0) {
     hdr->W = t[0];
-    if (TWO) hdr->Wl = t[NA - 1];
+    hdr->B = t[NA - 1];
   }
 }
 
@@ -890,11 +892,13 @@ int ed_corr_real(const ed_basis* b, const double2* lam, const double2* psi, bool
   ED_CUDA(cudaMemcpyAsync(&hh, hdr, sizeof(hh), cudaMemcpyDeviceToHost, ctx->stream));
   ED_CUDA(cudaStreamSynchronize(ctx->stream));
   out.real = hh.imag == 0;
-  // sum_r |w_r| <= B < 2^e (two vectors: Cauchy-Schwarz): every w_r and every
-  // integer sum stays below 2^124 at the scale 2^(124 - e) (the rounding of B
-  // moves it by far less than the spare bits)
-  const double B = two ? std::sqrt(hh.W) * std::sqrt(hh.Wl) : hh.W;
+  // sum_r |w_r| = B < 2^e: every w_r and every integer sum stays below 2^124 at
+  // the scale 2^(124 - e) (the rounding of B moves it by far less than the
+  // spare bits).  Below 2^-900 products and scales run out of exponents: the
+  // general kernels answer.
+  const double B = hh.B;
   if (!out.real || hh.nonfinite || !std::isfinite(B)) return ED_ENOTSUP;
+  if ((want_zz || gram) && B < 0x1p-900) return ED_ENOTSUP;
   out.N = N;
   out.W = hh.W;
   int e = 0;
