@@ -218,8 +218,9 @@ int ed_eps_set_tolerances(ed_eps* e, double tol, int max_it);
 int ed_eps_set_seed(ed_eps* e, uint64_t seed);
 /* Arithmetic of the restart combination V Y (the Krylov-Schur restart;
  * BVMultInPlace in SLEPc) in a real-storage solve (a real start vector and
- * the two-table H.v).  ED_RESTART_FP64: FP64 FMA beside exact integer
- * products.  ED_RESTART_PAIR: float-pair products on the FP32 units (each
+ * the two-table H.v).  ED_RESTART_FP64: every entry within (ncv + 1)
+ * 2^-53 of sum |V_i Y_ic|, as a chain of FP64 FMAs (digits of 68-bit fixed
+ * point on the tensor cores, small values in FP64).  ED_RESTART_PAIR: float-pair products on the FP32 units (each
  * FP64 value split into hi + lo, error below 2^-45 of |v y| per product;
  * storage and sums stay FP64), below FP64 accuracy, so only on request.
  * ED_RESTART_EXACT: exact slices on the tensor cores for the restart

@@ -378,7 +378,7 @@ static int eps_solve_real(ed_eps* e, int* nconv_out, int m, int nev, double tol,
   ed_ctx* ctx = H->ctx;
   const int64_t n = H->basis->dim;
   // float pairs and exact slices only on request; the default keeps every
-  // product at FP64 or better (FP64 FMA beside exact integers)
+  // value as good as FP64's (ed_combine.cu)
   e->restart_mode = e->restart_arith == ED_RESTART_AUTO ? ED_RESTART_FP64 : e->restart_arith;
   if (e->restart_mode == ED_RESTART_EXACT && m > 32)
     return ed_fail(ED_ENOTSUP, "the exact tensor-core restart takes at most 32 basis vectors (ncv <= 32)");

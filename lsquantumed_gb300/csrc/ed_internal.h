@@ -331,7 +331,7 @@ int ed_multidot_r(ed_ctx* ctx, const double* const* cols, int nv, double* w, int
 int ed_update_r(ed_ctx* ctx, const double* const* cols, int nv, const double* h_host, double* w, int64_t n,
                 double* wnorm2_host, double* wmax_host = nullptr, int arith = ED_RESTART_FP64);
 int ed_scale_copy_r(ed_ctx* ctx, const double* src, double* dst, double s, int64_t n);
-// arith: ED_RESTART_FP64 (FP64 FMA beside exact integer products),
+// arith: ED_RESTART_FP64 (FP64 accuracy, ed_combine.cu),
 // ED_RESTART_PAIR (float-pair products on the FP32 units, ed_linalg.cu) or
 // ED_RESTART_EXACT (exact slices on the tensor cores, ed_tc.cu; m <= 32).
 int ed_restart_combine_r(ed_ctx* ctx, const double* const* cols, int m, const double* Y, int ldY, int l,
