@@ -851,7 +851,8 @@ int ed_restart_combine_r(ed_ctx* ctx, const double* const* cols, int m, const do
                          double* const* out, int64_t n, int arith) {
   if (m > 127) return ed_fail(ED_ENOTSUP, "at most 127 basis vectors");
   if (arith == ED_RESTART_EXACT) return ed_restart_combine_tc(ctx, cols, m, Y, ldY, l, out, n);
-  if (arith == ED_RESTART_FP64) {
+  // fixed point has at most 32 columns, and the FP64 form serves the others
+  if (arith == ED_RESTART_FP64 || (arith == ED_RESTART_FIXED && m > 32)) {
     const int rc = ed_combine(ctx, cols, m, Y, ldY, l, out, n);
     if (rc != ED_ENOTSUP) return rc;
   }
