@@ -23,9 +23,10 @@
 // N rows, and N gathers of half-empty columns per t serve all N^2 / 2 pairs.
 // As FP64 FMAs it would be bound by the FP64 unit (7.4 ms at N=28), so it
 // runs on the tensor cores in exact 8-bit digits (k_corr_gram): 2.5 ms at
-// N=28 instead of 31.6 ms for 26 passes of 16 pairs before.  All S.S of the
-// N=28 state: 47.5 -> 2.9 ms; the energy gradient over 96 bonds at N=24:
-// 10.9 -> 0.30 ms.
+// N=28 (seven digits; now eight, 3% of the call more) instead of 31.6 ms for 26
+// passes of 16 pairs before.  Small flip sums are formed again in FP64, so a
+// list's length does not change their accuracy.  All S.S of the N=28 state:
+// 47.5 -> 3.04 ms; the energy gradient over 96 bonds at N=24: 10.9 -> 0.30 ms.
 #include "ed_internal.h"
 #include "ed_device.cuh"
 #include "ed_halves.cuh"
@@ -207,16 +208,16 @@ __global__ void __launch_bounds__(256) k_corr_cols(const double* __restrict__ pr
   atomicAdd(d + 3, (unsigned long long)((long long)hi >> 32));  // signed
 }
 
-// round(v 2^(54 - E)) for |v| < 2^E, E = emax - 1022, plus 128 in each of
-// the lower seven bytes: byte i is then digit i + 128 of the balanced base-256
-// representation, digits in [-128, 127] (|q| <= 2^54, so byte 7 is 0).
-constexpr unsigned long long GRAM_ZERO = 0x0080808080808080ull;
+// round(v 2^(62 - E)) for |v| < 2^E, E = emax - 1022, plus 128 in each byte:
+// byte i is then digit i + 128 of the balanced base-256 representation, digits
+// in [-128, 127] (|q| <= 2^62).
+constexpr unsigned long long GRAM_ZERO = 0x8080808080808080ull;
 __device__ __forceinline__ unsigned long long gram_entry(double v, int emax) {
   const long long b = __double_as_longlong(v);
   const int e = (int)((b >> 52) & 0x7FF);
   if (e == 0) return GRAM_ZERO;
   const unsigned long long mant = (unsigned long long)(b & 0xFFFFFFFFFFFFFll) | 0x10000000000000ull;
-  const int sh = e - emax + 1;  // <= 1
+  const int sh = e - emax + 9;  // <= 9
   unsigned long long q;
   if (sh >= 0) q = mant << sh;
   else if (sh > -60) q = (mant + (1ull << (-sh - 1))) >> (-sh);
@@ -331,15 +332,21 @@ __global__ void __launch_bounds__(256) k_corr_moments(const unsigned long long* 
 }
 
 // ---------------------------------------------------------------------------
-// Gram matrix F = Phi Phi^T on the tensor cores.  phi_i(t) in 55-bit fixed
-// point against the largest entry of the state (below FP64's rounding of the
-// sums), as seven balanced 8-bit digits, which FP16 holds exactly.  One
-// tcgen05.mma has M = 128 rows (digits 0..3 x 32 sites), N = 224 columns
-// (digits 0..6 x 32 sites) and K = 16 states; the digits are symmetric in
-// the two factors, so every product of digits i + j <= 6 (and more) is among
-// them or the transpose of one.  A digit product sum stays an exact integer
-// in the FP32 accumulator over GRAM_GROUP stages (1024 states x 128^2 =
-// 2^24), then four epilogue warps add it to 64-bit integers in shared memory.
+// Gram matrix F = Phi Phi^T on the tensor cores.  phi_i(t) in 63-bit fixed
+// point against the largest entry of the state, as eight balanced 8-bit digits,
+// which FP16 holds exactly.  One tcgen05.mma has M = 128 rows (digits 0..3 x 32
+// sites), N = 256 columns (digits 0..7 x 32 sites) and K = 16 states; the digits
+// are symmetric in the two factors, so every product of digits i + j <= 7 (and
+// more) is among them or the transpose of one.  A digit product sum stays an
+// exact integer in the FP32 accumulator over GRAM_GROUP stages (1024 states x
+// 128^2 = 2^24), then four epilogue warps add it to 64-bit integers in shared
+// memory.
+//
+// The rounded entries leave a root mean square error of at most 2^-62 / sqrt(12)
+// of 2^E times the norm: that of the last rounding of F for |F| >= 2^-9 2^E norm.
+// Smaller flip sums (sharply peaked states) are formed again in FP64
+// (ed_corr_real).  With 55 bits a flip sum of 6e-8 of a Neel-like state was off
+// by 1e-13 of itself.
 //
 // A stage is 128 states t = (c1, 128 consecutive low halves of one popcount).
 // The 16 producer warps take two sites each: a lane reads the entries of its
@@ -350,12 +357,13 @@ __global__ void __launch_bounds__(256) k_corr_moments(const unsigned long long* 
 // in registers while the stages run over the high halves.  The loads of the
 // next stage are issued before the current one is converted.
 // ---------------------------------------------------------------------------
-constexpr int GRAM_DIG = 7;
+constexpr int GRAM_DIG = 8;
+constexpr int GRAM_AGAIN = 9;                                  // a flip sum below 2^-9 2^E norm: again in FP64
 constexpr int GRAM_STATES = 128;
-constexpr int GRAM_ROWS = GRAM_DIG * CR_SITES;                 // 224
+constexpr int GRAM_ROWS = GRAM_DIG * CR_SITES;                 // 256
 constexpr int GRAM_N = GRAM_ROWS;
 constexpr int GRAM_LBO = GRAM_ROWS * 16 + 16;                  // + 16: the 16-byte rows of 8 lanes miss each other's banks
-constexpr int GRAM_STAGE = (GRAM_STATES / 8) * GRAM_LBO;       // 57600 bytes
+constexpr int GRAM_STAGE = (GRAM_STATES / 8) * GRAM_LBO;       // 65792 bytes
 constexpr int GRAM_GROUP = 8;                                  // stages per accumulation: 2^24 bound
 constexpr int GRAM_PROD = 16, GRAM_THREADS = (GRAM_PROD + 5) * 32;
 constexpr int GRAM_ACC = 128 * CR_SITES * 2;                   // 64-bit sums per CTA
@@ -570,7 +578,7 @@ __global__ void __launch_bounds__(GRAM_THREADS, 1) k_corr_gram(const unsigned lo
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
             const long long x = (long long)__float2int_rz(__uint_as_float(d[c]));
-            if (j < 4) H[c] = H[c] * 256 + x;
+            if (j < GRAM_DIG / 2) H[c] = H[c] * 256 + x;
             else L[c] = L[c] * 256 + x;
           }
         }
@@ -629,8 +637,8 @@ __global__ void __launch_bounds__(GRAM_THREADS, 1) k_corr_gram(const unsigned lo
 }
 
 // Sums over the CTAs and the four digits i, as 128-bit integers in units of
-// 2^24 q-units: out[b][a] = digit pairs (i, j <= 3), out[32 * 32 + b][a] =
-// (i, j = 4..6).  Block = site b, thread = TMEM lane (i, a).
+// 2^32 q-units: out[b][a] = digit pairs (i, j <= 3), out[32 * 32 + b][a] =
+// (i, j = 4..7).  Block = site b, thread = TMEM lane (i, a).
 __global__ void __launch_bounds__(256) k_corr_gram_sum(const long long* __restrict__ part, int ncta,
                                                        ulonglong2* __restrict__ out) {
   const int b = blockIdx.x, half = threadIdx.x >> 7, ln = threadIdx.x & 127, i = ln >> 5;
@@ -640,7 +648,7 @@ __global__ void __launch_bounds__(256) k_corr_gram_sum(const long long* __restri
     const long long x = p[(size_t)c * GRAM_ACC];
     add128(lo, hi, (unsigned long long)x, (unsigned long long)(x >> 63));
   }
-  const int sh = (half ? 24 : 48) - 8 * i;  // 0 .. 48
+  const int sh = (half ? 24 : 56) - 8 * i;  // 0 .. 56
   if (sh) {
     hi = (hi << sh) | (lo >> (64 - sh));
     lo <<= sh;
@@ -844,7 +852,10 @@ int ed_corr_real(const ed_basis* b, const double2* lam, const double2* psi, bool
   // every longer list.  Two vectors take direct passes.
   const bool gram = !two && (int64_t)flips.size() > ED_CORR_FEW;
   const bool few = !gram && !flips.empty();
-  const int64_t npass = few ? ((int64_t)flips.size() + ED_CORR_FEW - 1) / ED_CORR_FEW : 0;
+  // passes of the direct kernel per launch; behind the Gram kernel, for the
+  // pairs it leaves (GRAM_AGAIN)
+  int64_t npass = ((int64_t)flips.size() + ED_CORR_FEW - 1) / ED_CORR_FEW;
+  if (gram) npass = std::min<int64_t>(npass, 32);
   if (npass > 65535) return ED_ENOTSUP;  // grid.y
   const int nprep = (int)std::max<int64_t>(1, std::min<int64_t>((dim + 1023) / 1024, (int64_t)ctx->num_sms * 8));
   const int nflip = (int)std::max<int64_t>(1, std::min<int64_t>((dim + 255) / 256, (int64_t)ctx->num_sms * 4));
@@ -911,14 +922,16 @@ int ed_corr_real(const ed_basis* b, const double2* lam, const double2* psi, bool
                                                          seg, (unsigned long long*)(base + o_W0));
     ED_CHECK_LAUNCH(ctx);
   }
-  if (few) {
-    std::vector<FlipMasks> fm((size_t)npass);
+  // flip sums of flips[list[0 .. count - 1]] to o_f, count <= npass ED_CORR_FEW
+  auto direct = [&](const size_t* list, size_t count) -> int {
+    const size_t np_ = (count + ED_CORR_FEW - 1) / ED_CORR_FEW;
+    std::vector<FlipMasks> fm(np_);
     memset(fm.data(), 0, sizeof(FlipMasks) * fm.size());
     const uint32_t low = (1u << w0) - 1u;
-    for (size_t t = 0; t < flips.size(); ++t) {
+    for (size_t t = 0; t < count; ++t) {
       FlipMasks& pm = fm[t / ED_CORR_FEW];
       const int g = pm.n++;
-      const int i = pairs[2 * flips[t]], j = pairs[2 * flips[t] + 1];
+      const int i = pairs[2 * flips[list[t]]], j = pairs[2 * flips[list[t]] + 1];
       pm.m[g] = (1u << i) | (1u << j);
       pm.bi[g] = 1u << i;
       pm.ml[g] = pm.m[g] & low;
@@ -928,14 +941,17 @@ int ed_corr_real(const ed_basis* b, const double2* lam, const double2* psi, bool
                             ctx->stream));
     const size_t smem = sizeof(uint16_t) * ((size_t)1 << w0);
     auto kern = two ? k_expect_flip_r<true> : k_expect_flip_r<false>;
-    kern<<<dim3(nflip, (unsigned)npass), 256, smem, ctx->stream>>>(b->d_states, pr, pl, dim, b->d_lin_t0, b->d_lin_t1,
-                                                                   w0, (const FlipMasks*)(base + o_fm),
-                                                                   (double*)(base + o_fp), nflip);
+    kern<<<dim3(nflip, (unsigned)np_), 256, smem, ctx->stream>>>(b->d_states, pr, pl, dim, b->d_lin_t0, b->d_lin_t1,
+                                                                 w0, (const FlipMasks*)(base + o_fm),
+                                                                 (double*)(base + o_fp), nflip);
     ED_CHECK_LAUNCH(ctx);
-    k_flip_sum<<<(unsigned)flips.size(), 256, 0, ctx->stream>>>((const double*)(base + o_fp), nflip,
-                                                               (double*)(base + o_f));
+    k_flip_sum<<<(unsigned)count, 256, 0, ctx->stream>>>((const double*)(base + o_fp), nflip, (double*)(base + o_f));
     ED_CHECK_LAUNCH(ctx);
-  }
+    return ED_OK;
+  };
+  std::vector<size_t> list(flips.size());
+  for (size_t t = 0; t < list.size(); ++t) list[t] = t;
+  if (few) ED_TRY(direct(list.data(), list.size()));
   if (want_zz || gram) {
     const int gr = std::max(1, std::min((1 << w1) / 4, ctx->num_sms * 16));
     auto kern = gram ? k_corr_rows<true, false> : two ? k_corr_rows<false, true> : k_corr_rows<false, false>;
@@ -976,18 +992,37 @@ int ed_corr_real(const ed_basis* b, const double2* lam, const double2* psi, bool
   }
   out.F.assign(np, 0.0);
   out.Fl.assign(np, 0.0);
+  list.clear();
+  const double least = gram ? std::ldexp(std::sqrt(out.W), hh.emax - 1022 - GRAM_AGAIN) : 0.0;
   for (size_t t = 0; t < flips.size(); ++t) {
     const int i = pairs[2 * flips[t]], j = pairs[2 * flips[t] + 1];
     if (few) {
       memcpy(&out.F[flips[t]], res.data() + o_f + sizeof(double) * t, sizeof(double));
     } else if (nstages > 0) {
-      // F 2^(2 (54 - E) - 24), E = emax - 1022
+      // F 2^(2 (62 - E) - 32), E = emax - 1022
       const u128 x = get(o_G + 16 * (size_t)(i * 32 + j)) + get(o_G + 16 * (size_t)(1024 + i * 32 + j)) +
                      get(o_G + 16 * (size_t)(1024 + j * 32 + i));
-      const int sh = 2 * (hh.emax - 1022) - 108 + 24;
+      const int sh = 2 * (hh.emax - 1022) - 124 + 32;
       double rest;
       out.F[flips[t]] = std::ldexp(i128_split(x, rest), sh);
       out.Fl[flips[t]] = std::ldexp(rest, sh);
+      if (std::fabs(out.F[flips[t]]) < least) list.push_back(t);
+    }
+  }
+  if (list.empty()) return ED_OK;
+  // small flip sums again in FP64; the digits took the real parts' place
+  k_corr_prep<false><<<nprep, 256, 0, ctx->stream>>>(psi, psi, dim, pr, pr, hdr, (double*)(base + o_part));
+  ED_CHECK_LAUNCH(ctx);
+  const size_t most = (size_t)npass * ED_CORR_FEW;
+  for (size_t t0 = 0; t0 < list.size(); t0 += most) {
+    const size_t cnt = std::min(most, list.size() - t0);
+    ED_TRY(direct(list.data() + t0, cnt));
+    std::vector<double> f(cnt);
+    ED_CUDA(cudaMemcpyAsync(f.data(), base + o_f, sizeof(double) * cnt, cudaMemcpyDeviceToHost, ctx->stream));
+    ED_CUDA(cudaStreamSynchronize(ctx->stream));
+    for (size_t t = 0; t < cnt; ++t) {
+      out.F[flips[list[t0 + t]]] = f[t];
+      out.Fl[flips[list[t0 + t]]] = 0.0;
     }
   }
   return ED_OK;
