@@ -349,6 +349,8 @@ struct BCols {
 #define BU_REG 16  // k_batch_update_norm keeps up to this many coefficients in registers
 // With vj: first w <- w - a_b vj - bet_b vjm1 (coef = [a][B], [bet][B]),
 // written back, in the same pass (the local Lanczos projection).
+// A thread adds its rows in two chains: three blocks' chains are a third longer
+// than four blocks', and with them the rounding.
 // One instance per column count NI (0: the norm alone): the loads of a row are
 // issued together, without a test per column.  More than BD_MAXV columns: the
 // first BD_MAXV here, the others by the caller's next launches (item0).
@@ -368,11 +370,22 @@ __global__ void __launch_bounds__(256, BD_PER_SM) k_batch_dots(const BCols V, in
   for (int b0 = 0; b0 < B; b0 += Bp) {
     const int b = b0 + lane_b;
     double acc[NI + 1];
+    if (b0) __syncthreads();  // sh free
 #pragma unroll
     for (int i = 0; i <= NI; ++i) acc[i] = 0.0;
+    bool two = false;  // the first chain's sums are in this thread's places of sh
     if (lane_r < S && b < B) {
       const double ca = vj ? coef[b] : 0.0, cb = vj ? coef[B + b] : 0.0;
+      const int64_t half = r0 + lane_r + ((r1 - r0 + S - 1) / S + 1) / 2 * S;
       for (int64_t r = r0 + lane_r; r < r1; r += S) {
+        if (r == half) {
+#pragma unroll
+          for (int i = 0; i <= NI; ++i) {
+            sh[i * 256 + threadIdx.x] = acc[i];
+            acc[i] = 0.0;
+          }
+          two = true;
+        }
         const size_t k = (size_t)r * B + b;
         double wv = w[k], p = 0.0, q = 0.0, v[NI + 1];
         if (vj) p = vj[k];
@@ -389,9 +402,8 @@ __global__ void __launch_bounds__(256, BD_PER_SM) k_batch_dots(const BCols V, in
         if (norm) acc[NI] = fma(wv, wv, acc[NI]);
       }
     }
-    __syncthreads();  // sh free
 #pragma unroll
-    for (int i = 0; i <= NI; ++i) sh[i * 256 + threadIdx.x] = acc[i];
+    for (int i = 0; i <= NI; ++i) sh[i * 256 + threadIdx.x] = two ? sh[i * 256 + threadIdx.x] + acc[i] : acc[i];
     __syncthreads();
     // the items over all threads: thread = (item group, column)
     if (b < B)
@@ -487,7 +499,7 @@ __global__ void __launch_bounds__(256, BD_PER_SM) k_batch_update_norm(const BCol
   const int64_t r0 = (int64_t)blockIdx.x * rows_per, r1 = min(dim, r0 + rows_per);
   for (int b0 = 0; b0 < B; b0 += Bp) {
     const int b = b0 + lane_b;
-    double nrm = 0.0;
+    double nrm = 0.0, nrm1 = 0.0;  // two chains, as in k_batch_dots
     unsigned int amax = 0u;  // high word of max |w[r, b]|
     if (lane_r < S && b < B) {
       if (REG) {
@@ -513,24 +525,26 @@ __global__ void __launch_bounds__(256, BD_PER_SM) k_batch_update_norm(const BCol
           amax = ed_absmax_hi(amax, w0);
           if (has1) {
             w[k1] = w1;
-            nrm = fma(w1, w1, nrm);
+            nrm1 = fma(w1, w1, nrm1);
             amax = ed_absmax_hi(amax, w1);
           }
         }
       } else {
+        const int64_t half = r0 + (r1 - r0) / 2;
         for (int64_t r = r0 + lane_r; r < r1; r += S) {
           const size_t k = (size_t)r * B + b;
           double wv = w[k];
 #pragma unroll 4
           for (int i = 0; i < nv; ++i) wv = fma(-V.p[i][k], h[(size_t)i * B + b], wv);
           w[k] = wv;
-          nrm = fma(wv, wv, nrm);
+          if (r < half) nrm = fma(wv, wv, nrm);
+          else nrm1 = fma(wv, wv, nrm1);
           amax = ed_absmax_hi(amax, wv);
         }
       }
     }
     __syncthreads();
-    sh[threadIdx.x] = nrm;
+    sh[threadIdx.x] = nrm + nrm1;
     shm[threadIdx.x] = ed_absmax_hi_value(amax);
     __syncthreads();
     if (lane_r == 0 && b < B) {

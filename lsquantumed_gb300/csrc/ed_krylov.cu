@@ -116,6 +116,13 @@ __device__ __forceinline__ double block_sum256(double v, double* sh) {
   return a;
 }
 
+// A thread adds its rows in two chains, so that half as many threads with more
+// registers each do not mean longer chains: with one, and two blocks per SM, the
+// root mean square error of 16 dots of 10M rows was 1.32 times that of four
+// blocks per SM.  One more add per column and thread: 13 dots of 2.7M rows
+// 99 -> 100 us (four chains: 113).  Steps of one chain, of all:
+__device__ __forceinline__ int64_t kr_chain(int64_t steps) { return (steps + 1) / 2; }
+
 // Blocks per SM of k_kr_dots: registers for the loads of a row in flight.
 __host__ __device__ constexpr int kr_dots_per_sm(int ng) { return ng > 8 ? 2 : 3; }
 
@@ -144,9 +151,20 @@ __global__ void __launch_bounds__(KR_THREADS, kr_dots_per_sm(NG)) k_kr_dots(cons
   double acc[KR_GROUP];
 #pragma unroll
   for (int k = 0; k < KR_GROUP; ++k) acc[k] = 0.0;
+  __shared__ double sh[NG * (KR_THREADS + 1)];
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t half = r + kr_chain((n + U * stride - 1) / (U * stride)) * (U * stride);
+  bool two = false;  // the first chain's sums are in this thread's places of sh
   for (; r + (U - 1) * stride < n; r += U * stride) {
+    if (r == half) {
+#pragma unroll
+      for (int g = 0; g < NG; ++g) {
+        sh[g * (KR_THREADS + 1) + threadIdx.x] = acc[g];
+        acc[g] = 0.0;
+      }
+      two = true;
+    }
     double v[U][NG], wv[U], p[U], q[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -180,7 +198,10 @@ __global__ void __launch_bounds__(KR_THREADS, kr_dots_per_sm(NG)) k_kr_dots(cons
       for (int g = 0; g < NG; ++g) acc[g] = fma(kr_ld<DEP>(cp.p[g] + r), wv, acc[g]);
     }
   }
-  __shared__ double sh[NG * (KR_THREADS + 1)];
+  if (two) {
+#pragma unroll
+    for (int g = 0; g < NG; ++g) acc[g] += sh[g * (KR_THREADS + 1) + threadIdx.x];
+  }
   const int item = threadIdx.x >> 4, l = threadIdx.x & 15;
   const double s = block_sums16(acc, NG, sh);
   if (l == 0 && item < NG) partial[(size_t)item * gridDim.x + blockIdx.x] = s;
@@ -252,7 +273,14 @@ __global__ void __launch_bounds__(KR_THREADS, NV > 8 ? 3 : 4) k_kr_update(const 
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   if (NV > 0) {
     constexpr int U = NV <= 3 ? 4 : NV <= 8 ? 2 : 1;  // rows in flight per thread
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += U * stride) {
+    int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t half = r + kr_chain((n + U * stride - 1) / (U * stride)) * (U * stride);
+    double before = 0.0;  // the first chain
+    for (; r < n; r += U * stride) {
+      if (r == half) {
+        before = acc[0];
+        acc[0] = 0.0;
+      }
       double v[U][NV + 1], x[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -273,6 +301,7 @@ __global__ void __launch_bounds__(KR_THREADS, NV > 8 ? 3 : 4) k_kr_update(const 
         }
       }
     }
+    acc[0] += before;
   } else {
     for (int64_t r0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r0 < n; r0 += 2 * stride) {
       const int64_t r1 = r0 + stride;
