@@ -280,19 +280,23 @@ static int dsf_k(const ed_basis* b0, const ed_basis* b1, int op, const double2* 
 // Real vectors (eigenvectors of the real H) need only the products of the
 // real parts; any nonzero imaginary part raises *imag and the host runs the
 // complex form.
-// The signed sums cancel, so the large unsigned ones may not round: the warps'
-// sums are joined as pairs, a column's rows in chains of DZ_ROWS joined as
-// pairs, and the 256 columns of a block as exact integers.  With plain FP64
-// there the root mean square error against quad sums was up to 18% above
-// k_dsf's; with it, N=20, 12 real / complex states: 0.66-0.74e-16 / 0.92-1.0e-16
-// of the largest value against 0.92-0.97e-16 / 1.0-1.2e-16.  N=24, ten vectors:
-// 3.8 ms with k_dsf, 0.374 with plain sums, 0.394 so (the two reads of the
-// vectors, 0.95 GB, take 0.14).
+// The signed sums cancel, so the large unsigned ones may not round: a thread's
+// rows are added in chains of DZ_ROWS, and everything after is exact to 2^-70 of
+// the largest term or kept as a pair, up to the last rounding of c.  The root
+// mean square (largest) error against quad sums, relative to the largest c, N=20
+// and 24, ten real states of a few decades: 0.62-0.65e-16 (1.9-2.5e-16) against
+// 1.10-1.41e-16 (3.7-3.9e-16) with k_dsf; ten complex ones 0.82-0.88e-16
+// (3.5-3.6e-16) against 1.03-1.18e-16 (4.1-5.2e-16).  With the warps' and blocks'
+// sums rounded to FP64 it was 1.43-1.60e-16 (5.9-6.8e-16) and 1.30-1.48e-16
+// (7.3-7.5e-16).  N=24, ten real vectors, the call: 3.78 ms with k_dsf, 0.395
+// with those roundings, 0.480 so (the two reads of the vectors, 0.95 GB, take 0.14).
 // ---------------------------------------------------------------------------
 #define DZ_V 5
 #define DZ_SEG 32
 #define DZ_BITS 54
-#define DZ_ROWS 16  // rows of k_dsfz_low per plain FP64 chain
+#define DZ_MORE 20
+#define DZ_EMIN (DZ_BITS + DZ_MORE)
+#define DZ_ROWS 16  // rows per plain FP64 chain
 
 // (h, l) + x as an unevaluated pair (Knuth's TwoSum): the signed sums cancel,
 // so the few large partial sums here decide the rounding of the result
@@ -302,18 +306,54 @@ __device__ __forceinline__ void dsf_add(double& h, double& l, double x, double x
   h = t;
 }
 
-// partial[(((n * gridDim.x) + blk) * 32 + j) * 2]: re, im of site w0 + j
+// 2^(em - 1022 - DZ_BITS), the last place of fixed point against em, for em >=
+// DZ_EMIN; and the factor to units of 2^-DZ_MORE of it
+__device__ __forceinline__ double dsf_unit(int em) { return __longlong_as_double((long long)(em + 1 - DZ_BITS) << 52); }
+__device__ __forceinline__ double dsf_more(int em) {
+  return __longlong_as_double((long long)(2046 - (em + 1 - DZ_BITS - DZ_MORE)) << 52);
+}
+
+// The warp's sum of pairs, in every lane: as integers (54 + 20 bits against the
+// largest), 12 FP64 operations where five steps of dsf_add are 40.
+__device__ __forceinline__ void dsf_warp(double& h, double& l) {
+  const int em = (int)__reduce_max_sync(
+      0xffffffffu, (unsigned)(((unsigned long long)__double_as_longlong(h) >> 52) & 0x7FF));
+  if (em == 0x7FF || em < DZ_EMIN) {
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+      const double x = __shfl_xor_sync(0xffffffffu, h, s), xl = __shfl_xor_sync(0xffffffffu, l, s);
+      dsf_add(h, l, x, xl);
+    }
+    return;
+  }
+  const double u = dsf_unit(em);
+  long long q = ed_fx64_entry(h, em, DZ_BITS);
+  long long r = __double2ll_rn((fma(-(double)q, u, h) + l) * dsf_more(em));
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) {
+    q += __shfl_xor_sync(0xffffffffu, q, s);
+    r += __shfl_xor_sync(0xffffffffu, r, s);
+  }
+  const double hq = (double)q;
+  h = hq * u;
+  l = fma((double)r, 1.0 / (1 << DZ_MORE), (double)(q - (long long)hq)) * u;
+}
+
+// partial[(((n * gridDim.x) + blk) * 32 + j) * 4]: re, im of site w0 + j, as pairs
 template <bool REAL>
-__global__ void __launch_bounds__(128) k_dsfz_high(const double2* __restrict__ psi, const double2* __restrict__ vecs,
+__global__ void __launch_bounds__(128, REAL ? 5 : 3) k_dsfz_high(const double2* __restrict__ psi, const double2* __restrict__ vecs,
                                                    int64_t dim, int nev, int w0, int w1, int nup, const CorrGeom g,
                                                    const uint32_t* __restrict__ t1, double* __restrict__ partial,
                                                    int* __restrict__ imag) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int n0 = blockIdx.y * DZ_V, nv = min(DZ_V, nev - n0);
   const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
-  double hr[DZ_V], hi[DZ_V];
+  constexpr int C = REAL ? 1 : 2;  // parts: re, im
+  double hh[C][DZ_V], hl[C][DZ_V];  // the warp's signed sums of its runs
 #pragma unroll
-  for (int v = 0; v < DZ_V; ++v) hr[v] = hi[v] = 0.0;
+  for (int v = 0; v < DZ_V; ++v)
+#pragma unroll
+    for (int c = 0; c < C; ++c) hh[c][v] = hl[c][v] = 0.0;
   bool im = false;
   for (int c1 = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); c1 < (1 << w1); c1 += nwarps) {
     const int k = nup - __popc(c1);
@@ -321,58 +361,73 @@ __global__ void __launch_bounds__(128) k_dsfz_high(const double2* __restrict__ p
     const int n = g.nlow[k];
     const double2* p = psi + t1[c1];
     const double2* q = vecs + (size_t)n0 * dim + t1[c1];
-    double ar[DZ_V], ai[DZ_V];
+    double sh_[C][DZ_V], sl_[C][DZ_V];
 #pragma unroll
-    for (int v = 0; v < DZ_V; ++v) ar[v] = ai[v] = 0.0;
+    for (int v = 0; v < DZ_V; ++v)
+#pragma unroll
+      for (int c = 0; c < C; ++c) sh_[c][v] = sl_[c][v] = 0.0;
+    for (int o0 = lane; o0 < n; o0 += 32 * DZ_ROWS) {
+      double a[C][DZ_V];
+#pragma unroll
+      for (int v = 0; v < DZ_V; ++v)
+#pragma unroll
+        for (int c = 0; c < C; ++c) a[c][v] = 0.0;
+      const int o1 = min(n, o0 + 32 * DZ_ROWS);
 #pragma unroll 2
-    for (int o = lane; o < n; o += 32) {
-      const double2 x = p[o];
-      double2 y[DZ_V];
+      for (int o = o0; o < o1; o += 32) {
+        const double2 x = p[o];
+        double2 y[DZ_V];
 #pragma unroll
-      for (int v = 0; v < DZ_V; ++v) y[v] = v < nv ? q[(size_t)v * dim + o] : make_double2(0.0, 0.0);
-      if (REAL) im |= x.y != 0.0;
+        for (int v = 0; v < DZ_V; ++v) y[v] = v < nv ? q[(size_t)v * dim + o] : make_double2(0.0, 0.0);
+        if (REAL) im |= x.y != 0.0;
 #pragma unroll
-      for (int v = 0; v < DZ_V; ++v) {
-        if (REAL) {
-          im |= y[v].y != 0.0;
-          ar[v] = fma(y[v].x, x.x, ar[v]);
-        } else {  // conj(v) psi
-          ar[v] = fma(y[v].x, x.x, fma(y[v].y, x.y, ar[v]));
-          ai[v] = fma(y[v].x, x.y, fma(-y[v].y, x.x, ai[v]));
+        for (int v = 0; v < DZ_V; ++v) {
+          if (REAL) {
+            im |= y[v].y != 0.0;
+            a[0][v] = fma(y[v].x, x.x, a[0][v]);
+          } else {  // conj(v) psi
+            a[0][v] = fma(y[v].x, x.x, fma(y[v].y, x.y, a[0][v]));
+            a[C - 1][v] = fma(y[v].x, x.y, fma(-y[v].y, x.x, a[C - 1][v]));
+          }
         }
       }
+#pragma unroll
+      for (int v = 0; v < DZ_V; ++v)
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          if (o0 == lane) sh_[c][v] = a[c][v];  // the first chain
+          else dsf_add(sh_[c][v], sl_[c][v], a[c][v], 0.0);
+        }
     }
     const bool up = (c1 >> lane) & 1;
 #pragma unroll
-    for (int v = 0; v < DZ_V; ++v) {
+    for (int v = 0; v < DZ_V; ++v)
 #pragma unroll
-      for (int s = 16; s > 0; s >>= 1) {
-        ar[v] += __shfl_xor_sync(0xffffffffu, ar[v], s);
-        if (!REAL) ai[v] += __shfl_xor_sync(0xffffffffu, ai[v], s);
+      for (int c = 0; c < C; ++c) {
+        double h = sh_[c][v], l = sl_[c][v];
+        dsf_warp(h, l);
+        dsf_add(hh[c][v], hl[c][v], up ? h : -h, up ? l : -l);
       }
-      hr[v] += up ? ar[v] : -ar[v];
-      if (!REAL) hi[v] += up ? ai[v] : -ai[v];
-    }
   }
-  __shared__ double sh[2][DZ_V][4][32];
+  __shared__ double2 sh[C][DZ_V][4][32];
 #pragma unroll
-  for (int v = 0; v < DZ_V; ++v) {
-    sh[0][v][wid][lane] = hr[v];
-    sh[1][v][wid][lane] = hi[v];
-  }
+  for (int v = 0; v < DZ_V; ++v)
+#pragma unroll
+    for (int c = 0; c < C; ++c) sh[c][v][wid][lane] = make_double2(hh[c][v], hl[c][v]);
   if (REAL && __any_sync(0xffffffffu, im) && lane == 0) atomicOr(imag, 1);
   __syncthreads();
   for (int v = wid; v < nv; v += 4) {
-    double* d = partial + (((size_t)(n0 + v) * gridDim.x + blockIdx.x) * 32 + lane) * 2;
+    double2* d = (double2*)partial + (((size_t)(n0 + v) * gridDim.x + blockIdx.x) * 32 + lane) * 2;
     for (int c = 0; c < 2; ++c) {
-      double h = sh[c][v][0][lane], l = 0.0;
-      for (int w = 1; w < 4; ++w) dsf_add(h, l, sh[c][v][w][lane], 0.0);
-      d[c] = h + l;
+      double2 t = make_double2(0.0, 0.0);
+      if (c < C)
+        for (int w = 0; w < 4; ++w) dsf_add(t.x, t.y, sh[c][v][w][lane].x, sh[c][v][w][lane].y);
+      d[c] = t;
     }
   }
 }
 
-// partial[(((n * gridDim.x) + item) * 16 + i) * 2]: re, im of low site i
+// partial[(((n * gridDim.x) + item) * 16 + i) * 4]: re, im of low site i, as pairs
 template <bool REAL>
 __global__ void __launch_bounds__(256) k_dsfz_low(const double2* __restrict__ psi, const double2* __restrict__ vecs,
                                                   int64_t dim, int nev, const CorrGeom g,
@@ -387,32 +442,39 @@ __global__ void __launch_bounds__(256) k_dsfz_low(const double2* __restrict__ ps
   const int n0 = blockIdx.y * DZ_V, nv = min(DZ_V, nev - n0);
   __shared__ uint32_t base[DZ_SEG];
   __shared__ uint16_t c0[256];
-  __shared__ double sh[REAL ? 1 : 2][DZ_V][256];  // then the same as fixed point
+  constexpr int C = REAL ? 1 : 2;
+  __shared__ double sh[C][DZ_V][256];  // a column's sum, as fixed point
+  __shared__ int sr2[C][DZ_V][256];    // and what its rounding left, in 2^-DZ_MORE of its unit
   __shared__ int emax[REAL ? 1 : 2][DZ_V];
   if (threadIdx.x < (REAL ? 1 : 2) * DZ_V) (&emax[0][0])[threadIdx.x] = 0;
   if (threadIdx.x < nh) base[threadIdx.x] = t1[highs[g.high_off[k] + h0 + threadIdx.x]];
   const bool on = o < g.nlow[k];
   c0[threadIdx.x] = on ? lows[g.low_off[k] + o] : (uint16_t)0;
   __syncthreads();
-  double ar[DZ_V], ai[DZ_V];
+  double ar[DZ_V], ai[DZ_V], rr[DZ_V], ri[DZ_V];  // a column's sum and what its rounding left
 #pragma unroll
-  for (int v = 0; v < DZ_V; ++v) ar[v] = ai[v] = 0.0;
+  for (int v = 0; v < DZ_V; ++v) ar[v] = ai[v] = rr[v] = ri[v] = 0.0;
   if (on) {
     const double2* q = vecs + (size_t)n0 * dim;
     double sr[DZ_V], si[DZ_V], lr[DZ_V], li[DZ_V];  // chains of DZ_ROWS joined as pairs
 #pragma unroll
     for (int v = 0; v < DZ_V; ++v) sr[v] = si[v] = lr[v] = li[v] = 0.0;
-    auto join = [&]() {
+    auto join = [&](bool first) {
 #pragma unroll
       for (int v = 0; v < DZ_V; ++v) {
-        dsf_add(sr[v], lr[v], ar[v], 0.0);
-        if (!REAL) dsf_add(si[v], li[v], ai[v], 0.0);
+        if (first) {
+          sr[v] = ar[v];
+          si[v] = ai[v];
+        } else {
+          dsf_add(sr[v], lr[v], ar[v], 0.0);
+          if (!REAL) dsf_add(si[v], li[v], ai[v], 0.0);
+        }
         ar[v] = ai[v] = 0.0;
       }
     };
 #pragma unroll 2
     for (int h = 0; h < nh; ++h) {
-      if (h > 0 && h % DZ_ROWS == 0) join();
+      if (h > 0 && h % DZ_ROWS == 0) join(h == DZ_ROWS);
       const size_t r = (size_t)base[h] + o;
       const double2 x = psi[r];
       double2 y[DZ_V];
@@ -428,20 +490,24 @@ __global__ void __launch_bounds__(256) k_dsfz_low(const double2* __restrict__ ps
         }
       }
     }
-    join();
+    join(nh <= DZ_ROWS);
 #pragma unroll
     for (int v = 0; v < DZ_V; ++v) {
-      ar[v] = sr[v] + lr[v];
-      ai[v] = si[v] + li[v];
+      // |rest| <= half the last bit of the sum
+      ar[v] = sr[v];
+      dsf_add(ar[v], rr[v], lr[v], 0.0);
+      ai[v] = si[v];
+      dsf_add(ai[v], ri[v], li[v], 0.0);
     }
   }
   // The signed sums cancel: exact, as 54-bit integers against the block's
-  // largest column (256 of them stay below 2^62), rounded once.  FP64 adds are
-  // the scarcer unit too.  A column that is not finite: in FP64, as it was.
+  // largest column (256 of them stay below 2^62) and 20 bits more behind them.
+  // FP64 adds are the scarcer unit too.  A column that is not finite: in FP64, as
+  // it was.
 #pragma unroll
   for (int v = 0; v < DZ_V; ++v)
 #pragma unroll
-    for (int c = 0; c < (REAL ? 1 : 2); ++c) {
+    for (int c = 0; c < C; ++c) {
       const int e = (int)(((unsigned long long)__double_as_longlong(c ? ai[v] : ar[v]) >> 52) & 0x7FF);
       const int m = (int)__reduce_max_sync(0xffffffffu, (unsigned)e);
       if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(&emax[c][v], m);
@@ -450,35 +516,55 @@ __global__ void __launch_bounds__(256) k_dsfz_low(const double2* __restrict__ ps
 #pragma unroll
   for (int v = 0; v < DZ_V; ++v)
 #pragma unroll
-    for (int c = 0; c < (REAL ? 1 : 2); ++c) {
+    for (int c = 0; c < C; ++c) {
       const double x = c ? ai[v] : ar[v];
-      sh[c][v][threadIdx.x] =
-          emax[c][v] == 0x7FF ? x : __longlong_as_double(ed_fx64_entry(x, emax[c][v], DZ_BITS));
+      const int em = emax[c][v];
+      if (em == 0x7FF) {
+        sh[c][v][threadIdx.x] = x;
+      } else {
+        const long long q = ed_fx64_entry(x, em, DZ_BITS);
+        sh[c][v][threadIdx.x] = __longlong_as_double(q);
+        // |rest| is at most 2 units; its unit is a normal number for em >= DZ_EMIN
+        int r = 0;
+        if (em >= DZ_EMIN) {
+          const double rest = fma(-(double)q, dsf_unit(em), x) + (c ? ri[v] : rr[v]);
+          r = __double2int_rn(rest * dsf_more(em));
+        }
+        sr2[c][v][threadIdx.x] = r;
+      }
     }
   __syncthreads();
   // 16 threads per site: signed sums of the 256 columns
   const int i = threadIdx.x >> 4, l = threadIdx.x & 15;
   for (int v = 0; v < nv; ++v) {
-    double rm[2] = {0.0, 0.0};
+    double2 rm[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
 #pragma unroll
-    for (int p = 0; p < (REAL ? 1 : 2); ++p) {
+    for (int p = 0; p < C; ++p) {
       if (emax[p][v] == 0x7FF) {
-        for (int c = l; c < 256; c += 16) rm[p] += ((c0[c] >> i) & 1) ? sh[p][v][c] : -sh[p][v][c];
+        for (int c = l; c < 256; c += 16) rm[p].x += ((c0[c] >> i) & 1) ? sh[p][v][c] : -sh[p][v][c];
 #pragma unroll
-        for (int s = 8; s > 0; s >>= 1) rm[p] += __shfl_down_sync(0xffffffffu, rm[p], s, 16);
+        for (int s = 8; s > 0; s >>= 1) rm[p].x += __shfl_down_sync(0xffffffffu, rm[p].x, s, 16);
       } else {
         long long q = 0;
+        int r = 0;
         for (int c = l; c < 256; c += 16) {
           const long long x = __double_as_longlong(sh[p][v][c]);
-          q += ((c0[c] >> i) & 1) ? x : -x;
+          const bool up = (c0[c] >> i) & 1;
+          q += up ? x : -x;
+          r += up ? sr2[p][v][c] : -sr2[p][v][c];
         }
 #pragma unroll
-        for (int s = 8; s > 0; s >>= 1) q += __shfl_down_sync(0xffffffffu, q, s, 16);
-        rm[p] = ldexp((double)q, emax[p][v] - 1022 - DZ_BITS);
+        for (int s = 8; s > 0; s >>= 1) {
+          q += __shfl_down_sync(0xffffffffu, q, s, 16);
+          r += __shfl_down_sync(0xffffffffu, r, s, 16);
+        }
+        const double h = (double)q;
+        const double rest = (double)(q - (long long)h) + (double)r * (1.0 / (1 << DZ_MORE));
+        rm[p] = make_double2(ldexp(h, emax[p][v] - 1022 - DZ_BITS), ldexp(rest, emax[p][v] - 1022 - DZ_BITS));
       }
     }
     if (l == 0) {
-      double* d = partial + (((size_t)(n0 + v) * gridDim.x + blockIdx.x) * 16 + i) * 2;
+      double2* d = (double2*)partial + (((size_t)(n0 + v) * gridDim.x + blockIdx.x) * 16 + i) * 2;
       d[0] = rm[0];
       d[1] = rm[1];
     }
@@ -492,14 +578,14 @@ __global__ void __launch_bounds__(128) k_dsf_sum(const double* __restrict__ pl, 
                                                  double2* __restrict__ c) {
   const int i = blockIdx.x, n = blockIdx.y;
   const bool low = i < w0;
-  const double* p = low ? pl + ((size_t)n * nl * wl + i) * 2 : ph + ((size_t)n * nh * 32 + (i - w0)) * 2;
+  const double2* p = (const double2*)(low ? pl : ph) + ((size_t)n * (low ? nl * wl : nh * 32) + (low ? i : i - w0)) * 2;
   const int cnt = low ? nl : nh, ld = (low ? wl : 32) * 2;
   double h[2] = {0.0, 0.0}, l[2] = {0.0, 0.0};
 #pragma unroll 4
   for (int b = threadIdx.x; b < cnt; b += 128) {
-    const double2 v = *(const double2*)(p + (size_t)b * ld);
-    dsf_add(h[0], l[0], v.x, 0.0);
-    dsf_add(h[1], l[1], v.y, 0.0);
+    const double2 re = p[(size_t)b * ld], im = p[(size_t)b * ld + 1];
+    dsf_add(h[0], l[0], re.x, re.y);
+    dsf_add(h[1], l[1], im.x, im.y);
   }
   __shared__ double sh[4][4];
 #pragma unroll
@@ -541,7 +627,7 @@ __global__ void k_any_imag(const double2* __restrict__ a, int64_t na, const doub
 // of c1 in sector 1 at T0[c0 + site]; a high site's is the same offset of
 // the run of c1 + site, so consecutive lanes read consecutive entries.  One
 // pass over psi and v for all sites, one FMA per site that is down; grid.y
-// is the vector.  partial[(((n * gridDim.x) + blk) * 32 + site) * 2].
+// is the vector.  partial[(((n * gridDim.x) + blk) * 32 + site) * 4].
 __global__ void __launch_bounds__(128) k_dsfp_r(const double2* __restrict__ psi, const double2* __restrict__ vecs,
                                                 int64_t dim1, int w0, int w1, int nup, const CorrGeom g,
                                                 const uint16_t* __restrict__ lows, const uint16_t* __restrict__ t0,
@@ -590,9 +676,9 @@ __global__ void __launch_bounds__(128) k_dsfp_r(const double2* __restrict__ psi,
   }
   __syncthreads();
   if (threadIdx.x < 32) {
-    double* d = partial + (((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 32 + lane) * 2;
-    d[0] = (sh[0][lane] + sh[1][lane]) + (sh[2][lane] + sh[3][lane]);
-    d[1] = 0.0;
+    double2* d = (double2*)partial + (((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 32 + lane) * 2;
+    d[0] = make_double2((sh[0][lane] + sh[1][lane]) + (sh[2][lane] + sh[3][lane]), 0.0);
+    d[1] = make_double2(0.0, 0.0);
   }
 }
 
@@ -607,8 +693,8 @@ static int dsf_runs(const ed_basis* b0, const ed_basis* b1, int op, const double
   const CorrGeom g = corr_geom(b0, b0->nup, 256, [](int nh) { return (nh + DZ_SEG - 1) / DZ_SEG; });
   const int ni = g.prefix[CR_CLASSES];
   const size_t o_c = 256, o_h = o_c + ((sizeof(double2) * (size_t)N * nev + 255) & ~(size_t)255);
-  const size_t o_l = o_h + sizeof(double2) * 32 * (size_t)nb * nev;
-  ed_workspace ws(ctx, o_l + sizeof(double2) * 16 * (size_t)ni * nev);
+  const size_t o_l = o_h + 2 * sizeof(double2) * 32 * (size_t)nb * nev;
+  ed_workspace ws(ctx, o_l + 2 * sizeof(double2) * 16 * (size_t)ni * nev);
   if (!ws.ptr) return ED_ENOMEM;
   char* base = (char*)ws.ptr;
   int* imag = (int*)base;
@@ -633,7 +719,7 @@ static int dsf_runs(const ed_basis* b0, const ed_basis* b1, int op, const double
                                                         b0->d_lin_t0, b0->d_lin_t1, b1->d_lin_t1, ph);
     ED_CHECK_LAUNCH(ctx);
     // all sites in ph, low ones at 0 .., high ones at CR_MAXW0 ..
-    k_dsf_sum<<<dim3(N, nev), 128, 0, ctx->stream>>>(ph, nb, 32, ph + 2 * CR_MAXW0, nb, w0, 1.0, c);
+    k_dsf_sum<<<dim3(N, nev), 128, 0, ctx->stream>>>(ph, nb, 32, ph + 4 * CR_MAXW0, nb, w0, 1.0, c);
   }
   ED_CHECK_LAUNCH(ctx);
   std::vector<char> res(o_h);
