@@ -356,6 +356,7 @@ __global__ void __launch_bounds__(128, REAL ? 5 : 3) k_dsfz_high(const double2* 
     for (int c = 0; c < C; ++c) hh[c][v] = hl[c][v] = 0.0;
   bool im = false;
   for (int c1 = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); c1 < (1 << w1); c1 += nwarps) {
+    if (REAL && __any_sync(0xffffffffu, *(volatile int*)imag != 0)) break;  // the host asks for the complex form
     const int k = nup - __popc(c1);
     if (k < 0 || k > w0) continue;
     const int n = g.nlow[k];
@@ -399,6 +400,10 @@ __global__ void __launch_bounds__(128, REAL ? 5 : 3) k_dsfz_high(const double2* 
           else dsf_add(sh_[c][v], sl_[c][v], a[c][v], 0.0);
         }
     }
+    if (REAL && __any_sync(0xffffffffu, im)) {
+      if (lane == 0) atomicOr(imag, 1);
+      break;
+    }
     const bool up = (c1 >> lane) & 1;
 #pragma unroll
     for (int v = 0; v < DZ_V; ++v)
@@ -414,7 +419,6 @@ __global__ void __launch_bounds__(128, REAL ? 5 : 3) k_dsfz_high(const double2* 
   for (int v = 0; v < DZ_V; ++v)
 #pragma unroll
     for (int c = 0; c < C; ++c) sh[c][v][wid][lane] = make_double2(hh[c][v], hl[c][v]);
-  if (REAL && __any_sync(0xffffffffu, im) && lane == 0) atomicOr(imag, 1);
   __syncthreads();
   for (int v = wid; v < nv; v += 4) {
     double2* d = (double2*)partial + (((size_t)(n0 + v) * gridDim.x + blockIdx.x) * 32 + lane) * 2;
@@ -433,7 +437,9 @@ __global__ void __launch_bounds__(256) k_dsfz_low(const double2* __restrict__ ps
                                                   int64_t dim, int nev, const CorrGeom g,
                                                   const uint16_t* __restrict__ lows,
                                                   const uint32_t* __restrict__ highs,
-                                                  const uint32_t* __restrict__ t1, double* __restrict__ partial) {
+                                                  const uint32_t* __restrict__ t1, double* __restrict__ partial,
+                                                  const int* __restrict__ imag) {
+  if (REAL && *imag) return;  // k_dsfz_high met an imaginary part
   int k = 0;
   while (k < g.w0 && (int)blockIdx.x >= g.prefix[k + 1]) ++k;
   const int item = (int)blockIdx.x - g.prefix[k];
@@ -610,16 +616,25 @@ __global__ void __launch_bounds__(128) k_dsf_sum(const double* __restrict__ pl, 
   }
 }
 
-// *any = 1 if some entry has a nonzero imaginary part (two arrays)
+// *any = 1 if some entry has a nonzero imaginary part (two arrays); the first one
+// found ends the search
 __global__ void k_any_imag(const double2* __restrict__ a, int64_t na, const double2* __restrict__ b, int64_t nb,
                            int* __restrict__ any) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  bool f = false;
-#pragma unroll 4
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < na; i += stride) f |= a[i].y != 0.0;
-#pragma unroll 4
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += stride) f |= b[i].y != 0.0;
-  if (__any_sync(0xffffffffu, f) && (threadIdx.x & 31) == 0) atomicOr(any, 1);
+  for (int k = 0; k < 2; ++k) {
+    const double2* v = k ? b : a;
+    const int64_t n = k ? nb : na;
+    for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 - threadIdx.x < n; i0 += 8 * stride) {
+      if (__any_sync(0xffffffffu, *(volatile int*)any != 0)) return;
+      bool f = false;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) f |= i0 + u * stride < n && v[i0 + u * stride].y != 0.0;
+      if (__any_sync(0xffffffffu, f)) {
+        if ((threadIdx.x & 31) == 0) atomicOr(any, 1);
+        return;
+      }
+    }
+  }
 }
 
 // Sqp for real vectors: a warp takes the run of one c1 of sector 0; every site
@@ -632,7 +647,8 @@ __global__ void __launch_bounds__(128) k_dsfp_r(const double2* __restrict__ psi,
                                                 int64_t dim1, int w0, int w1, int nup, const CorrGeom g,
                                                 const uint16_t* __restrict__ lows, const uint16_t* __restrict__ t0,
                                                 const uint32_t* __restrict__ t1a, const uint32_t* __restrict__ t1b,
-                                                double* __restrict__ partial) {
+                                                double* __restrict__ partial, const int* __restrict__ imag) {
+  if (*imag) return;  // complex vectors: the general kernel answers
   extern __shared__ uint16_t t0s[];
   for (int i = threadIdx.x; i < (1 << w0); i += blockDim.x) t0s[i] = t0[i];
   __syncthreads();
@@ -706,7 +722,7 @@ static int dsf_runs(const ed_basis* b0, const ed_basis* b1, int op, const double
     k_dsfz_high<REAL><<<gh, 128, 0, ctx->stream>>>(psi, vecs, b0->dim, nev, w0, w1, b0->nup, g, b0->d_lin_t1, ph, imag);
     ED_CHECK_LAUNCH(ctx);
     k_dsfz_low<REAL><<<gl, 256, 0, ctx->stream>>>(psi, vecs, b0->dim, nev, g, b0->d_lin_lows, b0->d_lin_highs,
-                                                  b0->d_lin_t1, pl);
+                                                  b0->d_lin_t1, pl, imag);
     ED_CHECK_LAUNCH(ctx);
     k_dsf_sum<<<dim3(N, nev), 128, 0, ctx->stream>>>(pl, ni, 16, ph, nb, w0, 0.5, c);
   } else {
@@ -716,7 +732,7 @@ static int dsf_runs(const ed_basis* b0, const ed_basis* b1, int op, const double
     ED_CHECK_LAUNCH(ctx);
     const size_t smem = sizeof(uint16_t) * ((size_t)1 << w0);
     k_dsfp_r<<<dim3(nb, nev), 128, smem, ctx->stream>>>(psi, vecs, b1->dim, w0, w1, b0->nup, g, b0->d_lin_lows,
-                                                        b0->d_lin_t0, b0->d_lin_t1, b1->d_lin_t1, ph);
+                                                        b0->d_lin_t0, b0->d_lin_t1, b1->d_lin_t1, ph, imag);
     ED_CHECK_LAUNCH(ctx);
     // all sites in ph, low ones at 0 .., high ones at CR_MAXW0 ..
     k_dsf_sum<<<dim3(N, nev), 128, 0, ctx->stream>>>(ph, nb, 32, ph + 4 * CR_MAXW0, nb, w0, 1.0, c);
