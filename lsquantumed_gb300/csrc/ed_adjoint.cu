@@ -214,6 +214,17 @@ static int mixed_k(const ed_basis* b, const double2* lam, const double2* psi, co
   return ED_OK;
 }
 
+// Any vectors, FP64.
+static int mixed_general(const ed_basis* b, const double2* lam, const double2* psi, const int* kinds,
+                         const int32_t* ij, int64_t nt, double2* out) {
+  switch (b->rt.K) {
+    case 1: return mixed_k<1>(b, lam, psi, kinds, ij, nt, out);
+    case 2: return mixed_k<2>(b, lam, psi, kinds, ij, nt, out);
+    case 3: return mixed_k<3>(b, lam, psi, kinds, ij, nt, out);
+    default: return mixed_k<4>(b, lam, psi, kinds, ij, nt, out);
+  }
+}
+
 static int mixed(const ed_basis* b, const double2* lam, const double2* psi, const int* kinds, const int32_t* ij,
                  int64_t nt, double2* out) {
   {
@@ -248,12 +259,7 @@ static int mixed(const ed_basis* b, const double2* lam, const double2* psi, cons
     }
     if (rc != ED_ENOMEM && rc != ED_ENOTSUP) return rc;
   }
-  switch (b->rt.K) {
-    case 1: return mixed_k<1>(b, lam, psi, kinds, ij, nt, out);
-    case 2: return mixed_k<2>(b, lam, psi, kinds, ij, nt, out);
-    case 3: return mixed_k<3>(b, lam, psi, kinds, ij, nt, out);
-    default: return mixed_k<4>(b, lam, psi, kinds, ij, nt, out);
-  }
+  return mixed_general(b, lam, psi, kinds, ij, nt, out);
 }
 
 template <int K>
@@ -326,19 +332,20 @@ int ed_grad_energy(const ed_basis* b, const int32_t* pairs_host, int64_t nbonds,
     kinds.push_back(ED_TERM_ZZ); ij.push_back(pairs_host[2 * q]); ij.push_back(pairs_host[2 * q + 1]);
   }
   for (int i = 0; i < N; ++i) { kinds.push_back(ED_TERM_Z); ij.push_back(i); ij.push_back(i); }
-  std::vector<ed_cplx> out(kinds.size());
-  ED_TRY(ed_expect_mixed(b, kinds.data(), ij.data(), (int64_t)kinds.size(), psi_dev, psi_dev, out.data()));
+  std::vector<double2> out(kinds.size());
+  const double2* psi = (const double2*)psi_dev;
+  ED_TRY(mixed_general(b, psi, psi, kinds.data(), ij.data(), (int64_t)kinds.size(), out.data()));
   // <psi|psi> normalisation
   double2 nrm;
   double n2 = 0.0;
   ED_TRY(ed_multidot(b->ctx, nullptr, 0, (const double2*)psi_dev, b->dim, &nrm, &n2));
   const double inv = 1.0 / n2;
   for (int64_t q = 0; q < nbonds; ++q) {
-    if (dJ_host) dJ_host[q] = out[2 * q].re * inv;
-    if (dD_host) dD_host[q] = out[2 * q + 1].re * inv;
+    if (dJ_host) dJ_host[q] = out[2 * q].x * inv;
+    if (dD_host) dD_host[q] = out[2 * q + 1].x * inv;
   }
   for (int i = 0; i < N; ++i)
-    if (dh_host) dh_host[i] = out[2 * nbonds + i].re * inv;
+    if (dh_host) dh_host[i] = out[2 * nbonds + i].x * inv;
   return ED_OK;
 }
 
