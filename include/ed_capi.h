@@ -57,6 +57,11 @@ int ed_version(void);
  * creates its own non-blocking stream) or a cudaStream_t owned by the caller. */
 int ed_ctx_create(int device, void* stream, ed_ctx** out);
 int ed_ctx_destroy(ed_ctx* ctx);
+/* The measurements keep up to 512 MB of device scratch in the context from call
+ * to call.  An allocation of this library that finds the device full takes it
+ * back by itself; this call gives it back at once, for other users of the
+ * device.  No counterpart in the reference. */
+int ed_ctx_trim(ed_ctx* ctx);
 int ed_ctx_synchronize(ed_ctx* ctx);
 /* Number of kernels this context launched so far (for launch accounting). */
 int ed_ctx_kernel_count(const ed_ctx* ctx, int64_t* count);
@@ -335,9 +340,9 @@ int ed_batch_set_restart_arithmetic(ed_batch* bt, int mode);
  * the basis (PETSc VecDot convention: sum_s psi_s * conj((O psi)_s)).  For a
  * real psi (every imaginary part zero, as the solver's eigenvectors), the
  * S^z S^z part and the one-site sums are exact integer sums of the FP64
- * weights psi_s^2 rounded once, and the call holds a temporary copy of the
- * real parts (8 * dim bytes) on the device; without room for it, or for a
- * non-finite psi, the general FP64 kernel runs instead. */
+ * weights psi_s^2 rounded once, and the call holds a copy of the real parts (8 *
+ * dim bytes) in the context's scratch (ed_ctx_trim); without room for it, or for
+ * a non-finite psi, the general FP64 kernel runs instead. */
 int ed_expect_pairs(const ed_basis* b, int op, const ed_cplx* psi_dev, const int32_t* pairs_host,
                     int64_t npairs, ed_cplx* out_host);
 /* All N*N <S_i.S_j> (op = ED_OP_SISJ) into out_host[i*N + j]. */

@@ -44,6 +44,7 @@ SIGNATURES = {
     'ed_version': [],
     'ed_ctx_create': [i32, vp, P(vp)],
     'ed_ctx_destroy': [vp],
+    'ed_ctx_trim': [vp],
     'ed_ctx_synchronize': [vp],
     'ed_ctx_kernel_count': [vp, P(i64)],
     'ed_ctx_profile': [vp, i32],

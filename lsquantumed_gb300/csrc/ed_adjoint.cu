@@ -371,7 +371,7 @@ int ed_minres(ed_ham* h, double shift, const ed_cplx* rhs_dev, const ed_cplx* q_
   if (tol <= 0) tol = 1e-12;
   if (max_it <= 0) max_it = (int)std::min<int64_t>(10 * n, 100000);
   double2* buf = nullptr;
-  if (cudaMalloc(&buf, sizeof(double2) * (size_t)n * 7) != cudaSuccess) {
+  if (ed_malloc(&buf, sizeof(double2) * (size_t)n * 7) != cudaSuccess) {
     cudaGetLastError();
     return ed_fail(ED_ENOMEM, "MINRES workspace does not fit in device memory");
   }

@@ -825,7 +825,7 @@ static int batch_reduce_buf(ed_batch* bt, size_t doubles) {
   if (bt->h_red) cudaFreeHost(bt->h_red);
   bt->d_red = nullptr;
   bt->h_red = nullptr;
-  ED_CUDA(cudaMalloc(&bt->d_red, doubles * sizeof(double)));
+  ED_CUDA(ed_malloc(&bt->d_red, doubles * sizeof(double)));
   ED_CUDA(cudaMallocHost(&bt->h_red, doubles * sizeof(double)));
   bt->red_cap = doubles;
   return ED_OK;
@@ -1046,9 +1046,9 @@ int ed_batch_create(ed_ham* h, int B, const double* hi_host, ed_batch** out) {
   bt->dim = h->basis->dim;
   const size_t n = (size_t)bt->dim * B;
   double* dhi = nullptr;
-  if (cudaMalloc(&bt->d_diag, sizeof(double) * n) != cudaSuccess || cudaMalloc(&bt->d_xq, sizeof(longlong2) * n) != cudaSuccess ||
-      cudaMalloc(&bt->d_gmax, sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&dhi, sizeof(double) * (size_t)B * N) != cudaSuccess) {
+  if (ed_malloc(&bt->d_diag, sizeof(double) * n) != cudaSuccess || ed_malloc(&bt->d_xq, sizeof(longlong2) * n) != cudaSuccess ||
+      ed_malloc(&bt->d_gmax, sizeof(int)) != cudaSuccess ||
+      ed_malloc(&dhi, sizeof(double) * (size_t)B * N) != cudaSuccess) {
     cudaGetLastError();
     if (dhi) cudaFree(dhi);
     ed_batch_destroy(bt);
@@ -1170,19 +1170,19 @@ static int batch_solve_impl(ed_batch* bt, int nev, int ncv, double tol, int max_
   double* d_coef = nullptr;  // [64][B] double2 coefficients / scale factors
   int* d_idx = nullptr;      // [2][B] slot / realisation index lists
   double* dY = nullptr;
-  if (cudaMalloc(&pool, sizeof(double) * colB * pool_cols) != cudaSuccess ||
-      cudaMalloc(&w, sizeof(double) * colB) != cudaSuccess || cudaMalloc(&dg[0], sizeof(double) * colB) != cudaSuccess ||
-      cudaMalloc(&dg[1], sizeof(double) * colB) != cudaSuccess ||
-      cudaMalloc(&d_coef, sizeof(double2) * 64 * (size_t)B) != cudaSuccess ||
-      cudaMalloc(&d_idx, sizeof(int) * 2 * (size_t)B) != cudaSuccess ||
-      cudaMalloc(&dY, sizeof(double) * (size_t)B * m * l_keep) != cudaSuccess) {
+  if (ed_malloc(&pool, sizeof(double) * colB * pool_cols) != cudaSuccess ||
+      ed_malloc(&w, sizeof(double) * colB) != cudaSuccess || ed_malloc(&dg[0], sizeof(double) * colB) != cudaSuccess ||
+      ed_malloc(&dg[1], sizeof(double) * colB) != cudaSuccess ||
+      ed_malloc(&d_coef, sizeof(double2) * 64 * (size_t)B) != cudaSuccess ||
+      ed_malloc(&d_idx, sizeof(int) * 2 * (size_t)B) != cudaSuccess ||
+      ed_malloc(&dY, sizeof(double) * (size_t)B * m * l_keep) != cudaSuccess) {
     cudaGetLastError();
     cudaFree(pool); cudaFree(w); cudaFree(dg[0]); cudaFree(dg[1]); cudaFree(d_coef); cudaFree(d_idx); cudaFree(dY);
     return ed_fail(ED_ENOMEM, "batched Krylov basis does not fit in device memory");
   }
   if (bt->d_vecs) cudaFree(bt->d_vecs);
   bt->d_vecs = nullptr;
-  if (cudaMalloc(&bt->d_vecs, sizeof(double) * colB * nev) != cudaSuccess) {
+  if (ed_malloc(&bt->d_vecs, sizeof(double) * colB * nev) != cudaSuccess) {
     cudaGetLastError();
     cudaFree(pool); cudaFree(w); cudaFree(dg[0]); cudaFree(dg[1]); cudaFree(d_coef); cudaFree(d_idx); cudaFree(dY);
     return ed_fail(ED_ENOMEM, "batched eigenvectors do not fit in device memory");
@@ -1192,8 +1192,8 @@ static int batch_solve_impl(ed_batch* bt, int nev, int ncv, double tol, int max_
   double* st_buf = nullptr;
   int* st_int = nullptr;
   const size_t m1 = (size_t)m + 1;
-  if (cudaMalloc(&st_buf, sizeof(double) * (2 * m1 + 2) * (size_t)B) != cudaSuccess ||
-      cudaMalloc(&st_int, sizeof(int) * 8) != cudaSuccess) {
+  if (ed_malloc(&st_buf, sizeof(double) * (2 * m1 + 2) * (size_t)B) != cudaSuccess ||
+      ed_malloc(&st_int, sizeof(int) * 8) != cudaSuccess) {
     cudaGetLastError();
     cudaFree(st_buf);
     cudaFree(pool); cudaFree(w); cudaFree(dg[0]); cudaFree(dg[1]); cudaFree(d_coef); cudaFree(d_idx); cudaFree(dY);

@@ -21,35 +21,39 @@ int ed_cuda_fail(cudaError_t e, const char* what, const char* file, int line) {
   return e == cudaErrorMemoryAllocation ? ED_ENOMEM : ED_ECUDA;
 }
 
-ed_workspace::ed_workspace(ed_ctx* c, size_t bytes) : ctx(c) {
-  if (bytes <= ED_WS_KEEP && !c->ws_busy) {
-    if (bytes > c->ws_cap) {
-      if (c->ws) cudaFree(c->ws);
-      c->ws = nullptr;
-      c->ws_cap = 0;
-      if (cudaMalloc(&c->ws, bytes) != cudaSuccess) {
-        cudaGetLastError();
-        c->ws = nullptr;
-        return;
-      }
-      c->ws_cap = bytes;
+namespace {
+struct CudaMem {
+  static int get(void** p, size_t bytes) {
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) {
+      cudaGetLastError();  // an allocation that does not fit is not a failure of the device
+      *p = nullptr;
     }
-    c->ws_busy = true;
-    ptr = c->ws;
-    return;
+    return (int)e;
   }
-  if (cudaMalloc(&ptr, bytes) != cudaSuccess) {
-    cudaGetLastError();
-    ptr = nullptr;
-    return;
-  }
-  own = true;
+  static bool full(int e) { return e == (int)cudaErrorMemoryAllocation; }
+  // waits for the device: work queued on the slot's stream is done with it
+  static void put(void* p) { cudaFree(p); }
+};
+// never destroyed: contexts may outlive the end of main
+ed_scratch_pool<CudaMem>& pool() {
+  static auto* p = new ed_scratch_pool<CudaMem>();
+  return *p;
+}
+}  // namespace
+
+cudaError_t ed_malloc_bytes(void** p, size_t bytes) {
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  return (cudaError_t)pool().alloc(p, bytes, device);
 }
 
-ed_workspace::~ed_workspace() {
-  if (own) cudaFree(ptr);
-  else if (ptr) ctx->ws_busy = false;
+ed_workspace::ed_workspace(ed_ctx* c, size_t bytes) : ctx(c) {
+  ptr = pool().take(&c->scratch, bytes, ED_WS_KEEP, &own);
 }
+
+ed_workspace::~ed_workspace() { pool().give(&ctx->scratch, ptr, own); }
 
 extern "C" {
 
@@ -84,7 +88,16 @@ int ed_ctx_create(int device, void* stream, ed_ctx** out) {
     if (e != cudaSuccess) { delete c; return ed_cuda_fail(e, "cudaStreamCreate", __FILE__, __LINE__); }
     c->own_stream = true;
   }
+  c->scratch.device = device;
+  pool().add(&c->scratch);
   *out = c;
+  return ED_OK;
+}
+
+int ed_ctx_trim(ed_ctx* c) {
+  if (!c) return ed_fail(ED_EINVAL, "null context");
+  ED_CUDA(cudaSetDevice(c->device));
+  pool().trim(&c->scratch);
   return ED_OK;
 }
 
@@ -121,7 +134,7 @@ int ed_ctx_destroy(ed_ctx* c) {
   clear_profile(c);
   if (c->d_red) cudaFree(c->d_red);
   if (c->h_red) cudaFreeHost(c->h_red);
-  if (c->ws) cudaFree(c->ws);
+  pool().remove(&c->scratch);
   if (c->d_counter) cudaFree(c->d_counter);
   if (c->own_stream) cudaStreamDestroy(c->stream);
   delete c;
@@ -147,7 +160,7 @@ int ed_vec_create(ed_ctx* ctx, int64_t n, ed_cplx** vec_dev) {
   if (!ctx || !vec_dev || n < 0) return ed_fail(ED_EINVAL, "bad argument");
   ED_CUDA(cudaSetDevice(ctx->device));
   void* p = nullptr;
-  if (cudaMalloc(&p, sizeof(ed_cplx) * (size_t)std::max<int64_t>(n, 1)) != cudaSuccess) {
+  if (ed_malloc(&p, sizeof(ed_cplx) * (size_t)std::max<int64_t>(n, 1)) != cudaSuccess) {
     cudaGetLastError();
     return ed_fail(ED_ENOMEM, "vector does not fit in device memory");
   }
@@ -202,8 +215,8 @@ int ed_basis_create(ed_ctx* ctx, int nspins, int total_mag, ed_basis** out) {
   b->dim = compute_size(nspins, b->nup);
   int rc = ed_build_rank_tables(nspins, b->nup, b->rt, b->h_tab);
   if (rc != ED_OK) { delete b; return rc; }
-  cudaError_t e1 = cudaMalloc(&b->d_states, sizeof(uint32_t) * (size_t)b->dim);
-  cudaError_t e2 = cudaMalloc(&b->d_tab, sizeof(uint32_t) * (size_t)b->rt.total);
+  cudaError_t e1 = ed_malloc(&b->d_states, sizeof(uint32_t) * (size_t)b->dim);
+  cudaError_t e2 = ed_malloc(&b->d_tab, sizeof(uint32_t) * (size_t)b->rt.total);
   if (e1 != cudaSuccess || e2 != cudaSuccess) {
     cudaGetLastError();
     if (b->d_states) cudaFree(b->d_states);
@@ -273,8 +286,8 @@ int ed_basis_rank_host(const ed_basis* b, const uint64_t* states_host, int64_t* 
   ed_ctx* ctx = b->ctx;
   uint32_t* ds = nullptr;
   int64_t* dr = nullptr;
-  ED_CUDA(cudaMalloc(&ds, sizeof(uint32_t) * (size_t)n));
-  ED_CUDA(cudaMalloc(&dr, sizeof(int64_t) * (size_t)n));
+  ED_CUDA(ed_malloc(&ds, sizeof(uint32_t) * (size_t)n));
+  ED_CUDA(ed_malloc(&dr, sizeof(int64_t) * (size_t)n));
   ED_CUDA(cudaMemcpyAsync(ds, s.data(), sizeof(uint32_t) * (size_t)n, cudaMemcpyHostToDevice, ctx->stream));
   int rc = ed_launch_rank(ctx, b, ds, n, dr);
   if (rc == ED_OK) {
@@ -295,8 +308,8 @@ int ed_basis_unrank_host(const ed_basis* b, const int64_t* ranks_host, uint64_t*
   ed_ctx* ctx = b->ctx;
   uint32_t* ds = nullptr;
   int64_t* dr = nullptr;
-  ED_CUDA(cudaMalloc(&ds, sizeof(uint32_t) * (size_t)n));
-  ED_CUDA(cudaMalloc(&dr, sizeof(int64_t) * (size_t)n));
+  ED_CUDA(ed_malloc(&ds, sizeof(uint32_t) * (size_t)n));
+  ED_CUDA(ed_malloc(&dr, sizeof(int64_t) * (size_t)n));
   ED_CUDA(cudaMemcpyAsync(dr, ranks_host, sizeof(int64_t) * (size_t)n, cudaMemcpyHostToDevice, ctx->stream));
   int rc = ed_launch_unrank(ctx, b, dr, n, ds);
   std::vector<uint32_t> s((size_t)n);
@@ -384,7 +397,7 @@ int ed_lattice_bonds(int ltype, int nspins, int lx, int ly, int32_t* nn_pairs, i
 static int ham_alloc(ed_ctx* ctx, const ed_basis* b, ed_ham* h) {
   h->ctx = ctx;
   h->basis = b;
-  if (cudaMalloc(&h->d_diag, sizeof(double) * (size_t)b->dim) != cudaSuccess) {
+  if (ed_malloc(&h->d_diag, sizeof(double) * (size_t)b->dim) != cudaSuccess) {
     cudaGetLastError();
     return ed_fail(ED_ENOMEM, "diagonal does not fit in device memory");
   }
@@ -547,8 +560,8 @@ int ed_ham_apply_host(ed_ham* h, const ed_cplx* x_host, ed_cplx* y_host) {
   if (!h || !x_host || !y_host) return ed_fail(ED_EINVAL, "null argument");
   ed_ctx* ctx = h->ctx;
   const size_t bytes = sizeof(double2) * (size_t)h->basis->dim;
-  if (!h->d_x) ED_CUDA(cudaMalloc(&h->d_x, bytes));
-  if (!h->d_y) ED_CUDA(cudaMalloc(&h->d_y, bytes));
+  if (!h->d_x) ED_CUDA(ed_malloc(&h->d_x, bytes));
+  if (!h->d_y) ED_CUDA(ed_malloc(&h->d_y, bytes));
   ED_CUDA(cudaMemcpyAsync(h->d_x, x_host, bytes, cudaMemcpyHostToDevice, ctx->stream));
   ED_TRY(ed_launch_hv(h, h->d_x, h->d_y));
   ED_CUDA(cudaMemcpyAsync(y_host, h->d_y, bytes, cudaMemcpyDeviceToHost, ctx->stream));

@@ -386,7 +386,7 @@ static int eps_solve_real(ed_eps* e, int* nconv_out, int m, int nev, double tol,
   // columns a multiple of 128 bytes apart (16-byte loads of row pairs), the
   // work vector and the device state behind them
   const int64_t ld = (n + 15) & ~(int64_t)15;
-  if (cudaMalloc(&e->pool_r, sizeof(double) * (size_t)ld * (e->pool_cols + 1) + sizeof(KrState)) != cudaSuccess) {
+  if (ed_malloc(&e->pool_r, sizeof(double) * (size_t)ld * (e->pool_cols + 1) + sizeof(KrState)) != cudaSuccess) {
     cudaGetLastError();
     eps_free(e);
     return ed_fail(ED_ENOMEM, "Krylov basis does not fit in device memory");
@@ -510,8 +510,8 @@ static int eps_solve_impl(ed_eps* e, int* nconv_out) {
     if (real_start && ed_lin_supported(H)) return eps_solve_real(e, nconv_out, m, nev, tol, max_it);
   }
   e->pool_cols = 2 * m + 1;
-  if (cudaMalloc(&e->pool, sizeof(double2) * (size_t)n * e->pool_cols) != cudaSuccess ||
-      cudaMalloc(&e->w, sizeof(double2) * (size_t)n) != cudaSuccess) {
+  if (ed_malloc(&e->pool, sizeof(double2) * (size_t)n * e->pool_cols) != cudaSuccess ||
+      ed_malloc(&e->w, sizeof(double2) * (size_t)n) != cudaSuccess) {
     cudaGetLastError();
     eps_free(e);
     return ed_fail(ED_ENOMEM, "Krylov basis does not fit in device memory");
@@ -694,7 +694,7 @@ int ed_eps_set_initial_vector(ed_eps* e, const ed_cplx* v, int on_device) {
     return ED_OK;
   }
   const size_t bytes = sizeof(double2) * (size_t)e->h->basis->dim;
-  if (!e->v0) ED_CUDA(cudaMalloc(&e->v0, bytes));
+  if (!e->v0) ED_CUDA(ed_malloc(&e->v0, bytes));
   ED_CUDA(cudaMemcpyAsync(e->v0, v, bytes, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, ctx->stream));
   return ED_OK;
 }

@@ -587,9 +587,9 @@ __global__ void __launch_bounds__(256) k_hv_fx64(const uint32_t* __restrict__ st
 static int ensure_fixed_buffers(ed_ham* h) {
   const int64_t dim = h->basis->dim;
   if (!h->d_xq) {
-    if (cudaMalloc(&h->d_xq, sizeof(longlong2) * (size_t)dim) != cudaSuccess ||
-        cudaMalloc(&h->d_xe, sizeof(uint16_t) * (size_t)((dim + 31) / 32)) != cudaSuccess ||
-        cudaMalloc(&h->d_gmax, ED_GMAX_BYTES) != cudaSuccess) {
+    if (ed_malloc(&h->d_xq, sizeof(longlong2) * (size_t)dim) != cudaSuccess ||
+        ed_malloc(&h->d_xe, sizeof(uint16_t) * (size_t)((dim + 31) / 32)) != cudaSuccess ||
+        ed_malloc(&h->d_gmax, ED_GMAX_BYTES) != cudaSuccess) {
       cudaGetLastError();
       return ed_fail(ED_ENOMEM, "H.v scratch does not fit in device memory");
     }
@@ -1024,14 +1024,14 @@ static int csr_build_k(ed_ham* h) {
   for (int i = 0; i < ub.n; ++i) { ub.mask[i] = masks[i]; ub.val[i] = vals[i]; }
   const int64_t dim = b->dim;
   int64_t* counts = nullptr;
-  ED_CUDA(cudaMalloc(&counts, sizeof(int64_t) * (size_t)dim));
-  if (!h->d_rowptr) ED_CUDA(cudaMalloc(&h->d_rowptr, sizeof(int64_t) * (size_t)(dim + 1)));
+  ED_CUDA(ed_malloc(&counts, sizeof(int64_t) * (size_t)dim));
+  if (!h->d_rowptr) ED_CUDA(ed_malloc(&h->d_rowptr, sizeof(int64_t) * (size_t)(dim + 1)));
   k_csr_count<K><<<grid_cap(ctx, dim, 256, 8), 256, 0, ctx->stream>>>(b->d_states, dim, dp, ub, counts);
   ED_CHECK_LAUNCH(ctx);
   const int nblk = std::max(1, std::min<int>(4096, (int)((dim + 4095) / 4096)));
   const int64_t per_block = (dim + nblk - 1) / nblk;
   int64_t* sums = nullptr;
-  ED_CUDA(cudaMalloc(&sums, sizeof(int64_t) * nblk));
+  ED_CUDA(ed_malloc(&sums, sizeof(int64_t) * nblk));
   k_scan_blocks<<<nblk, 256, 0, ctx->stream>>>(counts, dim, per_block, sums);
   ED_CHECK_LAUNCH(ctx);
   std::vector<int64_t> hs(nblk), ho(nblk);
@@ -1045,8 +1045,8 @@ static int csr_build_k(ed_ham* h) {
   const int64_t nnz = acc;
   if (h->d_cols) { cudaFree(h->d_cols); h->d_cols = nullptr; }
   if (h->d_vals) { cudaFree(h->d_vals); h->d_vals = nullptr; }
-  cudaError_t e1 = cudaMalloc(&h->d_cols, sizeof(uint32_t) * (size_t)std::max<int64_t>(nnz, 1));
-  cudaError_t e2 = cudaMalloc(&h->d_vals, sizeof(double) * (size_t)std::max<int64_t>(nnz, 1));
+  cudaError_t e1 = ed_malloc(&h->d_cols, sizeof(uint32_t) * (size_t)std::max<int64_t>(nnz, 1));
+  cudaError_t e2 = ed_malloc(&h->d_vals, sizeof(double) * (size_t)std::max<int64_t>(nnz, 1));
   if (e1 != cudaSuccess || e2 != cudaSuccess) {
     cudaGetLastError();
     cudaFree(counts); cudaFree(sums);

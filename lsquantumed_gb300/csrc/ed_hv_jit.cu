@@ -746,7 +746,7 @@ int ed_jit_launch(ed_ham* h, uint64_t signature, int budget, const void* x, void
     if (h->jit_t1n) cudaFree(h->jit_t1n);
     h->jit_t1n = nullptr;
     h->jit_t1n_key = nullptr;
-    if (cudaMalloc(&h->jit_t1n, bytes) != cudaSuccess) {
+    if (ed_malloc(&h->jit_t1n, bytes) != cudaSuccess) {
       cudaGetLastError();
       h->jit_t1n = nullptr;
       return ed_fail(ED_ENOMEM, "neighbour table of the run-time compiled H.v does not fit in device memory");

@@ -82,8 +82,8 @@ int ed_basis_lin_tables(ed_basis* b) {
     }
     t1[c] = (uint32_t)v;
   }
-  if (cudaMalloc(&b->d_lin_t0, t0.size() * sizeof(uint16_t)) != cudaSuccess ||
-      cudaMalloc(&b->d_lin_t1, t1.size() * sizeof(uint32_t)) != cudaSuccess) {
+  if (ed_malloc(&b->d_lin_t0, t0.size() * sizeof(uint16_t)) != cudaSuccess ||
+      ed_malloc(&b->d_lin_t1, t1.size() * sizeof(uint32_t)) != cudaSuccess) {
     cudaGetLastError();
     return ed_fail(ED_ENOMEM, "rank tables do not fit in device memory");
   }
@@ -104,8 +104,8 @@ int ed_basis_lin_tables(ed_basis* b) {
   for (int k = 0; k <= w1; ++k)
     for (uint32_t c = 0; c < t1.size(); ++c)
       if (__builtin_popcount(c) == k) highs.push_back(c);
-  if (cudaMalloc(&b->d_lin_lows, lows.size() * sizeof(uint16_t)) != cudaSuccess ||
-      cudaMalloc(&b->d_lin_highs, highs.size() * sizeof(uint32_t)) != cudaSuccess) {
+  if (ed_malloc(&b->d_lin_lows, lows.size() * sizeof(uint16_t)) != cudaSuccess ||
+      ed_malloc(&b->d_lin_highs, highs.size() * sizeof(uint32_t)) != cudaSuccess) {
     cudaGetLastError();
     return ed_fail(ED_ENOMEM, "rank tables do not fit in device memory");
   }
@@ -172,7 +172,7 @@ static int lin_prepare(ed_ham* h) {
       const int kc = 125 - ed_fx64_sbits(h) - lg;
       for (double v : cf) L->coef.push_back(std::llround(std::ldexp(v, kc - e)));
       L->pbexp = e - kc;
-      if (!L->d_coef && cudaMalloc(&L->d_coef, sizeof(long long) * ED_MAX_BONDS) != cudaSuccess) {
+      if (!L->d_coef && ed_malloc(&L->d_coef, sizeof(long long) * ED_MAX_BONDS) != cudaSuccess) {
         cudaGetLastError();
         L->d_coef = nullptr;
         return ed_fail(ED_ENOMEM, "per-bond coefficient table does not fit in device memory");

@@ -5,6 +5,7 @@
 #include <string>
 #include <vector>
 #include "../../include/ed_capi.h"
+#include "ed_pool.h"
 
 #define ED_MAX_BONDS 256
 #define ED_MAX_TYPES 256
@@ -95,10 +96,7 @@ struct ed_ctx {
   // blocks-done counter of the kernels whose last block finishes a reduction
   // (zero between launches)
   unsigned* d_counter = nullptr;
-  // scratch kept between calls (ed_workspace), at most ED_WS_KEEP bytes
-  void* ws = nullptr;
-  size_t ws_cap = 0;
-  bool ws_busy = false;
+  ed_scratch_slot scratch;  // kept between calls (ed_workspace), at most ED_WS_KEEP bytes
   // H.v launch timing (events on the stream)
   bool profiling = false;
   std::vector<cudaEvent_t> prof_events;  // pairs (start, stop)
@@ -121,9 +119,18 @@ struct ed_basis {
   uint32_t* d_lin_highs = nullptr;
 };
 
+// cudaMalloc of the library: where the device is full, the scratch that contexts
+// keep (ed_pool.h) is given back and the allocation tried once more.
+cudaError_t ed_malloc_bytes(void** p, size_t bytes);
+template <typename T>
+cudaError_t ed_malloc(T** p, size_t bytes) {
+  return ed_malloc_bytes((void**)p, bytes);
+}
+
 // Device scratch of one call, in stream order: the context keeps up to
 // ED_WS_KEEP bytes from call to call (an allocation and its free cost more
-// than a small measurement); a larger request is allocated and freed with
+// than a small measurement), until ed_ctx_trim, the context's end, or an
+// allocation that needs the room; a larger request is allocated and freed with
 // the call.  ptr is null when it does not fit.
 #define ED_WS_KEEP ((size_t)512 << 20)
 struct ed_workspace {

@@ -27,7 +27,7 @@ int ed_ensure_reduce(ed_ctx* ctx, size_t doubles) {
   ctx->d_red = nullptr;
   ctx->h_red = nullptr;
   size_t cap = std::max<size_t>(doubles, 1 << 16);
-  ED_CUDA(cudaMalloc(&ctx->d_red, cap * sizeof(double)));
+  ED_CUDA(ed_malloc(&ctx->d_red, cap * sizeof(double)));
   ED_CUDA(cudaMallocHost(&ctx->h_red, cap * sizeof(double)));
   ctx->red_cap = cap;
   return ED_OK;
@@ -35,7 +35,7 @@ int ed_ensure_reduce(ed_ctx* ctx, size_t doubles) {
 
 int ed_ensure_counter(ed_ctx* ctx) {
   if (ctx->d_counter) return ED_OK;
-  ED_CUDA(cudaMalloc(&ctx->d_counter, 256));
+  ED_CUDA(ed_malloc(&ctx->d_counter, 256));
   ED_CUDA(cudaMemsetAsync(ctx->d_counter, 0, 256, ctx->stream));
   return ED_OK;
 }
@@ -427,7 +427,7 @@ __global__ void k_imag_any(const double2* __restrict__ v, int64_t n, int* __rest
 
 int ed_is_real(ed_ctx* ctx, const double2* v, int64_t n, bool* real) {
   int* d_any = nullptr;
-  ED_CUDA(cudaMalloc(&d_any, sizeof(int)));
+  ED_CUDA(ed_malloc(&d_any, sizeof(int)));
   int h_any = 0;
   cudaError_t e = cudaMemsetAsync(d_any, 0, sizeof(int), ctx->stream);
   if (e == cudaSuccess) {

@@ -99,7 +99,7 @@ int time_probe(ed_ctx* ctx, F launch, double flops, double* tflops) {
 extern "C" int ed_probe_rates(ed_ctx* ctx, double* dfma_tflops, double* dmma_tflops, double* hmma_tflops) {
   if (!ctx) return ed_fail(ED_EINVAL, "null context");
   double* sink = nullptr;
-  ED_CUDA(cudaMalloc(&sink, 64));
+  ED_CUDA(ed_malloc(&sink, 64));
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_peak_dfma, PK_THREADS, 0);
   const int grid = ctx->num_sms * std::max(per_sm, 1);

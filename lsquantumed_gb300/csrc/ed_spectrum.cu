@@ -55,7 +55,7 @@ extern "C" int ed_dsf_spectrum(ed_ctx* ctx, int nspins, int nev, const ed_cplx* 
   const size_t bytes = sizeof(double2) * nc + sizeof(double) * ((size_t)nev + 2 * (size_t)nq + 2 * (size_t)nspins +
                                                                 (size_t)nq * nev);
   char* buf = nullptr;
-  ED_CUDA(cudaMalloc(&buf, bytes));
+  ED_CUDA(ed_malloc(&buf, bytes));
   double2* c = (double2*)buf;
   double* dE = (double*)(c + nc);
   double* q = dE + nev;

@@ -128,6 +128,10 @@ class Environment:
     def synchronize(self):
         call('ed_ctx_synchronize', self._h)
 
+    def trim(self):
+        """Give the device scratch that measurements keep (up to 512 MB) back."""
+        call('ed_ctx_trim', self._h)
+
     def kernel_count(self):
         c = ctypes.c_int64()
         call('ed_ctx_kernel_count', self._h, ctypes.byref(c))
