@@ -198,7 +198,8 @@ int ed_ham_size(const ed_ham* h, int64_t* size);
  * reference; for reports. */
 int ed_ham_hv_variant(const ed_ham* h, int dot, char* buf, size_t len);
 /* Force the matrix-free H.v launch variant: "u4-b6", "u4-b4", "u8-b4",
- * "u8-b1" (static kernels: unroll depth and register budget), "jit" /
+ * "u8-b1" (static kernels: unroll depth and register budget), "u8-t64" (blocks
+ * of 64 threads, the choice below 256 rows per SM), "jit" /
  * "jit-b4" / "jit-b3" (kernel compiled at run time for this operator's bonds,
  * blocks of 256 threads, 2 / 4 / 3 blocks per SM), "jit-w3" / "jit-w4" (the
  * same with one block of 768 / 1024 threads per SM) or "auto" (autotuner,

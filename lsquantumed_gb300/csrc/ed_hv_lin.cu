@@ -397,17 +397,19 @@ typedef void (*LinKernel)(const uint32_t*, const double*, const double2*, const 
 struct LinVariant {
   LinKernel plain, dot;
   const char* name;
+  int nt;  // threads per block
 };
 static const LinVariant kLinVariants[] = {
-    {k_hv_lin<false, 4, 6>, k_hv_lin<true, 4, 5>, "u4-b6"},
-    {k_hv_lin<false, 4, 4>, k_hv_lin<true, 4, 4>, "u4-b4"},
-    {k_hv_lin<false, 8, 4>, k_hv_lin<true, 8, 4>, "u8-b4"},
-    {k_hv_lin<false, 8, 1>, k_hv_lin<true, 8, 1>, "u8-b1"},
+    {k_hv_lin<false, 4, 6>, k_hv_lin<true, 4, 5>, "u4-b6", 256},
+    {k_hv_lin<false, 4, 4>, k_hv_lin<true, 4, 4>, "u4-b4", 256},
+    {k_hv_lin<false, 8, 4>, k_hv_lin<true, 8, 4>, "u8-b4", 256},
+    {k_hv_lin<false, 8, 1>, k_hv_lin<true, 8, 1>, "u8-b1", 256},
+    // the choice for fewer rows than 256 threads per SM: blocks of 64, so that every
+    // SM takes part (the FP64 work of a row and the sums are what a block waits for)
+    {k_hv_lin<false, 8, 1, 64>, k_hv_lin<true, 8, 1, 64>, "u8-t64", 64},
 };
-// Fewer rows than 256 threads per SM: blocks of 64, so that every SM takes
-// part (the FP64 work of a row and the sums are what a block waits for).
-static const LinKernel kLinSmall[2] = {k_hv_lin<false, 8, 1, 64>, k_hv_lin<true, 8, 1, 64>};
 static const int kNumLinVariants = (int)(sizeof(kLinVariants) / sizeof(kLinVariants[0]));
+static const int kSmallVariant = kNumLinVariants - 1;
 
 // Variants kNumLinVariants + 0 .. 4 are the run-time specialised kernel
 // (ed_hv_jit.cu) with its five register budgets and block shapes.
@@ -426,9 +428,8 @@ static int lin_launch(ed_ham* h, int v, const void* x, void* y, bool dot, int sb
     return ed_jit_launch(h, lin_signature(h), v - kJitVariant, x, y, dot, sbits, nblk_out, L->segs.word, L->segs.seg,
                          L->segs.w0, rio, L->per_bond ? L->coef.data() : nullptr, L->d_coef, L->pbexp, skip);
   const size_t smem = sizeof(uint16_t) * ((size_t)1 << b->lin_w0);
-  const bool small = b->dim < (int64_t)ctx->num_sms * 256;
-  const int nt = small ? 64 : 256;
-  LinKernel k = small ? kLinSmall[dot ? 1 : 0] : dot ? kLinVariants[v].dot : kLinVariants[v].plain;
+  const int nt = kLinVariants[v].nt;
+  LinKernel k = dot ? kLinVariants[v].dot : kLinVariants[v].plain;
   int per_sm = 0;
   ED_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, nt, smem));
   if (per_sm < 1) per_sm = 1;
@@ -469,7 +470,7 @@ static int lin_autotune(ed_ham* h, const void* x, void* y, int sbits, bool dot, 
   ed_lin* L = h->lin;
   ed_ctx* ctx = h->ctx;
   int& chosen = L->variant[2 * (dot ? 1 : 0) + (rio ? 1 : 0)];
-  chosen = L->per_bond ? kJitVariant + 1 : 0;
+  chosen = L->per_bond ? kJitVariant + 1 : h->basis->dim < (int64_t)ctx->num_sms * 256 ? kSmallVariant : 0;
   if (h->basis->dim < (int64_t)1 << 20) return ED_OK;
   const auto key =
       std::make_tuple(ctx->device, h->basis->nspins, h->basis->nup, lin_signature(h), dot ? 1 : 0, rio ? 1 : 0);
@@ -488,6 +489,7 @@ static int lin_autotune(ed_ham* h, const void* x, void* y, int sbits, bool dot, 
   int rc = ED_OK;
   bool first = true;
   for (int v = L->per_bond ? kJitVariant : 0; v < kNumAllVariants && rc == ED_OK; ++v) {
+    if (v == kSmallVariant) continue;  // not for vectors of this length
     rc = lin_launch(h, v, x, y, dot, sbits, nullptr, rio, skip);
     if (v >= kJitVariant && rc == ED_ENOTSUP) {  // no run-time compiler here: keep the static choice
       rc = ED_OK;
