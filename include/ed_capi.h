@@ -337,11 +337,14 @@ int ed_batch_set_restart_arithmetic(ed_batch* bt, int mode);
 
 /* ---- measurements: replace SiSj/SzSz/SpSm/SmSp::ExpectVal
  *      (src/spinOperators/correlation.cpp:38-299) --------------------------- */
-/* out[p] = ExpectVal(op, i_p, j_p, psi) for npairs pairs, 16 per pass over
- * the basis (PETSc VecDot convention: sum_s psi_s * conj((O psi)_s)).  For a
- * real psi (every imaginary part zero, as the solver's eigenvectors), the
- * S^z S^z part and the one-site sums are exact integer sums of the FP64
- * weights psi_s^2 rounded once, and the call holds a copy of the real parts (8 *
+/* out[p] = ExpectVal(op, i_p, j_p, psi) for npairs pairs (PETSc VecDot
+ * convention: sum_s psi_s * conj((O psi)_s)).  For a real psi (every imaginary
+ * part zero, as the solver's eigenvectors), the S^z S^z part and the one-site
+ * sums are exact integer sums of the FP64 weights psi_s^2 rounded once; flip sums
+ * are FP64 for up to 16 pairs of different sites, beyond that exact sums of
+ * amplitudes in 63 bits against the largest one, and FP64 again for a sum below
+ * 2^-9 of that one's binade times the norm, so that the list's length does not
+ * change the accuracy.  The call holds a copy of the real parts (8 *
  * dim bytes) in the context's scratch (ed_ctx_trim); without room for it, or for
  * a non-finite psi, the general FP64 kernel runs instead. */
 int ed_expect_pairs(const ed_basis* b, int op, const ed_cplx* psi_dev, const int32_t* pairs_host,
