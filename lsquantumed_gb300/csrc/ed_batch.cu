@@ -349,7 +349,7 @@ struct BCols {
 #define BU_REG 16  // k_batch_update_norm keeps up to this many coefficients in registers
 // With vj: first w <- w - a_b vj - bet_b vjm1 (coef = [a][B], [bet][B]),
 // written back, in the same pass (the local Lanczos projection).
-// A thread adds its rows in two chains: three blocks' chains are a third longer
+// A thread adds many rows in two chains: three blocks' chains are a third longer
 // than four blocks', and with them the rounding.
 // One instance per column count NI (0: the norm alone): the loads of a row are
 // issued together, without a test per column.  More than BD_MAXV columns: the
@@ -376,7 +376,8 @@ __global__ void __launch_bounds__(256, BD_PER_SM) k_batch_dots(const BCols V, in
     bool two = false;  // the first chain's sums are in this thread's places of sh
     if (lane_r < S && b < B) {
       const double ca = vj ? coef[b] : 0.0, cb = vj ? coef[B + b] : 0.0;
-      const int64_t half = r0 + lane_r + ((r1 - r0 + S - 1) / S + 1) / 2 * S;
+      const int64_t steps = (r1 - r0 + S - 1) / S;
+      const int64_t half = r0 + lane_r + (steps < 32 ? steps : (steps + 1) / 2) * S;
       for (int64_t r = r0 + lane_r; r < r1; r += S) {
         if (r == half) {
 #pragma unroll

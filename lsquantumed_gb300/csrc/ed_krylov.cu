@@ -92,8 +92,14 @@ __device__ __forceinline__ double block_sums16(const double (&acc)[KR_GROUP], in
   const int item = threadIdx.x >> 4, l = threadIdx.x & 15;
   double a = 0.0;
   if (item < ni) {
+    double t[16];  // pairwise: half the rounding of one after the other, as many adds
 #pragma unroll
-    for (int q = 0; q < 16; ++q) a += sh[item * (KR_THREADS + 1) + l + 16 * q];
+    for (int q = 0; q < 16; ++q) t[q] = sh[item * (KR_THREADS + 1) + l + 16 * q];
+#pragma unroll
+    for (int w = 8; w > 0; w >>= 1)
+#pragma unroll
+      for (int q = 0; q < w; ++q) t[q] += t[q + w];
+    a = t[0];
   }
 #pragma unroll
   for (int s = 8; s > 0; s >>= 1) a += __shfl_down_sync(0xffffffffu, a, s, 16);
@@ -116,12 +122,20 @@ __device__ __forceinline__ double block_sum256(double v, double* sh) {
   return a;
 }
 
-// A thread adds its rows in two chains, so that half as many threads with more
-// registers each do not mean longer chains: with one, and two blocks per SM, the
-// root mean square error of 16 dots of 10M rows was 1.32 times that of four
-// blocks per SM.  One more add per column and thread: 13 dots of 2.7M rows
-// 99 -> 100 us (four chains: 113).  Steps of one chain, of all:
-__device__ __forceinline__ int64_t kr_chain(int64_t steps) { return (steps + 1) / 2; }
+// Rounding of the dots.  Half as many threads with more registers each would mean
+// chains twice as long, so a thread adds its rows in two: with one, and two blocks
+// per SM, the root mean square error of 16 dots of 10M rows was 1.32 times that of
+// four blocks per SM.  One more add per column and thread, so only from KR_CHAIN
+// rows on (2.7M rows, 16 columns: 116 -> 123 us); below, the sums over threads and
+// blocks round more, and those are pairwise and in four chains.  Errors of 16 dots
+// in units of 1e-16 / sqrt(n), one chain and sequential sums -> now (four blocks
+// per SM): 13k rows 2.14 -> 1.95 (1.97), 185k 2.71 -> 2.22 (2.21), 705k 2.85 -> 2.27
+// (2.23), 2.7M 3.11 -> 2.46 (2.49), 10.4M 5.14 -> 3.61 (3.77).  Steps of the first
+// chain, of all steps of rows each:
+constexpr int KR_CHAIN = 32;
+__device__ __forceinline__ int64_t kr_chain(int64_t steps, int rows) {
+  return steps * rows < KR_CHAIN ? steps : (steps + 1) / 2;
+}
 
 // Blocks per SM of k_kr_dots: registers for the loads of a row in flight.
 __host__ __device__ constexpr int kr_dots_per_sm(int ng) { return ng > 8 ? 2 : 3; }
@@ -154,7 +168,7 @@ __global__ void __launch_bounds__(KR_THREADS, kr_dots_per_sm(NG)) k_kr_dots(cons
   __shared__ double sh[NG * (KR_THREADS + 1)];
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t half = r + kr_chain((n + U * stride - 1) / (U * stride)) * (U * stride);
+  const int64_t half = r + kr_chain((n + U * stride - 1) / (U * stride), U) * (U * stride);
   bool two = false;  // the first chain's sums are in this thread's places of sh
   for (; r + (U - 1) * stride < n; r += U * stride) {
     if (r == half) {
@@ -207,8 +221,15 @@ __global__ void __launch_bounds__(KR_THREADS, kr_dots_per_sm(NG)) k_kr_dots(cons
   if (l == 0 && item < NG) partial[(size_t)item * gridDim.x + blockIdx.x] = s;
   if (!ed_last_block(counter)) return;
   double t = 0.0;
-  if (item < NG)
-    for (unsigned q = l; q < gridDim.x; q += 16) t += __ldcg(partial + (size_t)item * gridDim.x + q);
+  if (item < NG) {
+    double c[4] = {0.0, 0.0, 0.0, 0.0};  // four chains of blocks
+    for (unsigned q = l; q < gridDim.x; q += 64) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (q + 16 * k < gridDim.x) c[k] += __ldcg(partial + (size_t)item * gridDim.x + q + 16 * k);
+    }
+    t = (c[0] + c[1]) + (c[2] + c[3]);
+  }
 #pragma unroll
   for (int k = 8; k > 0; k >>= 1) t += __shfl_down_sync(0xffffffffu, t, k, 16);
   if (l == 0 && item < NG) out[item] = t;
@@ -274,7 +295,7 @@ __global__ void __launch_bounds__(KR_THREADS, NV > 8 ? 3 : 4) k_kr_update(const 
   if (NV > 0) {
     constexpr int U = NV <= 3 ? 4 : NV <= 8 ? 2 : 1;  // rows in flight per thread
     int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t half = r + kr_chain((n + U * stride - 1) / (U * stride)) * (U * stride);
+    const int64_t half = r + kr_chain((n + U * stride - 1) / (U * stride), U) * (U * stride);
     double before = 0.0;  // the first chain
     for (; r < n; r += U * stride) {
       if (r == half) {
