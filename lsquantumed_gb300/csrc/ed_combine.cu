@@ -28,8 +28,8 @@
 // per thread, and the fragment layout lets the thread that loads and splits
 // the entries also own the accumulators of the same rows, so nothing passes
 // through shared memory.  The splitting and rounding bound the kernel.  At 40.1M
-// rows and 16 columns: 8 outputs 5.90 -> 3.12 ms, 9 outputs 7.13 -> 4.10 ms, 15
-// outputs 4.55 ms (58 bits: 2.39, 3.25 and 3.54 ms).  Conversion costs more
+// rows and 16 columns: 8 outputs 5.90 -> 3.02 ms, 9 outputs 7.13 -> 3.99 ms, 15
+// outputs 4.40 ms (58 bits: 2.39, 3.25 and 3.54 ms).  Conversion costs more
 // than 16 FP64 FMAs per entry group, so the Gram-Schmidt dots and updates, one
 // FMA per entry, stay FP64.
 //
@@ -49,7 +49,7 @@ constexpr int CB_DIG = 7, CB_LEV = 7;
 constexpr int CB_MAXM = 127;
 constexpr int CB_CELL = 4;  // 16-byte words per lane and cell: 14 words of digits
 constexpr int CB_THREADS = 128;
-constexpr int CB_MINB = 4;  // 128 registers: nine outputs, 40.1M rows, 3 blocks 4.49 ms, 4 4.10
+constexpr int CB_MINB = 4;  // 128 registers: nine outputs, 40.1M rows, 3 blocks 4.49 ms, 4 3.99
 
 template <int NC>
 struct CombineArgs {
@@ -273,20 +273,17 @@ __device__ __forceinline__ void combine_digits(const double2 (&v)[4], int e0, in
   digit_pairs(digits10(v[2].y, e1), digits10(v[3].y, e1), a[3]);
 }
 
-template <typename Args>
-__device__ __forceinline__ double combine_fp64(const Args& A, int m, int o, int64_t r) {
-  double s = 0.0;
-  for (int i = 0; i < m; ++i) s = fma(A.v[i][r], A.y[i][o], s);
-  return s;
-}
-
 // Rows in FP64 (the four lanes of a row pair).
 template <typename Args>
 __device__ __noinline__ void combine_row_fp64(const Args& A, int m, int nout, int t, bool slow0, bool slow1,
                                               int64_t row, int64_t n) {
   for (int h = 0; h < 2; ++h) {
     if (!(h ? slow1 : slow0) || row + h >= n) continue;
-    for (int o = t; o < nout; o += 4) A.out[o][row + h] = combine_fp64(A, m, o, row + h);
+    for (int o = t; o < nout; o += 4) {
+      double s = 0.0;
+      for (int i = 0; i < m; ++i) s = fma(A.v[i][row + h], A.y[i][o], s);
+      A.out[o][row + h] = s;
+    }
   }
 }
 
@@ -294,23 +291,31 @@ __device__ __noinline__ void combine_row_fp64(const Args& A, int m, int nout, in
 // FP64 where no product reaches 2^-11 of the scales 2^(E + F) that the digits
 // were cut against, or the value may leave the normal range.  Where one does, the
 // value is small because the products cancel, and its error is below m 2^-53 of
-// that product.  One at a time, as they were met, they took 13% of the kernel.
+// that product.  Random orthonormal columns have 0.1% of such values; the restarts
+// of a disordered N=24 solve up to 13%, two thirds of them then FP64: its 19
+// restarts take 2.4 ms of 63.6 for this.  One at a time, as they were met, the
+// random ones took 13% of the kernel; 5.0 ms of the solve with the coefficients
+// read from the kernel's parameters and the entries read twice.
 constexpr int CB_LIST = 64;
 template <typename Args>
-__device__ __noinline__ void combine_small(const Args& A, int m, const unsigned long long* list, int count) {
+__device__ __noinline__ void combine_small(const Args& A, int m, const double (*Y)[16], const unsigned long long* list,
+                                           int count) {
   __syncwarp();  // the list, and the values stored before
   for (int q = threadIdx.x & 31; q < count; q += 32) {
     const int64_t r = (int64_t)(list[q] >> 4);
     const int o = (int)(list[q] & 15u);
     int ev = CB_EMIN, ey = CB_EMIN, ep = 0;  // largest exponents: entry, coefficient, product
+    double s = 0.0;
 #pragma unroll 8
-    for (int i = 0; i < m; ++i) {
-      const int x = biased_exp(A.v[i][r]), y = biased_exp(A.y[i][o]);
+    for (int i = 0; i < m; ++i) {  // one pass: the loads are what a round waits for
+      const double v = A.v[i][r], c = Y[i][o];
+      const int x = biased_exp(v), y = biased_exp(c);
       ev = max(ev, x);
       ey = max(ey, y);
       ep = max(ep, x + y);
+      s = fma(v, c, s);
     }
-    if (ep < ev + ey - 9 || ev + ey < 2044 - 950) A.out[o][r] = combine_fp64(A, m, o, r);
+    if (ep < ev + ey - 9 || ev + ey < 2044 - 950) A.out[o][r] = s;
   }
   __syncwarp();  // the list is free
 }
@@ -325,22 +330,23 @@ __device__ __forceinline__ unsigned combine_mine(int nout) {
   return mine;
 }
 
-// Notes the values of need.  All lanes of the warp.
+// Notes the values of need, one of every lane at a time.  All lanes of the warp.
 template <typename Args>
-__device__ __forceinline__ void combine_note(const Args& A, int m, unsigned need, int64_t row, int64_t n,
-                                             unsigned long long* list, int& count) {
+__device__ __forceinline__ void combine_note(const Args& A, int m, const double (*Y)[16], unsigned need, int64_t row,
+                                             int64_t n, unsigned long long* list, int& count) {
   const int lane = threadIdx.x & 31, t = lane & 3;
-#pragma unroll 1
-  for (int b = 0; b < 8; ++b) {
-    const int o = 8 * (b >> 2) + 2 * t + ((b >> 1) & 1);
-    const int64_t r = row + (b & 1);
-    const bool on = ((need >> b) & 1u) && r < n;
-    const unsigned mk = __ballot_sync(0xffffffffu, on);
+  if (row >= n) need = 0u;
+  if (row + 1 >= n) need &= 0x55u;
+  for (unsigned mk = __ballot_sync(0xffffffffu, need); mk; mk = __ballot_sync(0xffffffffu, need)) {
     if (count + __popc(mk) > CB_LIST) {
-      combine_small(A, m, list, count);
+      combine_small(A, m, Y, list, count);
       count = 0;
     }
-    if (on) list[count + __popc(mk & ((1u << lane) - 1u))] = (unsigned long long)r << 4 | (unsigned)o;
+    if (need) {
+      const int b = __ffs(need) - 1, o = 8 * (b >> 2) + 2 * t + ((b >> 1) & 1);
+      list[count + __popc(mk & ((1u << lane) - 1u))] = (unsigned long long)(row + (b & 1)) << 4 | (unsigned)o;
+      need &= need - 1u;
+    }
     count += __popc(mk);
   }
 }
@@ -383,13 +389,15 @@ template <int NC, int NT, bool VEC>
 __global__ void __launch_bounds__(CB_THREADS, NC == 1 ? CB_MINB : 3) k_combine(const __grid_constant__ CombineArgs<NC> A,
                                                                          int m, int nout, int64_t n) {
   __shared__ uint4 sB[NC * NT * 32 * CB_CELL];
+  __shared__ double sY[16 * NC][16];  // the coefficients, for combine_small
   __shared__ unsigned long long lists[CB_THREADS / 32][CB_LIST];
   unsigned long long* list = lists[threadIdx.x >> 5];
   int count = 0;
   const unsigned mine = combine_mine(nout);
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   int F[NT][2];  // exponents of outputs 8 nt + 2 t, + 1
-  combine_setup<NT>(A, 16 * NC, sB, F);
+  for (int k = threadIdx.x; k < 16 * NC * 16; k += CB_THREADS) sY[k >> 4][k & 15] = A.y[k >> 4][k & 15];
+  combine_setup<NT>(A, 16 * NC, sB, F);  // ends with a barrier
   const double* col[NC][4];
 #pragma unroll
   for (int c = 0; c < NC; ++c)
@@ -475,12 +483,12 @@ __global__ void __launch_bounds__(CB_THREADS, NC == 1 ? CB_MINB : 3) k_combine(c
       }
     }
     need &= rp.keep & mine;
-    if (__any_sync(0xffffffffu, need)) combine_note(A, m, need, row, n, list, count);
+    if (__any_sync(0xffffffffu, need)) combine_note(A, m, sY, need, row, n, list, count);
     __syncwarp();  // the stores above come first
     if (rp.slow0 || rp.slow1) combine_row_fp64(A, m, nout, t, rp.slow0, rp.slow1, row, n);
     __syncwarp();
   }
-  if (count) combine_small(A, m, list, count);
+  if (count) combine_small(A, m, sY, list, count);
 }
 
 // More than 32 columns: the row exponents from a first read of the columns,
@@ -496,7 +504,9 @@ __global__ void __launch_bounds__(CB_THREADS, 3) k_combine_many(const __grid_con
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int ng = (m + 15) / 16, NT = (nout + 7) / 8;
   int F[2][2];
-  combine_setup<2>(A, m, sBd, F);
+  double(*sY)[16] = (double(*)[16])(sBd + ng * 2 * 32 * CB_CELL);  // the coefficients, for combine_small
+  for (int k = threadIdx.x; k < m * 16; k += CB_THREADS) sY[k >> 4][k & 15] = A.y[k >> 4][k & 15];
+  combine_setup<2>(A, m, sBd, F);  // ends with a barrier
   const int64_t stride = (int64_t)gridDim.x * (CB_THREADS / 32) * 16;
   for (int64_t r = ((int64_t)blockIdx.x * (CB_THREADS / 32) + (threadIdx.x >> 5)) * 16; r < n; r += stride) {
     const int64_t row = r + 2 * g;
@@ -558,17 +568,18 @@ __global__ void __launch_bounds__(CB_THREADS, 3) k_combine_many(const __grid_con
         combine_out<VEC>(A, 8 * nt + 2 * t + k, res, nout, row, n);
       }
     need &= rp.keep & mine;
-    if (__any_sync(0xffffffffu, need)) combine_note(A, m, need, row, n, list, count);
+    if (__any_sync(0xffffffffu, need)) combine_note(A, m, sY, need, row, n, list, count);
     __syncwarp();  // the stores above come first
     if (rp.slow0 || rp.slow1) combine_row_fp64(A, m, nout, t, rp.slow0, rp.slow1, row, n);
     __syncwarp();
   }
-  if (count) combine_small(A, m, list, count);
+  if (count) combine_small(A, m, sY, list, count);
 }
 
 template <int NC, int NT, bool VEC>
 int combine_launch(ed_ctx* ctx, const CombineArgs<NC>& A, int m, int nout, int64_t n) {
   auto go = [&](auto kern, size_t smem) -> int {
+    if (smem > 0) ED_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     ED_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, CB_THREADS, smem));
     const int64_t tiles = (n + 15) / 16, b = (tiles + CB_THREADS / 32 - 1) / (CB_THREADS / 32);
@@ -577,7 +588,7 @@ int combine_launch(ed_ctx* ctx, const CombineArgs<NC>& A, int m, int nout, int64
     ED_CHECK_LAUNCH(ctx);
     return ED_OK;
   };
-  if constexpr (NC > 2) return go(k_combine_many<VEC>, sizeof(uint4) * (size_t)((m + 15) / 16) * 2 * 32 * CB_CELL);
+  if constexpr (NC > 2) return go(k_combine_many<VEC>, sizeof(uint4) * (size_t)((m + 15) / 16) * 2 * 32 * CB_CELL + sizeof(double) * 16 * (size_t)m);
   else return go(k_combine<NC, NT, VEC>, 0);
 }
 
