@@ -313,14 +313,13 @@ int ed_grad_energy(const ed_basis* b, const int32_t* pairs_host, int64_t nbonds,
     ed_corr c;
     const int rc = ed_corr_real(b, (const double2*)psi_dev, (const double2*)psi_dev, true, pairs_host, nbonds, c);
     if (rc == ED_OK) {
-      const double inv = 1.0 / c.W;
       for (int64_t q = 0; q < nbonds; ++q) {
         const int i = pairs_host[2 * q], j = pairs_host[2 * q + 1];
-        if (dJ_host) dJ_host[q] = (i == j ? 0.5 * c.zz(i, i) : c.F[q]) * inv;
-        if (dD_host) dD_host[q] = 0.25 * c.zz(i, j) * inv;
+        if (dJ_host) dJ_host[q] = (i == j ? 0.5 * c.zz(i, i) : c.F[q]) / c.W;
+        if (dD_host) dD_host[q] = 0.25 * c.zz(i, j) / c.W;
       }
       for (int i = 0; i < N; ++i)
-        if (dh_host) dh_host[i] = c.sz(i) * inv;
+        if (dh_host) dh_host[i] = c.sz(i) / c.W;
       return ED_OK;
     }
     if (rc != ED_ENOMEM && rc != ED_ENOTSUP) return rc;

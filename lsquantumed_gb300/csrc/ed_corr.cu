@@ -670,7 +670,14 @@ __global__ void __launch_bounds__(256) k_corr_gram_sum(const long long* __restri
 // alternate marked rows (state, psi and rank halves by shuffle), four
 // gathers in flight each.  A row and pair that contribute nothing cost no FMA
 // and no gather.  TWO: sum over the same rows of (lam_r psi_r' + lam_r' psi_r)
-// / 2 with lam in pl.  partial[(pass ED_CORR_FEW + g) nblk + blk] (FP64).
+// / 2 with lam in pl.  A lane adds FL_FOLD chunks in a plain chain; the chains of
+// a lane, the lanes and the blocks are joined as pairs, so that few long chains
+// (16 pairs share the lanes) do not round more than the one row per thread and
+// term of the general kernels: 1.6-1.7 times their error at N=24 as plain chains,
+// 0.6-1.0 times so.  Two blocks per SM (three with two vectors, whose loads per
+// gather are two), all resident: the registers then hold the loads in flight.  16
+// bonds of a gradient at N=28 2.25 -> 2.22 ms, at N=16 93 -> 100 us; mixed
+// expectations of 96 bonds at N=24 1.23 -> 1.26 ms.  partial[(pass ED_CORR_FEW + g) nblk + blk]: pairs.
 struct FlipMasks {
   int n;
   uint32_t m[ED_CORR_FEW];   // (1 << i) | (1 << j)
@@ -680,13 +687,14 @@ struct FlipMasks {
 };
 
 constexpr int FL_U = 4;
+constexpr int FL_FOLD = 4;
 template <bool TWO>
-__global__ void __launch_bounds__(256, 3) k_expect_flip_r(const uint32_t* __restrict__ states,
+__global__ void __launch_bounds__(256, TWO ? 3 : 2) k_expect_flip_r(const uint32_t* __restrict__ states,
                                                        const double* __restrict__ pr, const double* __restrict__ pl,
                                                        int64_t dim, const uint16_t* __restrict__ t0,
                                                        const uint32_t* __restrict__ t1, int w0,
                                                        const FlipMasks* __restrict__ fm,
-                                                       double* __restrict__ partial, int nblk) {
+                                                       double2* __restrict__ partial, int nblk) {
   __shared__ FlipMasks pm;
   if (threadIdx.x < sizeof(FlipMasks) / 4) ((uint32_t*)&pm)[threadIdx.x] = ((const uint32_t*)(fm + blockIdx.y))[threadIdx.x];
   partial += (size_t)blockIdx.y * ED_CORR_FEW * nblk;
@@ -694,7 +702,7 @@ __global__ void __launch_bounds__(256, 3) k_expect_flip_r(const uint32_t* __rest
   for (int i = threadIdx.x; i < (1 << w0); i += blockDim.x) t0s[i] = t0[i];
   __syncthreads();
   const unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
   const int gl = lane >> 1, par = lane & 1;  // this lane's pair and its turn
   const bool gl_on = gl < pm.n;
   const uint32_t my_m = pm.m[gl], my_ml = pm.ml[gl], my_mh = pm.mh[gl];
@@ -704,7 +712,13 @@ __global__ void __launch_bounds__(256, 3) k_expect_flip_r(const uint32_t* __rest
     mm[g] = pm.m[g];
     mb[g] = g < pm.n ? pm.bi[g] : 0xFFFFFFFFu;  // past the list: never met
   }
-  double fl = 0.0;
+  // the chains before the current one, in shared memory: registers are what keeps
+  // loads in flight
+  __shared__ double2 shf[8 * 32];
+  shf[threadIdx.x] = make_double2(0.0, 0.0);
+  double fl = 0.0;  // the current chain
+  int chunk = 0;
+  bool folded = false;
   const uint32_t low = (1u << w0) - 1u;
   const int64_t step = (((int64_t)gridDim.x * blockDim.x) >> 5) * 32;
   int64_t base = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32;
@@ -770,25 +784,55 @@ __global__ void __launch_bounds__(256, 3) k_expect_flip_r(const uint32_t* __rest
       for (int u = 0; u < FL_U; ++u)
         if (has[u]) fl = TWO ? fma(yk[u], q[u], fma(xk[u], ql[u], fl)) : fma(xk[u], q[u], fl);
     }
+    if (++chunk == FL_FOLD) {
+      double2 p = shf[threadIdx.x];
+      ed_pair_add(p.x, p.y, fl, 0.0);
+      shf[threadIdx.x] = p;
+      fl = 0.0;
+      chunk = 0;
+      folded = true;
+    }
   }
-  __shared__ double shf[8 * 32];
-  shf[wid * 32 + lane] = fl;
+  {
+    double2 p = shf[threadIdx.x];
+    if (folded) ed_pair_add(p.x, p.y, fl, 0.0);
+    else p.x = fl;
+    shf[threadIdx.x] = p;
+  }
   __syncthreads();
-  if (threadIdx.x < ED_CORR_FEW) {
-    const int g = threadIdx.x;
-    double a = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) a += shf[w * 32 + 2 * g] + shf[w * 32 + 2 * g + 1];
-    partial[(size_t)g * nblk + blockIdx.x] = TWO ? 0.5 * a : a;
-  }
+  // one warp: a lane adds its place of the eight warps, then the pair's two lanes
+  // (64 FP64 instructions; 16 threads per pair in four steps are 256, which
+  // bounded 80 pairs of short vectors)
+  if (threadIdx.x >= 32) return;
+  double2 p = shf[lane];
+#pragma unroll
+  for (int w = 1; w < 8; ++w) ed_pair_add(p.x, p.y, shf[w * 32 + lane].x, shf[w * 32 + lane].y);
+  const double x = __shfl_xor_sync(FULL, p.x, 1), xl = __shfl_xor_sync(FULL, p.y, 1);
+  ed_pair_add(p.x, p.y, x, xl);
+  if (!par) partial[(size_t)gl * nblk + blockIdx.x] = TWO ? make_double2(0.5 * p.x, 0.5 * p.y) : p;
 }
 
-__global__ void __launch_bounds__(256) k_flip_sum(const double* __restrict__ partial, int nblk,
-                                                  double* __restrict__ out) {
-  double a[1] = {0.0};
-  for (int b = threadIdx.x; b < nblk; b += blockDim.x) a[0] += partial[(size_t)blockIdx.x * nblk + b];
-  __shared__ double sh[32];
-  ed_block_reduce<1>(a, sh);
-  if (threadIdx.x == 0) out[blockIdx.x] = a[0];
+// out[pair]: the sum rounded to FP64, and what that left
+__global__ void __launch_bounds__(128) k_flip_sum(const double2* __restrict__ partial, int nblk,
+                                                  double2* __restrict__ out) {
+  double h = 0.0, l = 0.0;
+  for (int b = threadIdx.x; b < nblk; b += blockDim.x) {
+    const double2 v = partial[(size_t)blockIdx.x * nblk + b];
+    ed_pair_add(h, l, v.x, v.y);
+  }
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) {
+    const double x = __shfl_down_sync(0xffffffffu, h, s), xl = __shfl_down_sync(0xffffffffu, l, s);
+    ed_pair_add(h, l, x, xl);
+  }
+  __shared__ double2 sh[4];
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = make_double2(h, l);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 4; ++w) ed_pair_add(h, l, sh[w].x, sh[w].y);
+    const double f = h + l;
+    out[blockIdx.x] = make_double2(f, l - (f - h));
+  }
 }
 
 typedef unsigned __int128 u128;
@@ -858,7 +902,8 @@ int ed_corr_real(const ed_basis* b, const double2* lam, const double2* psi, bool
   if (gram) npass = std::min<int64_t>(npass, 32);
   if (npass > 65535) return ED_ENOTSUP;  // grid.y
   const int nprep = (int)std::max<int64_t>(1, std::min<int64_t>((dim + 1023) / 1024, (int64_t)ctx->num_sms * 8));
-  const int nflip = (int)std::max<int64_t>(1, std::min<int64_t>((dim + 255) / 256, (int64_t)ctx->num_sms * 4));
+  // all blocks of a pass resident at once
+  const int nflip = (int)std::max<int64_t>(1, std::min<int64_t>((dim + 255) / 256, (int64_t)ctx->num_sms * (two ? 3 : 2)));
   // long segments where there is work for every SM (fewer table adds), short
   // ones below, where the chain of loads is what takes time (21 us at N=16
   // with 64)
@@ -880,12 +925,12 @@ int ed_corr_real(const ed_basis* b, const double2* lam, const double2* psi, bool
   const size_t o_zero = at;  // cleared up to here
   const size_t o_P = take(sizeof(ulonglong2) * (size_t)(npairs + 1));
   const size_t o_G = take(sizeof(ulonglong2) * 2048);
-  const size_t o_f = take(sizeof(double) * ED_CORR_FEW * (size_t)npass);
+  const size_t o_f = take(sizeof(double2) * ED_CORR_FEW * (size_t)npass);
   const size_t o_res = at;  // read back: header .. here
   const size_t o_part = take(sizeof(double) * 2 * (size_t)nprep);
   const size_t o_M = take((sizeof(ulonglong2) * (size_t)(w0 + 1)) << w1);
   const size_t o_fm = take(sizeof(FlipMasks) * (size_t)npass);
-  const size_t o_fp = take(sizeof(double) * (size_t)ED_CORR_FEW * (size_t)npass * nflip);
+  const size_t o_fp = take(sizeof(double2) * (size_t)ED_CORR_FEW * (size_t)npass * nflip);
   const size_t o_gp = take(gram ? sizeof(long long) * (size_t)GRAM_ACC * ncta : 0);
   const size_t o_pr = take(sizeof(double) * (size_t)dim);
   const size_t o_pl = take(two ? sizeof(double) * (size_t)dim : 0);
@@ -943,9 +988,9 @@ int ed_corr_real(const ed_basis* b, const double2* lam, const double2* psi, bool
     auto kern = two ? k_expect_flip_r<true> : k_expect_flip_r<false>;
     kern<<<dim3(nflip, (unsigned)np_), 256, smem, ctx->stream>>>(b->d_states, pr, pl, dim, b->d_lin_t0, b->d_lin_t1,
                                                                  w0, (const FlipMasks*)(base + o_fm),
-                                                                 (double*)(base + o_fp), nflip);
+                                                                 (double2*)(base + o_fp), nflip);
     ED_CHECK_LAUNCH(ctx);
-    k_flip_sum<<<(unsigned)count, 256, 0, ctx->stream>>>((const double*)(base + o_fp), nflip, (double*)(base + o_f));
+    k_flip_sum<<<(unsigned)count, 128, 0, ctx->stream>>>((const double2*)(base + o_fp), nflip, (double2*)(base + o_f));
     ED_CHECK_LAUNCH(ctx);
     return ED_OK;
   };
@@ -989,6 +1034,7 @@ int ed_corr_real(const ed_basis* b, const double2* lam, const double2* psi, bool
     out.P.resize(npairs);
     for (int q = 0; q < npairs; ++q) out.P[q] = get(o_P + 16 * (size_t)q);
     out.T = get(o_P + 16 * (size_t)npairs);
+    if (!two) out.W = i128_to_double(out.T) * out.inv_scale;  // exact, rounded once
   }
   out.F.assign(np, 0.0);
   out.Fl.assign(np, 0.0);
@@ -997,7 +1043,11 @@ int ed_corr_real(const ed_basis* b, const double2* lam, const double2* psi, bool
   for (size_t t = 0; t < flips.size(); ++t) {
     const int i = pairs[2 * flips[t]], j = pairs[2 * flips[t] + 1];
     if (few) {
-      memcpy(&out.F[flips[t]], res.data() + o_f + sizeof(double) * t, sizeof(double));
+      double2 f;
+      memcpy(&f, res.data() + o_f + sizeof(f) * t, sizeof(f));
+      out.F[flips[t]] = f.x;
+      out.Fl[flips[t]] = f.y;
+      if (!std::isfinite(f.x)) return ED_ENOTSUP;  // a pair makes NaN of an infinity: the general kernels answer
     } else if (nstages > 0) {
       // F 2^(2 (62 - E) - 32), E = emax - 1022
       const u128 x = get(o_G + 16 * (size_t)(i * 32 + j)) + get(o_G + 16 * (size_t)(1024 + i * 32 + j)) +
@@ -1017,12 +1067,12 @@ int ed_corr_real(const ed_basis* b, const double2* lam, const double2* psi, bool
   for (size_t t0 = 0; t0 < list.size(); t0 += most) {
     const size_t cnt = std::min(most, list.size() - t0);
     ED_TRY(direct(list.data() + t0, cnt));
-    std::vector<double> f(cnt);
-    ED_CUDA(cudaMemcpyAsync(f.data(), base + o_f, sizeof(double) * cnt, cudaMemcpyDeviceToHost, ctx->stream));
+    std::vector<double2> f(cnt);
+    ED_CUDA(cudaMemcpyAsync(f.data(), base + o_f, sizeof(double2) * cnt, cudaMemcpyDeviceToHost, ctx->stream));
     ED_CUDA(cudaStreamSynchronize(ctx->stream));
     for (size_t t = 0; t < cnt; ++t) {
-      out.F[flips[list[t0 + t]]] = f[t];
-      out.Fl[flips[list[t0 + t]]] = 0.0;
+      out.F[flips[list[t0 + t]]] = f[t].x;
+      out.Fl[flips[list[t0 + t]]] = f[t].y;
     }
   }
   return ED_OK;

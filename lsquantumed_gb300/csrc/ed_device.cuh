@@ -155,6 +155,14 @@ __device__ __forceinline__ void ed_block_max(double& v, double* sh) {
   }
 }
 
+// (h, l) + (x, xl) as an unevaluated pair (Knuth's TwoSum), for the few large
+// partial sums whose rounding would decide that of the result.
+__device__ __forceinline__ void ed_pair_add(double& h, double& l, double x, double xl) {
+  const double t = __dadd_rn(h, x), z = __dsub_rn(t, h);
+  l = __dadd_rn(l, __dadd_rn(__dadd_rn(__dsub_rn(h, __dsub_rn(t, z)), __dsub_rn(x, z)), xl));
+  h = t;
+}
+
 // The last block of the grid to get here; all threads of every block call it
 // after their block's result is written.  The counter is zero before and after
 // the launch.

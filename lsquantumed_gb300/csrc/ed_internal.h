@@ -154,7 +154,7 @@ struct ed_corr {
   unsigned __int128 T = 0;               // sum w
   std::vector<unsigned __int128> P;      // [a (a + 1) / 2 + b], b <= a: sum w over the states with a and b up
   std::vector<double> F;                 // flip sum per pair of the call (0 for i == j)
-  std::vector<double> Fl;                // what the rounding of F left (0 where F was summed in FP64)
+  std::vector<double> Fl;                // what the rounding of F left
   double zz(int i, int j) const;         // sum w sigma_i sigma_j
   double sisj(int i, int j, int64_t q) const;  // zz(i, j) / 4 + F[q], i != j, rounded once
   double up(int i) const;                // sum w over the states with i up

@@ -298,14 +298,6 @@ static int dsf_k(const ed_basis* b0, const ed_basis* b1, int op, const double2* 
 #define DZ_EMIN (DZ_BITS + DZ_MORE)
 #define DZ_ROWS 16  // rows per plain FP64 chain
 
-// (h, l) + x as an unevaluated pair (Knuth's TwoSum): the signed sums cancel,
-// so the few large partial sums here decide the rounding of the result
-__device__ __forceinline__ void dsf_add(double& h, double& l, double x, double xl) {
-  const double t = __dadd_rn(h, x), z = __dsub_rn(t, h);
-  l = __dadd_rn(l, __dadd_rn(__dadd_rn(__dsub_rn(h, __dsub_rn(t, z)), __dsub_rn(x, z)), xl));
-  h = t;
-}
-
 // 2^(em - 1022 - DZ_BITS), the last place of fixed point against em, for em >=
 // DZ_EMIN; and the factor to units of 2^-DZ_MORE of it
 __device__ __forceinline__ double dsf_unit(int em) { return __longlong_as_double((long long)(em + 1 - DZ_BITS) << 52); }
@@ -314,7 +306,7 @@ __device__ __forceinline__ double dsf_more(int em) {
 }
 
 // The warp's sum of pairs, in every lane: as integers (54 + 20 bits against the
-// largest), 12 FP64 operations where five steps of dsf_add are 40.
+// largest), 12 FP64 operations where five steps of ed_pair_add are 40.
 __device__ __forceinline__ void dsf_warp(double& h, double& l) {
   const int em = (int)__reduce_max_sync(
       0xffffffffu, (unsigned)(((unsigned long long)__double_as_longlong(h) >> 52) & 0x7FF));
@@ -322,7 +314,7 @@ __device__ __forceinline__ void dsf_warp(double& h, double& l) {
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) {
       const double x = __shfl_xor_sync(0xffffffffu, h, s), xl = __shfl_xor_sync(0xffffffffu, l, s);
-      dsf_add(h, l, x, xl);
+      ed_pair_add(h, l, x, xl);
     }
     return;
   }
@@ -397,7 +389,7 @@ __global__ void __launch_bounds__(128, REAL ? 5 : 3) k_dsfz_high(const double2* 
 #pragma unroll
         for (int c = 0; c < C; ++c) {
           if (o0 == lane) sh_[c][v] = a[c][v];  // the first chain
-          else dsf_add(sh_[c][v], sl_[c][v], a[c][v], 0.0);
+          else ed_pair_add(sh_[c][v], sl_[c][v], a[c][v], 0.0);
         }
     }
     if (REAL && __any_sync(0xffffffffu, im)) {
@@ -411,7 +403,7 @@ __global__ void __launch_bounds__(128, REAL ? 5 : 3) k_dsfz_high(const double2* 
       for (int c = 0; c < C; ++c) {
         double h = sh_[c][v], l = sl_[c][v];
         dsf_warp(h, l);
-        dsf_add(hh[c][v], hl[c][v], up ? h : -h, up ? l : -l);
+        ed_pair_add(hh[c][v], hl[c][v], up ? h : -h, up ? l : -l);
       }
   }
   __shared__ double2 sh[C][DZ_V][4][32];
@@ -425,7 +417,7 @@ __global__ void __launch_bounds__(128, REAL ? 5 : 3) k_dsfz_high(const double2* 
     for (int c = 0; c < 2; ++c) {
       double2 t = make_double2(0.0, 0.0);
       if (c < C)
-        for (int w = 0; w < 4; ++w) dsf_add(t.x, t.y, sh[c][v][w][lane].x, sh[c][v][w][lane].y);
+        for (int w = 0; w < 4; ++w) ed_pair_add(t.x, t.y, sh[c][v][w][lane].x, sh[c][v][w][lane].y);
       d[c] = t;
     }
   }
@@ -472,8 +464,8 @@ __global__ void __launch_bounds__(256) k_dsfz_low(const double2* __restrict__ ps
           sr[v] = ar[v];
           si[v] = ai[v];
         } else {
-          dsf_add(sr[v], lr[v], ar[v], 0.0);
-          if (!REAL) dsf_add(si[v], li[v], ai[v], 0.0);
+          ed_pair_add(sr[v], lr[v], ar[v], 0.0);
+          if (!REAL) ed_pair_add(si[v], li[v], ai[v], 0.0);
         }
         ar[v] = ai[v] = 0.0;
       }
@@ -501,9 +493,9 @@ __global__ void __launch_bounds__(256) k_dsfz_low(const double2* __restrict__ ps
     for (int v = 0; v < DZ_V; ++v) {
       // |rest| <= half the last bit of the sum
       ar[v] = sr[v];
-      dsf_add(ar[v], rr[v], lr[v], 0.0);
+      ed_pair_add(ar[v], rr[v], lr[v], 0.0);
       ai[v] = si[v];
-      dsf_add(ai[v], ri[v], li[v], 0.0);
+      ed_pair_add(ai[v], ri[v], li[v], 0.0);
     }
   }
   // The signed sums cancel: exact, as 54-bit integers against the block's
@@ -590,8 +582,8 @@ __global__ void __launch_bounds__(128) k_dsf_sum(const double* __restrict__ pl, 
 #pragma unroll 4
   for (int b = threadIdx.x; b < cnt; b += 128) {
     const double2 re = p[(size_t)b * ld], im = p[(size_t)b * ld + 1];
-    dsf_add(h[0], l[0], re.x, re.y);
-    dsf_add(h[1], l[1], im.x, im.y);
+    ed_pair_add(h[0], l[0], re.x, re.y);
+    ed_pair_add(h[1], l[1], im.x, im.y);
   }
   __shared__ double sh[4][4];
 #pragma unroll
@@ -599,7 +591,7 @@ __global__ void __launch_bounds__(128) k_dsf_sum(const double* __restrict__ pl, 
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) {
       const double x = __shfl_down_sync(0xffffffffu, h[k], s), xl = __shfl_down_sync(0xffffffffu, l[k], s);
-      dsf_add(h[k], l[k], x, xl);
+      ed_pair_add(h[k], l[k], x, xl);
     }
     if ((threadIdx.x & 31) == 0) {
       sh[threadIdx.x >> 5][2 * k] = h[k];
@@ -609,8 +601,8 @@ __global__ void __launch_bounds__(128) k_dsf_sum(const double* __restrict__ pl, 
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int w = 1; w < 4; ++w) {
-      dsf_add(h[0], l[0], sh[w][0], sh[w][1]);
-      dsf_add(h[1], l[1], sh[w][2], sh[w][3]);
+      ed_pair_add(h[0], l[0], sh[w][0], sh[w][1]);
+      ed_pair_add(h[1], l[1], sh[w][2], sh[w][3]);
     }
     c[(size_t)n * gridDim.x + i] = make_double2(f * (h[0] + l[0]), f * (h[1] + l[1]));
   }
