@@ -23,10 +23,11 @@
 // N rows, and N gathers of half-empty columns per t serve all N^2 / 2 pairs.
 // As FP64 FMAs it would be bound by the FP64 unit (7.4 ms at N=28), so it
 // runs on the tensor cores in exact 8-bit digits (k_corr_gram): 2.5 ms at
-// N=28 (seven digits; now eight, 3% of the call more) instead of 31.6 ms for 26
-// passes of 16 pairs before.  Small flip sums are formed again in FP64, so a
-// list's length does not change their accuracy.  All S.S of the N=28 state:
-// 47.5 -> 3.04 ms; the energy gradient over 96 bonds at N=24: 10.9 -> 0.30 ms.
+// N=28 (seven digits; now eight and a second product, 10% of the call more)
+// instead of 31.6 ms for 26 passes of 16 pairs before.  Small flip sums are formed
+// again in FP64, so a list's length does not change their accuracy.  All S.S of
+// the N=28 state: 47.5 -> 3.23 ms; the energy gradient over 96 bonds at N=24: 10.9
+// -> 0.35 ms.
 #include "ed_internal.h"
 #include "ed_device.cuh"
 #include "ed_halves.cuh"
@@ -210,7 +211,9 @@ __global__ void __launch_bounds__(256) k_corr_cols(const double* __restrict__ pr
 
 // round(v 2^(62 - E)) for |v| < 2^E, E = emax - 1022, plus 128 in each byte:
 // byte i is then digit i + 128 of the balanced base-256 representation, digits
-// in [-128, 127] (|q| <= 2^62).
+// in [-128, 127] (|q| <= 2^62).  Halves round to even: half of the entries ten
+// binades below the largest are halves, and rounding them up added to the sums of
+// a state of one sign.
 constexpr unsigned long long GRAM_ZERO = 0x8080808080808080ull;
 __device__ __forceinline__ unsigned long long gram_entry(double v, int emax) {
   const long long b = __double_as_longlong(v);
@@ -220,7 +223,7 @@ __device__ __forceinline__ unsigned long long gram_entry(double v, int emax) {
   const int sh = e - emax + 9;  // <= 9
   unsigned long long q;
   if (sh >= 0) q = mant << sh;
-  else if (sh > -60) q = (mant + (1ull << (-sh - 1))) >> (-sh);
+  else if (sh > -60) q = (mant + (1ull << (-sh - 1)) - 1ull + ((mant >> -sh) & 1ull)) >> (-sh);
   else q = 0ull;
   return b < 0 ? GRAM_ZERO - q : GRAM_ZERO + q;
 }
@@ -336,11 +339,19 @@ __global__ void __launch_bounds__(256) k_corr_moments(const unsigned long long* 
 // point against the largest entry of the state, as eight balanced 8-bit digits,
 // which FP16 holds exactly.  One tcgen05.mma has M = 128 rows (digits 0..3 x 32
 // sites), N = 256 columns (digits 0..7 x 32 sites) and K = 16 states; the digits
-// are symmetric in the two factors, so every product of digits i + j <= 7 (and
-// more) is among them or the transpose of one.  A digit product sum stays an
-// exact integer in the FP32 accumulator over GRAM_GROUP stages (1024 states x
-// 128^2 = 2^24), then four epilogue warps add it to 64-bit integers in shared
-// memory.
+// are symmetric in the two factors, so every product with a digit of 0..3 is
+// among them or the transpose of one.  Of the products of digits 4..7 alone a
+// second MMA (M = digits 4..7, N = digit 4) brings those that matter: (4, 4) is
+// 2^-62 of the squared scale per state with a random sign, and without it the
+// flip sums of a state of a few decades at N=24 had 5 times the error of FP64
+// chains (6.5e-18 where the last rounding is 5.2e-19, as it is now); what is left,
+// (5, 5) and below, is 2^-78.  It takes 6% of the kernel, the one set of
+// accumulators 12%; two sets, with the first MMA split in halves, were slower (3.69
+// against 3.23 ms for all pairs at N=28).  A digit product sum stays an exact
+// integer in the FP32 accumulator over GRAM_GROUP stages (1024 states x 128^2 =
+// 2^24), then four epilogue warps add it to 64-bit integers in shared memory.  The
+// accumulators fill more than half of the TMEM, so there is one set; the producers,
+// which bound the kernel, go on for two stages while it is read.
 //
 // The rounded entries leave a root mean square error of at most 2^-62 / sqrt(12)
 // of 2^E times the norm: that of the last rounding of F for |F| >= 2^-9 2^E norm.
@@ -366,11 +377,13 @@ constexpr int GRAM_LBO = GRAM_ROWS * 16 + 16;                  // + 16: the 16-b
 constexpr int GRAM_STAGE = (GRAM_STATES / 8) * GRAM_LBO;       // 65792 bytes
 constexpr int GRAM_GROUP = 8;                                  // stages per accumulation: 2^24 bound
 constexpr int GRAM_PROD = 16, GRAM_THREADS = (GRAM_PROD + 5) * 32;
-constexpr int GRAM_ACC = 128 * CR_SITES * 2;                   // 64-bit sums per CTA
+constexpr int GRAM_PLANE = 3;                                  // columns 0..3, 4..7, and digit 4 x digits 4..7
+constexpr int GRAM_ACC = 128 * CR_SITES * GRAM_PLANE;          // 64-bit sums per CTA
+constexpr int GRAM_LOW = GRAM_N;                               // TMEM column of the second MMA's sums
 constexpr size_t GRAM_SMEM = 2 * (size_t)GRAM_STAGE + (size_t)GRAM_ACC * 8;
 
 struct GramShared {
-  uint64_t full[2], empty[2], tfull[2], tempty[2], done;
+  uint64_t full[2], empty[2], tfull, tempty, done;
   uint32_t tmem;
 };
 
@@ -403,6 +416,25 @@ struct GramAt {
   }
 };
 
+__device__ __forceinline__ void gram_ld8(uint32_t taddr, uint32_t (&d)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7])
+               : "r"(taddr));
+}
+
+// orders the uses of loaded registers after the wait before it
+__device__ __forceinline__ void gram_loaded(uint32_t (&d)[8]) {
+#pragma unroll
+  for (int c = 0; c < 8; ++c) asm volatile("" : "+r"(d[c]));
+}
+
+__device__ __forceinline__ void gram_mma(uint32_t dcol, uint64_t a, uint64_t b, uint32_t idesc, uint32_t keep) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(dcol),
+      "l"(a), "l"(b), "r"(idesc), "r"(keep));
+}
+
 __global__ void __launch_bounds__(GRAM_THREADS, 1) k_corr_gram(const unsigned long long* __restrict__ q,
                                                                const __grid_constant__ CorrGeom g, int nstages,
                                                                const uint16_t* __restrict__ t0,
@@ -413,7 +445,7 @@ __global__ void __launch_bounds__(GRAM_THREADS, 1) k_corr_gram(const unsigned lo
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ GramShared S;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  long long* acc = (long long*)(smem + 2 * GRAM_STAGE);  // [site b][2][TMEM lane]
+  long long* acc = (long long*)(smem + 2 * GRAM_STAGE);  // [site b][plane][TMEM lane]
   for (int i = tid; i < GRAM_ACC; i += GRAM_THREADS) acc[i] = 0ll;
   if (warp == GRAM_PROD + 4) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&S.tmem)),
@@ -424,9 +456,9 @@ __global__ void __launch_bounds__(GRAM_THREADS, 1) k_corr_gram(const unsigned lo
     for (int i = 0; i < 2; ++i) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&S.full[i])), "r"(GRAM_PROD));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&S.empty[i])));
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&S.tfull[i])));
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(smem_u32(&S.tempty[i])));
     }
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&S.tfull)));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(smem_u32(&S.tempty)));
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&S.done)));
     asm volatile("fence.mbarrier_init.release.cluster;");
   }
@@ -555,71 +587,68 @@ __global__ void __launch_bounds__(GRAM_THREADS, 1) k_corr_gram(const unsigned lo
     const int sub = warp - GRAM_PROD;
     const int ngroups = (s1 - s0 + GRAM_GROUP - 1) / GRAM_GROUP;
     for (int gq = 0; gq < ngroups; ++gq) {
-      const int ac = gq & 1;
-      if (!mbar_wait(smem_u32(&S.tfull[ac]), (gq >> 1) & 1, TC_WAIT_POLLS)) {
+      if (!mbar_wait(smem_u32(&S.tfull), gq & 1, TC_WAIT_POLLS)) {
         atomicExch(err, 1);
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;");
-      const uint32_t taddr = tmem + ((uint32_t)(sub * 32) << 16) + (uint32_t)(ac * 256);
+      const uint32_t taddr = tmem + ((uint32_t)(sub * 32) << 16);
 #pragma unroll 1
       for (int b0 = 0; b0 < CR_SITES; b0 += 8) {
-        long long H[8], L[8];
+        long long* ab = acc + (size_t)(b0 * GRAM_PLANE) * 128 + sub * 32 + lane;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) H[c] = L[c] = 0ll;
+        for (int pl = 0; pl < 2; ++pl) {  // digits 0..3, 4..7 of the second factor
+          uint32_t d[4][8];
 #pragma unroll
-        for (int j = 0; j < GRAM_DIG; ++j) {
-          uint32_t d[8];
-          asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-              : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7])
-              : "r"(taddr + (uint32_t)(j * CR_SITES + b0)));
+          for (int j = 0; j < 4; ++j) gram_ld8(taddr + (uint32_t)((4 * pl + j) * CR_SITES + b0), d[j]);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
+          for (int j = 0; j < 4; ++j) gram_loaded(d[j]);
+#pragma unroll
           for (int c = 0; c < 8; ++c) {
-            const long long x = (long long)__float2int_rz(__uint_as_float(d[c]));
-            if (j < GRAM_DIG / 2) H[c] = H[c] * 256 + x;
-            else L[c] = L[c] * 256 + x;
+            long long t = 0ll;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) t = t * 256 + (long long)__float2int_rz(__uint_as_float(d[j][c]));
+            ab[(c * GRAM_PLANE + pl) * 128] += t;
           }
         }
+        uint32_t d[8];  // digit 4 + sub of the first factor x digit 4
+        gram_ld8(taddr + (uint32_t)(GRAM_LOW + b0), d);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        gram_loaded(d);
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          long long* a = acc + (size_t)((b0 + c) * 2) * 128 + sub * 32 + lane;
-          a[0] += H[c];
-          a[128] += L[c];
-        }
+        for (int c = 0; c < 8; ++c)
+          ab[(c * GRAM_PLANE + 2) * 128] += (long long)__float2int_rz(__uint_as_float(d[c]));
       }
       asm volatile("tcgen05.fence::before_thread_sync;");
       __syncwarp();
-      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&S.tempty[ac])) : "memory");
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&S.tempty)) : "memory");
     }
   } else if (lane == 0) {
-    const uint32_t idesc = umma_idesc_f16(128, GRAM_N);
+    const uint32_t idesc = umma_idesc_f16(128, GRAM_N), idesc_low = umma_idesc_f16(128, CR_SITES);
     const uint32_t base = smem_u32(smem);
     for (int s = s0; s < s1; ++s) {
-      const int it = s - s0, st = it & 1, gq = it / GRAM_GROUP, ac = gq & 1, in = it % GRAM_GROUP;
+      const int it = s - s0, st = it & 1, gq = it / GRAM_GROUP, in = it % GRAM_GROUP;
       if (!mbar_wait(smem_u32(&S.full[st]), (it >> 1) & 1, TC_WAIT_POLLS) ||
-          (in == 0 && !mbar_wait(smem_u32(&S.tempty[ac]), ((gq >> 1) & 1) ^ 1, TC_WAIT_POLLS))) {
+          (in == 0 && !mbar_wait(smem_u32(&S.tempty), (gq & 1) ^ 1, TC_WAIT_POLLS))) {
         atomicExch(err, 1);
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;");
+      // rows 0 .. 127 of a stage are digits 0..3, rows 128 .. 255 digits 4..7
+      auto rows = [&](int ks, int r) { return umma_desc(base + st * GRAM_STAGE + ks * 2 * GRAM_LBO + r * 16, GRAM_LBO, 128); };
 #pragma unroll
       for (int ks = 0; ks < GRAM_STATES / 16; ++ks) {
-        // the first factor is the first 128 rows (digits 0..3) of the second
-        const uint64_t desc = umma_desc(base + st * GRAM_STAGE + ks * 2 * GRAM_LBO, GRAM_LBO, 128);
         const uint32_t keep = in > 0 || ks > 0 ? 1u : 0u;
-        asm volatile(
-            "{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n"
-            " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem + (uint32_t)(ac * 256)),
-            "l"(desc), "l"(desc), "r"(idesc), "r"(keep));
+        gram_mma(tmem, rows(ks, 0), rows(ks, 0), idesc, keep);
+        gram_mma(tmem + (uint32_t)GRAM_LOW, rows(ks, 128), rows(ks, 128), idesc_low, keep);
       }
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                        smem_u32(&S.empty[st]))
                    : "memory");
       if (in == GRAM_GROUP - 1 || s + 1 == s1)
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                         smem_u32(&S.tfull[ac]))
+                         smem_u32(&S.tfull))
                      : "memory");
     }
     // every MMA issued has completed before the TMEM is freed
@@ -636,30 +665,39 @@ __global__ void __launch_bounds__(GRAM_THREADS, 1) k_corr_gram(const unsigned lo
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
 }
 
-// Sums over the CTAs and the four digits i, as 128-bit integers in units of
-// 2^32 q-units: out[b][a] = digit pairs (i, j <= 3), out[32 * 32 + b][a] =
-// (i, j = 4..7).  Block = site b, thread = TMEM lane (i, a).
-__global__ void __launch_bounds__(256) k_corr_gram_sum(const long long* __restrict__ part, int ncta,
-                                                       ulonglong2* __restrict__ out) {
-  const int b = blockIdx.x, half = threadIdx.x >> 7, ln = threadIdx.x & 127, i = ln >> 5;
-  const long long* p = part + (size_t)(b * 2 + half) * 128 + ln;
+// Sums over the CTAs and the digits i, as 128-bit integers in units of 2^32
+// q-units: out[b][a] = digit pairs (i, j <= 3), out[1024 + 32 b + a] = (i, j = 4..7),
+// out[2048 + ..] = (4, 4), out[3072 + ..] = (5, 4) and (6, 4) ((7, 4) lies below the
+// unit).  Block = site b, thread = plane and TMEM lane (i, a).
+__global__ void __launch_bounds__(128 * GRAM_PLANE) k_corr_gram_sum(const long long* __restrict__ part, int ncta,
+                                                                    ulonglong2* __restrict__ out) {
+  const int b = blockIdx.x, plane = threadIdx.x >> 7, ln = threadIdx.x & 127, i = ln >> 5;
+  const long long* p = part + (size_t)(b * GRAM_PLANE + plane) * 128 + ln;
   unsigned long long lo = 0ull, hi = 0ull;
   for (int c = 0; c < ncta; ++c) {
     const long long x = p[(size_t)c * GRAM_ACC];
     add128(lo, hi, (unsigned long long)x, (unsigned long long)(x >> 63));
   }
-  const int sh = (half ? 24 : 56) - 8 * i;  // 0 .. 56
-  if (sh) {
+  const int sh = (plane == 0 ? 56 : plane == 1 ? 24 : 16) - 8 * i;  // 0 .. 56, below 0: (7, 4)
+  if (sh > 0) {
     hi = (hi << sh) | (lo >> (64 - sh));
     lo <<= sh;
   }
-  __shared__ unsigned long long sl[256], sh_[256];
+  __shared__ unsigned long long sl[128 * GRAM_PLANE], sh_[128 * GRAM_PLANE];
   sl[threadIdx.x] = lo;
   sh_[threadIdx.x] = hi;
   __syncthreads();
-  if (ln < 32) {
+  if (ln >= 32) return;
+  ulonglong2* o = out + (size_t)plane * 1024 + b * 32 + ln;
+  if (plane < 2) {
     for (int w = 1; w < 4; ++w) add128(lo, hi, sl[threadIdx.x + 32 * w], sh_[threadIdx.x + 32 * w]);
-    out[(size_t)half * 1024 + b * 32 + ln] = make_ulonglong2(lo, hi);
+    *o = make_ulonglong2(lo, hi);
+  } else {
+    *o = make_ulonglong2(lo, hi);
+    lo = sl[threadIdx.x + 32];
+    hi = sh_[threadIdx.x + 32];
+    add128(lo, hi, sl[threadIdx.x + 64], sh_[threadIdx.x + 64]);
+    o[1024] = make_ulonglong2(lo, hi);
   }
 }
 
@@ -892,7 +930,7 @@ int ed_corr_real(const ed_basis* b, const double2* lam, const double2* psi, bool
   for (int64_t p = 0; p < np; ++p)
     if (pairs[2 * p] != pairs[2 * p + 1]) flips.push_back(p);
   // up to 16 pairs are one pass of the direct kernel (1.2 ms at N=28, 0.08 ms
-  // at N=24); the Gram kernel serves all pairs for 2.5 and 0.2 ms, so it takes
+  // at N=24); the Gram kernel serves all pairs for 2.8 and 0.2 ms, so it takes
   // every longer list.  Two vectors take direct passes.
   const bool gram = !two && (int64_t)flips.size() > ED_CORR_FEW;
   const bool few = !gram && !flips.empty();
@@ -924,7 +962,7 @@ int ed_corr_real(const ed_basis* b, const double2* lam, const double2* psi, bool
   const size_t o_W0 = take(want_zz ? sizeof(unsigned long long) * 4 << w0 : 0);
   const size_t o_zero = at;  // cleared up to here
   const size_t o_P = take(sizeof(ulonglong2) * (size_t)(npairs + 1));
-  const size_t o_G = take(sizeof(ulonglong2) * 2048);
+  const size_t o_G = take(sizeof(ulonglong2) * 4096);
   const size_t o_f = take(sizeof(double2) * ED_CORR_FEW * (size_t)npass);
   const size_t o_res = at;  // read back: header .. here
   const size_t o_part = take(sizeof(double) * 2 * (size_t)nprep);
@@ -1016,7 +1054,7 @@ int ed_corr_real(const ed_basis* b, const double2* lam, const double2* psi, bool
                                                                b->d_lin_t1, b->d_lin_lows, b->d_lin_highs,
                                                                (long long*)(base + o_gp), &hdr->err);
     ED_CHECK_LAUNCH(ctx);
-    k_corr_gram_sum<<<CR_SITES, 256, 0, ctx->stream>>>((const long long*)(base + o_gp), ncta,
+    k_corr_gram_sum<<<CR_SITES, 128 * GRAM_PLANE, 0, ctx->stream>>>((const long long*)(base + o_gp), ncta,
                                                        (ulonglong2*)(base + o_G));
     ED_CHECK_LAUNCH(ctx);
   }
@@ -1050,8 +1088,9 @@ int ed_corr_real(const ed_basis* b, const double2* lam, const double2* psi, bool
       if (!std::isfinite(f.x)) return ED_ENOTSUP;  // a pair makes NaN of an infinity: the general kernels answer
     } else if (nstages > 0) {
       // F 2^(2 (62 - E) - 32), E = emax - 1022
-      const u128 x = get(o_G + 16 * (size_t)(i * 32 + j)) + get(o_G + 16 * (size_t)(1024 + i * 32 + j)) +
-                     get(o_G + 16 * (size_t)(1024 + j * 32 + i));
+      const size_t ij = i * 32 + j, ji = j * 32 + i;
+      const u128 x = get(o_G + 16 * ij) + get(o_G + 16 * (1024 + ij)) + get(o_G + 16 * (1024 + ji)) +
+                     get(o_G + 16 * (2048 + ij)) + get(o_G + 16 * (3072 + ij)) + get(o_G + 16 * (3072 + ji));
       const int sh = 2 * (hh.emax - 1022) - 124 + 32;
       double rest;
       out.F[flips[t]] = std::ldexp(i128_split(x, rest), sh);

@@ -1,7 +1,8 @@
-"""Rounding of flip sums (mixed expectations of two real vectors, gradients over
-few bonds) on long vectors: no more than that of FP64 multiply-add chains over
-the rows of two blocks of 256 threads per SM, joined in a tree.  Root mean square
-over 144 sums each, whose ratio has a spread of 8%: two of those are allowed."""
+"""Rounding of flip sums on long vectors (mixed expectations of two real vectors and
+gradients over few bonds; lists of more than 16 pairs, also of vectors of a few
+decades): no more than that of FP64 multiply-add chains over the rows of two blocks
+of 256 threads per SM, joined in a tree.  Root mean square over 144 sums or more
+each, whose ratio has a spread of 8%: two of those are allowed."""
 import numpy as np
 import pytest
 
@@ -36,7 +37,7 @@ def _tree(h, l):
     return h[..., 0], l[..., 0]
 
 
-@pytest.mark.parametrize('what', ['mixed', 'gradient'])
+@pytest.mark.parametrize('what', ['mixed', 'gradient', 'pairs', 'pairs of a few decades'])
 def test_flip_rounding(what):
     import torch
     from lsquantumed_gb300.build import build
@@ -49,7 +50,8 @@ def test_flip_rounding(what):
     s = torch.from_numpy(b.int_basis.astype(np.int64)).cuda()
     threads = torch.cuda.get_device_properties(0).multi_processor_count * 2 * 256
     rng = np.random.default_rng(3)
-    bonds = [tuple(int(k) for k in rng.choice(N, 2, replace=False)) for _ in range(12)]
+    count = 17 if what.startswith('pairs') else 12
+    bonds = [tuple(int(k) for k in rng.choice(N, 2, replace=False)) for _ in range(count)]
     rows = []
     for i, j in bonds:
         to = torch.arange(b.size, device='cuda')
@@ -61,12 +63,18 @@ def test_flip_rounding(what):
     for seed in range(12):
         g = torch.Generator(device='cuda').manual_seed(seed)
         psi = torch.randn(b.size, dtype=torch.float64, device='cuda', generator=g)
+        if what.endswith('decades'):
+            psi = (1.0 + psi) * torch.exp(1.5 * torch.randn(b.size, dtype=torch.float64, device='cuda', generator=g))
         psi /= psi.norm()
-        lam = torch.randn(b.size, dtype=torch.float64, device='cuda', generator=g) if what == 'mixed' else psi
-        lam = lam / lam.norm()
+        lam = psi
+        if what == 'mixed':
+            lam = torch.randn(b.size, dtype=torch.float64, device='cuda', generator=g)
+            lam /= lam.norm()
         cpsi, clam = torch.complex(psi, torch.zeros_like(psi)), torch.complex(lam, torch.zeros_like(lam))
         if what == 'mixed':
             xy = A.expect_mixed(b, [(A.XY, i, j) for i, j in bonds], clam, cpsi)
+        elif what.startswith('pairs'):
+            xy = ed.SpSm(env, b).ExpectValPairs(bonds, cpsi)
         else:  # a ratio: times the norm again, 2 roundings of a sum of 1e-3
             h, l = _tree(*_two_prod(psi, psi))
             xy = A.energy_gradient(b, bonds, cpsi)[0] * float(h)
