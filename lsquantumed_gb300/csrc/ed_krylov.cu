@@ -125,16 +125,16 @@ __device__ __forceinline__ double block_sum256(double v, double* sh) {
 // Rounding of the dots.  Half as many threads with more registers each would mean
 // chains twice as long, so a thread adds its rows in two: with one, and two blocks
 // per SM, the root mean square error of 16 dots of 10M rows was 1.32 times that of
-// four blocks per SM.  One more add per column and thread, so only from KR_CHAIN
-// rows on (2.7M rows, 16 columns: 116 -> 123 us); below, the sums over threads and
-// blocks round more, and those are pairwise and in four chains.  Errors of 16 dots
-// in units of 1e-16 / sqrt(n), one chain and sequential sums -> now (four blocks
+// four blocks per SM.  One more FP64 add per column and thread, so only from 32 rows
+// on (2.7M rows, 16 columns: 116 -> 123 us), 16 for up to eight columns, which
+// memory bounds; four chains cost a solve at N=24 1.3% more.  Below, the sums over
+// threads and blocks round more, and those are pairwise and in four chains.  Errors
+// of 16 dots in units of 1e-16 / sqrt(n), one chain and sequential sums -> now (four blocks
 // per SM): 13k rows 2.14 -> 1.95 (1.97), 185k 2.71 -> 2.22 (2.21), 705k 2.85 -> 2.27
 // (2.23), 2.7M 3.11 -> 2.46 (2.49), 10.4M 5.14 -> 3.61 (3.77).  Steps of the first
 // chain, of all steps of rows each:
-constexpr int KR_CHAIN = 32;
-__device__ __forceinline__ int64_t kr_chain(int64_t steps, int rows) {
-  return steps * rows < KR_CHAIN ? steps : (steps + 1) / 2;
+__device__ __forceinline__ int64_t kr_chain(int64_t steps, int rows, int cols) {
+  return steps * rows < (cols > 8 ? 32 : 16) ? steps : (steps + 1) / 2;
 }
 
 // Blocks per SM of k_kr_dots: registers for the loads of a row in flight.
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(KR_THREADS, kr_dots_per_sm(NG)) k_kr_dots(cons
   __shared__ double sh[NG * (KR_THREADS + 1)];
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t half = r + kr_chain((n + U * stride - 1) / (U * stride), U) * (U * stride);
+  const int64_t half = r + kr_chain((n + U * stride - 1) / (U * stride), U, NG) * (U * stride);
   bool two = false;  // the first chain's sums are in this thread's places of sh
   for (; r + (U - 1) * stride < n; r += U * stride) {
     if (r == half) {
@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(KR_THREADS, NV > 8 ? 3 : 4) k_kr_update(const 
   if (NV > 0) {
     constexpr int U = NV <= 3 ? 4 : NV <= 8 ? 2 : 1;  // rows in flight per thread
     int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t half = r + kr_chain((n + U * stride - 1) / (U * stride), U) * (U * stride);
+    const int64_t half = r + kr_chain((n + U * stride - 1) / (U * stride), U, NV) * (U * stride);
     double before = 0.0;  // the first chain
     for (; r < n; r += U * stride) {
       if (r == half) {
