@@ -42,9 +42,10 @@ def test_small_flip_sums(N, mag, per_flip):
         size.append(np.abs(p).sum())
     ref, size = np.array(ref), np.array(size)
     op = ed.SpSm(env, b)
-    for n in (16, 17, len(pairs)):
-        got = op.ExpectValPairs(pairs[:n], psi).real
-        assert (np.abs(got - ref[:n]) <= 64 * 2.0 ** -53 * size[:n]).all(), \
-            (n, float((np.abs(got - ref[:n]) / size[:n]).max() * 2.0 ** 53))
+    many = list(range(len(pairs))) * 5  # more than one launch of passes for the small ones
+    for at in (many[:16], many[:17], many[:len(pairs)], many):
+        got = op.ExpectValPairs([pairs[k] for k in at], psi).real
+        assert (np.abs(got - ref[at]) <= 64 * 2.0 ** -53 * size[at]).all(), \
+            (len(at), float((np.abs(got - ref[at]) / size[at]).max() * 2.0 ** 53))
     dJ = ed.Adjoint.energy_gradient(b, pairs, psi)[0]
     assert (np.abs(dJ - ref) <= 67 * 2.0 ** -53 * size).all()  # divided by the norm as well
